@@ -64,6 +64,7 @@ class _Graph:
         self.lengths = torch.zeros(rows, dtype=torch.int64, device=dev)
         self.out = torch.empty(rows, dtype=torch.float64, device=dev)
         self.graph = None
+        self.work = None  # count-table workspace, None where the index walk serves the shape
         self._scorer = weakref.ref(scorer)  # no cycle: graphs go with their scorer
 
     @property
@@ -76,12 +77,15 @@ class _Graph:
         self.fwd, self.rc, self.counts = engine.pack(spec, self.codes, self.lengths)
         if s.table is not None:
             return
+        self.order = torch.argsort(self.counts, descending=True).to(torch.int32)
+        self.work = engine.table_workspace(s.index, *self.fwd.shape, 0, self.fwd.device, s.work)
+        if self.work is not None:
+            return  # the query counts the rows' self-kernels, too
         if s.normalize:
             dx = engine.self_kernel(spec, self.fwd, self.rc, self.counts)
             self.inv_dx = 1.0 / torch.sqrt(torch.clamp(dx, min=1e-20))
         else:
             self.inv_dx = torch.ones(self.rows, dtype=torch.float64, device=self.fwd.device)
-        self.order = torch.argsort(self.counts, descending=True).to(torch.int32)
 
     def _query(self):
         s = self.scorer
@@ -89,6 +93,10 @@ class _Graph:
         if s.table is not None:
             self.out.copy_(engine.table_score(m._spec(), s.table, self.fwd, self.rc, self.counts, m.bias,
                                               s.normalize))
+            return
+        if self.work is not None:
+            s.index.table_query(self.fwd, self.counts, work=self.work, order=self.order, normalize=s.normalize,
+                                inv_ds=s.inv_ds, coef=s.coef, gamma=s.gamma, rbf=s.rbf, bias=m.bias, scores=self.out)
             return
         s.index.score(self.fwd, self.counts, self.inv_dx, s.inv_ds, s.coef, s.gamma, s.rbf, m.bias, self.order,
                       out=self.out, check=False)
@@ -164,6 +172,7 @@ class BatchedScorer:
             self.inv_ds = model._inv_ds()
             self.coef = model._sv_coef()
         self.use_graphs = use_graphs
+        self.work = engine.Workspace()  # count tables, shared by the buckets (their passes are serial)
         self._graphs: dict = {}
 
     def _graph(self, B: int, L: int) -> _Graph:
@@ -182,8 +191,7 @@ class BatchedScorer:
         B, L = codes.shape
         g = self._graph(B, L)
         self._last = g
-        if self.index is not None:
-            self._before = self.index.counters()
+        self._before = self.index.counters() if self.index is not None else None
         g.codes[:B, :L].copy_(codes)
         if L < g.L:
             g.codes[:B, L:].zero_()
@@ -201,7 +209,7 @@ class BatchedScorer:
             g._query()
             if events:
                 events[1].record()
-        if check:
+        if check and g.work is None:  # count tables are exact: nothing to wait for
             self.check_flags(g)
         return g.out[:B]
 
@@ -211,9 +219,12 @@ class BatchedScorer:
         keeps the fast kernel).  Returns True when it reran."""
         if g is None:
             g = self._last
-        if self.index is not None:
-            return self.index.settle(self._before, g._body)
-        return False
+        if self.index is None:
+            return False
+        if g.work is not None:  # count tables are exact
+            torch.cuda.current_stream().synchronize()
+            return False
+        return self.index.settle(self._before, g._body)
 
 
 class DirectScorer:
@@ -245,6 +256,9 @@ class DirectScorer:
             events[0].record()
         if self.table is not None:
             out = engine.table_score(spec, self.table, fwd, rc, counts, m.bias, self.normalize)
+        elif (out := self.index.scores(fwd, rc, counts, self.normalize, m._inv_ds(), m._sv_coef(), self.gamma,
+                                       self.rbf, m.bias)) is not None:
+            self._rerun = None  # count tables: exact
         else:
             if self.normalize:
                 dx = engine.self_kernel(spec, fwd, rc, counts)
@@ -326,6 +340,7 @@ class _PerRowRunner:
         self.model = model
         self._graphs: dict = {}
         self._uses: dict = {}
+        self.table_work = engine.Workspace()  # count tables, shared by the buckets (their passes are serial)
 
     def body(self, codes, lengths):  # [rows, 4, L] on the device, no host synchronisation
         raise NotImplementedError
@@ -391,7 +406,7 @@ class BatchedIsm(_PerRowRunner):
                 self._work = torch.empty(need, dtype=torch.uint8, device=codes.device)
                 self._works.append(self._work)
             work = self._work[:need]  # the call sizes its passes by the bytes it is given
-        return _ism_rows(m, codes, lengths, codes.device, check=False, work=work)
+        return _ism_rows(m, codes, lengths, codes.device, check=False, work=work, table_work=self.table_work)
 
 
 class BatchedExplain(_PerRowRunner):
@@ -414,4 +429,5 @@ class BatchedExplain(_PerRowRunner):
             # the explain table, if the model's switch calls for one, is chosen
             # once per runner (a large call's cost model)
             self._table[pert] = _explain_table(m, 1 << 62, pert, codes.device)
-        return _explain_rows(m, codes, lengths, self.mode, codes.device, self._table[pert], check=False)
+        return _explain_rows(m, codes, lengths, self.mode, codes.device, self._table[pert], check=False,
+                             work=self.table_work)

@@ -125,7 +125,27 @@ struct gkm_index {
     unsigned int *status; // [2] query event counts (see gkm_index_status)
     unsigned int *queues;            // [GKM_QUEUE_SLOTS] work-queue heads, one per call in flight
     mutable std::atomic<unsigned> next_queue{0};
+    // count-table queries (gkm_count_table.cu); ct_ids null: not built
+    int32_t strands;     // 2: the columns' reverse complements are indexed too
+    uint64_t *wsum;      // host [wd_len + 1]: sums of wd[0 .. k) (weighted)
+    uint32_t *ct_ids;    // table rows of each SV's forward windows
+    uint8_t *ct_wts;     // their window weights (weighted)
+    uint32_t *ct_off;    // [S + 1] into ct_ids, in gather order
+    uint32_t *ct_perm;   // [S] gather order
+    uint32_t *ct_lists;  // neighbour masks by bank class
+    int64_t ct_entries;
 };
+
+// Built with the index / freed with it (gkm_count_table.cu).
+int gkm_ct_build(gkm_index *ix, const uint32_t *fwd, const int32_t *counts, cudaStream_t st);
+void gkm_ct_free(gkm_index *ix);
+// Sum of the window weights of a row of n windows (0: past the weight table).
+uint64_t gkm_weight_sum(const gkm_index *ix, int64_t n);
+// Device-wide exclusive scan and stable LSD radix sort of pairs (gkm_index.cu);
+// the sort may swap the buffers it is given.
+int gkm_scan_exclusive(const uint32_t *in, uint32_t *out, int64_t n, cudaStream_t st);
+int gkm_radix_sort(uint32_t *&keys, uint32_t *&vals, uint32_t *&ktmp, uint32_t *&vtmp, int64_t n, int bits,
+                   cudaStream_t st);
 
 // Concurrent query calls on one index (different streams) each take their own
 // work-queue counter; more than this many in flight at once would share one.

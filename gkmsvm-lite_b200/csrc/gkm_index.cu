@@ -790,6 +790,24 @@ __global__ void lmer_weights_kernel(const uint32_t *__restrict__ off, const uint
 
 }  // namespace
 
+int gkm_scan_exclusive(const uint32_t *in, uint32_t *out, int64_t n, cudaStream_t st)
+{
+    return scan_exclusive(in, out, n, st);
+}
+
+int gkm_radix_sort(uint32_t *&keys, uint32_t *&vals, uint32_t *&ktmp, uint32_t *&vtmp, int64_t n, int bits,
+                   cudaStream_t st)
+{
+    return radix_sort(keys, vals, ktmp, vtmp, n, bits, st);
+}
+
+uint64_t gkm_weight_sum(const gkm_index *ix, int64_t n)
+{
+    // distances n/2 .. 0 on one side, 1 .. n - 1 - n/2 on the other
+    if (!ix->wsum || n < 1 || n / 2 + 1 > ix->spec.wd_len) return 0;
+    return ix->wsum[n / 2 + 1] + ix->wsum[n - n / 2] - ix->wsum[1];
+}
+
 int gkm_smem_limit()
 {
     int dev = 0, v = 0;
@@ -856,6 +874,7 @@ extern "C" int gkm_index_create(const gkm_spec *spec, const uint32_t *fwd, const
     ix->nlev = nlev;
     ix->n_lmers = (int64_t)1 << (2 * spec->l);
     ix->n_masks = n_masks;
+    ix->strands = nb;
     ix->acc_bytes = acc_bytes;
     ix->wide = spec->weighted ? 1 : 0;
     ix->packed = packed;
@@ -872,6 +891,9 @@ extern "C" int gkm_index_create(const gkm_spec *spec, const uint32_t *fwd, const
         }
         ix->wmax = 0;
         for (int32_t k = 0; k < spec->wd_len; k++) ix->wmax = h[k] > ix->wmax ? h[k] : ix->wmax;
+        ix->wsum = (uint64_t *)malloc(sizeof(uint64_t) * ((size_t)spec->wd_len + 1));
+        if (ix->wsum) ix->wsum[0] = 0;
+        for (int32_t k = 0; k < spec->wd_len && ix->wsum; k++) ix->wsum[k + 1] = ix->wsum[k] + h[k];
         free(h);
         if (ix->wmax == 0) ix->wmax = 1;
     }
@@ -964,6 +986,7 @@ extern "C" int gkm_index_create(const gkm_spec *spec, const uint32_t *fwd, const
         cudaMemsetAsync(ix->status, 0, 2 * sizeof(unsigned int), st);
         ix->bytes = (int64_t)sizeof(uint32_t) * ((ix->bwords ? 2 : 1) * nbuckets + 1) + (int64_t)eb +
                     sizeof(uint32_t) * n_masks;
+        status = gkm_ct_build(ix, fwd, counts, st);
     } while (0);
     cudaFreeAsync(ecount, st);
     cudaFreeAsync(keys, st);
@@ -992,6 +1015,8 @@ extern "C" int gkm_index_free(gkm_index_t *ix)
     cudaFree(ix->masks);
     cudaFree(ix->status);
     cudaFree(ix->queues);
+    gkm_ct_free(ix);
+    free(ix->wsum);
     delete ix;
     return GKM_OK;
 }

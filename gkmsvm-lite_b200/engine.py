@@ -206,6 +206,32 @@ def masks_tensor(base, device) -> torch.Tensor:
     return torch.from_numpy(m.view(np.int32).copy()).to(device)
 
 
+class Workspace:
+    """A device buffer that grows on request; every buffer handed out is kept
+    for the object's life, because captured graphs refer to it.  For one
+    stream at a time."""
+
+    def __init__(self):
+        self._buffers = []
+
+    def get(self, n: int, device) -> torch.Tensor:
+        if not self._buffers or self._buffers[-1].numel() < n:
+            self._buffers.append(torch.empty(n, dtype=torch.uint8, device=device))
+        return self._buffers[-1][:n]
+
+
+def table_workspace(index, B: int, W: int, windows: int, device, work: Workspace | None = None):
+    """The workspace of a count-table query, or None where the walk serves the
+    call or the device has no room for it."""
+    n = index.table_bytes(B, W, windows)
+    if n == 0:
+        return None
+    try:
+        return torch.empty(n, dtype=torch.uint8, device=device) if work is None else work.get(n, device)
+    except torch.cuda.OutOfMemoryError:
+        return None
+
+
 class DeviceIndex:
     """An l-mer index handle over packed columns (owned; freed on close)."""
 
@@ -310,6 +336,51 @@ class DeviceIndex:
             return out
 
         return self.checked(run) if check else run()
+
+    def table_bytes(self, B: int, W: int, windows: int = 0) -> int:
+        """Workspace bytes of a count-table query of B rows of W window slots
+        (windows in all; 0: unknown); 0 where the index walk serves it."""
+        n = ctypes.c_int64()
+        call("gkm_count_table_workspace", self.handle, B, W, int(windows), ctypes.byref(n))
+        return n.value
+
+    def table_query(self, bx, cx, *, work, order=None, normalize=True, inv_dx=None, diag=None, diag_offset=None,
+                    raw=None, inv_ds=None, coef=None, gamma=0.0, rbf=False, bias=0.0, scores=None):
+        """Scores [B] or K_raw [B, S] (into scores / raw) through count tables,
+        exact with no check to settle; diag (nullable) gets the rows' K(x, x).
+        work: a uint8 tensor of table_bytes(B, W)."""
+        B, W = bx.shape
+        call("gkm_count_table_query", self.handle, ptr(bx), ptr(cx), B, W, ptr(order), int(bool(normalize)),
+             ptr(inv_dx), ptr(diag), -1 if diag_offset is None else int(diag_offset), ptr(raw), ptr(inv_ds),
+             ptr(coef), float(gamma), int(rbf), float(bias), ptr(scores), ptr(work), int(work.numel()), _st())
+
+    def rows(self, bx, rx, cx, normalize, *, diag_offset=None, out=None, check=True, windows=0, work=None):
+        """(K_raw [B, S], K(x, x) [B] or None without normalize) of packed
+        rows: through count tables where they are the cheaper form (work: a
+        Workspace that outlives the call, for captured graphs), else by the
+        walk and the self-kernel."""
+        B, W = bx.shape
+        tw = table_workspace(self, B, W, windows, bx.device, work)
+        if tw is None:
+            raw, _ = self.pairwise(bx, cx, diag_offset, out=out, check=check)
+            return raw, self_kernel(self.spec, bx, rx, cx) if normalize else None
+        if out is None:
+            out = torch.empty((B, self.S), dtype=torch.float64, device=bx.device)
+        diag = torch.empty(B, dtype=torch.float64, device=bx.device) if normalize else None
+        self.table_query(bx, cx, work=tw, diag=diag, diag_offset=diag_offset, raw=out)
+        return out, diag
+
+    def scores(self, bx, rx, cx, normalize, inv_ds, coef, gamma, rbf, bias, order=None, *, windows=0, work=None):
+        """[B] scores of packed rows through count tables, or None where the
+        walk (score) serves them."""
+        B, W = bx.shape
+        tw = table_workspace(self, B, W, windows, bx.device, work)
+        if tw is None:
+            return None
+        out = torch.empty(B, dtype=torch.float64, device=bx.device)
+        self.table_query(bx, cx, work=tw, order=order, normalize=normalize, inv_ds=inv_ds, coef=coef, gamma=gamma,
+                         rbf=rbf, bias=bias, scores=out)
+        return out
 
     def count(self, bx, cx):
         """(lookups, hits) an index query over rows bx makes."""

@@ -160,10 +160,10 @@ def gkmexplain(model, x, *, mode="importance", lengths=None, batch_size=50, verb
     return per_position(out, batch, short)
 
 
-def _explain_rows(model, x, lengths, mode, dev, table=None, check=True):
+def _explain_rows(model, x, lengths, mode, dev, table=None, check=True, work=None):
     """[B, 4, L] attributions of one pass (x: host or device codes).
     check=False: no host synchronisation (the index's exactness check is the
-    caller's)."""
+    caller's).  work: an engine.Workspace for captured passes."""
     kernel = model.kernel
     base = kernel.base
     spec = model._spec()
@@ -175,21 +175,24 @@ def _explain_rows(model, x, lengths, mode, dev, table=None, check=True):
     spec.check_rows(int(fwd.shape[1]))
     perturbation = mode == "perturbation"
     B, W = fwd.shape
-    if base.normalize:
-        dx = engine.self_kernel(spec, fwd, rc, counts)
-        inv_dx = 1.0 / torch.sqrt(torch.clamp(dx, min=1e-20))
-    else:
+    V = index = w = out = raw = dx = None
+    pairs = table is None and _explain_uses_pairs(model, perturbation)
+    if table is None and not pairs and isinstance(kernel, RbfKernel):
+        index = model._sv_index()  # not None: _explain_uses_pairs
+        raw, dx = index.rows(fwd, rc, counts, base.normalize, check=check, work=work)
+    if not base.normalize:
         inv_dx = torch.ones(B, dtype=torch.float64, device=dev)
-    V = index = w = out = None
-    if table is None and _explain_uses_pairs(model, perturbation):
+    else:
+        if dx is None:
+            dx = engine.self_kernel(spec, fwd, rc, counts)
+        inv_dx = 1.0 / torch.sqrt(torch.clamp(dx, min=1e-20))
+    if pairs:
         out = _explain_pairs(model, spec, fwd, counts, inv_dx, L, perturbation, dev)
     elif table is not None:
         out = torch.empty((B, 4, L), dtype=torch.float64, device=dev)
         call("gkm_explain_table", spec.ref, ptr(table), ptr(fwd), ptr(counts), B, W, L, ptr(inv_dx),
              int(perturbation), ptr(out), stream_handle())
-    elif isinstance(kernel, RbfKernel):
-        index = model._sv_index()  # not None: _explain_uses_pairs
-        raw, _ = index.pairwise(fwd, counts, check=check)
+    elif raw is not None:
         inv_ds = model._inv_ds()
         k_norm = raw * inv_dx[:, None] * inv_ds[None, :]
         w = (model._sv_coef() * inv_ds)[None, :] * _rbf_scale(k_norm, kernel.gamma)
@@ -266,11 +269,13 @@ def mutation_impact(model, ref, alt, *, ref_lengths=None, alt_lengths=None, batc
                 dk = dk / torch.sqrt(torch.clamp(diag[:n], min=1e-10))
             parts.append(dk)
             continue
-        dr = engine.self_kernel(spec, fwd[:n], None if rc is None else rc[:n], counts[:n]) if base.normalize else None
+        dr = None
         index = model._sv_index()
         if index is not None:
-            kb, _ = index.pairwise(fwd, counts)
+            kb, dr = index.rows(fwd, rc, counts, base.normalize)
         else:
+            if base.normalize:
+                dr = engine.self_kernel(spec, fwd[:n], None if rc is None else rc[:n], counts[:n])
             by, ry, cy = model._sv_packed()
             kb, _ = engine.pairwise(spec, fwd, counts, by, ry, cy)
         ds = model._sv_diag() if base.normalize else None

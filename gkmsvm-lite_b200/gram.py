@@ -39,16 +39,14 @@ def compute_gram(kernel, X, Y=None, *, chunk_size=1000, verbose=False, out=None,
         by, ry, cy = engine.pack(spec, yb.on(dev), yb.lengths)
     spec.check_rows(int(max(bx.shape[1], by.shape[1])))
     dx = dy = None
-    if base.normalize:
-        dx = engine.self_kernel(spec, bx, rx, cx)
-        dy = dx if symmetric else engine.self_kernel(spec, by, ry, cy)
     n_windows = int(cy.sum().item()) * (2 if base.include_rc else 1)
     use_index = isinstance(base, DirectGkmKernel) and n_windows > 0 and base.index_applies(n_windows)
     raw = torch.zeros((N, M), dtype=torch.float64, device=dev)
     if use_index:
         index = engine.DeviceIndex(spec, by, ry, cy, engine.masks_tensor(base, dev))
         try:
-            index.pairwise(bx, cx, diag_offset=0 if symmetric else None, out=raw)
+            _, dx = index.rows(bx, rx, cx, base.normalize, diag_offset=0 if symmetric else None, out=raw,
+                               windows=xb.n_windows(base.l))
         finally:
             index.close()
     else:
@@ -56,6 +54,10 @@ def compute_gram(kernel, X, Y=None, *, chunk_size=1000, verbose=False, out=None,
         for s in range(0, N, step):
             r, _ = engine.pairwise(spec, bx[s:s + step], cx[s:s + step], by, ry, cy)
             raw[s:s + step] = r
+        if base.normalize:
+            dx = engine.self_kernel(spec, bx, rx, cx)
+    if base.normalize:
+        dy = dx if symmetric else engine.self_kernel(spec, by, ry, cy)
     rbf = isinstance(kernel, RbfKernel)
     gram = engine.gram_finish(raw, dx, dy, kernel.gamma if rbf else 0.0, rbf, symmetric)
     host = gram.cpu().numpy()

@@ -47,7 +47,7 @@ def ism(model, x, *, lengths=None, batch_size=None, verbose=False) -> torch.Tens
     return per_position(out, batch, short)
 
 
-def _ism_rows(model, x, lengths, dev, check=True, work=None):
+def _ism_rows(model, x, lengths, dev, check=True, work=None, table_work=None):
     """[B, 4, L] deltas of one pass (x: host or device codes).  check=False:
     no host synchronisation (the index's exactness check is the caller's)."""
     base = model.kernel.base
@@ -62,10 +62,10 @@ def _ism_rows(model, x, lengths, dev, check=True, work=None):
     if table is not None:
         _, raw, diag = engine.table_score(spec, table, fwd, rc, counts, 0.0, base.normalize, want_parts=True)
         return engine.ism_table(spec, table, fwd, counts, L, raw, diag, base.normalize)
-    return _ism_index(model, fwd, rc, counts, L, check, work)
+    return _ism_index(model, fwd, rc, counts, L, check, work, table_work)
 
 
-def _ism_index(model, fwd, rc, counts, L, check=True, work=None):
+def _ism_index(model, fwd, rc, counts, L, check=True, work=None, table_work=None):
     kernel = model.kernel
     base = kernel.base
     spec = model._spec()
@@ -76,21 +76,20 @@ def _ism_index(model, fwd, rc, counts, L, check=True, work=None):
     B, W = fwd.shape
     rbf = isinstance(kernel, RbfKernel)
     gamma = kernel.gamma if rbf else 0.0
-    if base.normalize:
-        diag = engine.self_kernel(spec, fwd, rc, counts)
-        mut = engine.mutant_diag(spec, fwd, counts, L, diag)
-        inv_dx = 1.0 / torch.sqrt(torch.clamp(diag, min=1e-20))
-        inv_dmut = 1.0 / torch.sqrt(torch.clamp(mut, min=1e-20))
-    else:
-        inv_dx = torch.ones(B, dtype=torch.float64, device=fwd.device)
-        inv_dmut = torch.ones((4, L, B), dtype=torch.float64, device=fwd.device)
     out = torch.empty((B, 4, L), dtype=torch.float64, device=fwd.device)
     if work is None:
         work = ism_workspace(model, B, L, fwd.device)
 
     def run():
         # the reference rows' K_raw; their scores come from it inside the call
-        ref_raw, _ = index.pairwise(fwd, counts, check=False)
+        ref_raw, diag = index.rows(fwd, rc, counts, base.normalize, check=False, work=table_work)
+        if base.normalize:
+            mut = engine.mutant_diag(spec, fwd, counts, L, diag)
+            inv_dx = 1.0 / torch.sqrt(torch.clamp(diag, min=1e-20))
+            inv_dmut = 1.0 / torch.sqrt(torch.clamp(mut, min=1e-20))
+        else:
+            inv_dx = torch.ones(B, dtype=torch.float64, device=fwd.device)
+            inv_dmut = torch.ones((4, L, B), dtype=torch.float64, device=fwd.device)
         call("gkm_index_mutants", index.handle, ptr(fwd), ptr(counts), B, W, L, ptr(ref_raw), None,
              ptr(inv_dx), ptr(inv_dmut), ptr(model._inv_ds()), ptr(model._sv_coef()), float(gamma), int(rbf),
              ptr(out), ptr(work), int(work.numel()), stream_handle())

@@ -237,8 +237,9 @@ class GkmSVM:
 
     # -- scoring ----------------------------------------------------------------
 
-    def _score_packed(self, fwd, rc, counts) -> torch.Tensor:
-        """[B] scores (bias included) of packed rows on the model's device."""
+    def _score_packed(self, fwd, rc, counts, windows: int = 0) -> torch.Tensor:
+        """[B] scores (bias included) of packed rows on the model's device
+        (windows: their windows in all, 0: unknown)."""
         kernel = self.kernel
         base = kernel.base
         spec = self._spec()
@@ -248,14 +249,20 @@ class GkmSVM:
             return engine.table_score(spec, table, fwd, rc, counts, self.bias, base.normalize)
         rbf = isinstance(kernel, RbfKernel)
         gamma = kernel.gamma if rbf else 0.0
-        dx = engine.self_kernel(spec, fwd, rc, counts) if base.normalize else None
         index = self._sv_index()
+        order = None
+        if index is not None:
+            order = torch.argsort(counts, descending=True).to(torch.int32)
+            out = index.scores(fwd, rc, counts, base.normalize, self._inv_ds(), self._sv_coef(), gamma, rbf, self.bias,
+                               order, windows=windows)
+            if out is not None:
+                return out
+        dx = engine.self_kernel(spec, fwd, rc, counts) if base.normalize else None
         if index is not None:
             if dx is None:
                 inv_dx = torch.ones(fwd.shape[0], dtype=torch.float64, device=fwd.device)
             else:
                 inv_dx = 1.0 / torch.sqrt(torch.clamp(dx, min=1e-20))
-            order = torch.argsort(counts, descending=True).to(torch.int32)
             return index.score(fwd, counts, inv_dx, self._inv_ds(), self._sv_coef(), gamma, rbf,
                                self.bias, order)
         by, ry, cy = self._sv_packed()
@@ -273,7 +280,12 @@ class GkmSVM:
         dev = self._require_gpu()
         xt = device_codes(codes, dev)
         fwd, rc, counts = engine.pack(self._spec(), xt, lengths)
-        return self._score_packed(fwd, rc, counts)
+        windows = 0
+        if lengths is None:
+            windows = int(fwd.numel())
+        elif not isinstance(lengths, torch.Tensor):
+            windows = int(np.clip(lengths - self.kernel.l + 1, 0, None).sum())
+        return self._score_packed(fwd, rc, counts, windows)
 
     def _score_unbatched(self, batch: SeqBatch) -> torch.Tensor:
         W = max(batch.L - self.kernel.l + 1, 1)
