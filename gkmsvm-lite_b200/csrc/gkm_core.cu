@@ -142,52 +142,193 @@ __device__ void block_reduce_levels(uint64_t *tot, uint64_t *red, uint64_t *sums
     __syncthreads();
 }
 
-// sw: windows the shared memory holds per strand (2 * sw words)
-__device__ __forceinline__ RowView stage_row(const uint32_t *fwd, const uint32_t *rc, int64_t W,
-                                             int n, bool has_rc, uint32_t *sm, int sw)
+// Mismatches of 32 neighbouring window pairs at once, bit-sliced: bit p of plane
+// k is bit k of the mismatches of the windows at p, given e (bit p: the bases at p
+// differ) and the word after it.  The L shifted copies of e are summed by carry-
+// save adders (a full adder is two logic operations).  L = 0: run-time length l.
+struct Planes {
+    uint32_t v[4];
+};
+
+template <int L>
+__device__ __forceinline__ Planes mismatch_planes(uint32_t e, uint32_t en, int l)
 {
-    RowView rv;
-    rv.W = W;
-    if (n <= sw) {
-        for (int k = threadIdx.x; k < n; k += blockDim.x) {
-            sm[k] = fwd[k];
-            if (has_rc) sm[sw + k] = rc[W - 1 - k];
+    Planes r;
+    if constexpr (L == 0) {
+        r.v[0] = r.v[1] = r.v[2] = r.v[3] = 0;
+        for (int k = 0; k < l; k++) {
+            uint32_t c = __funnelshift_r(e, en, k);
+#pragma unroll
+            for (int j = 0; j < 4; j++) {
+                const uint32_t x = r.v[j] & c;
+                r.v[j] ^= c;
+                c = x;
+            }
         }
-        rv.f = sm;
-        rv.r = sm + sw;
-        rv.reversed = false;
     } else {
-        rv.f = fwd;
-        rv.r = rc;
-        rv.reversed = true;
+        uint32_t a[4][L];
+        int n[4] = {L, 0, 0, 0};
+#pragma unroll
+        for (int k = 0; k < L; k++) a[0][k] = k ? __funnelshift_r(e, en, k) : e;
+#pragma unroll
+        for (int j = 0; j < 4; j++) {
+#pragma unroll
+            for (int k = 0; k < L; k++) {  // at most L adders a plane
+                if (n[j] >= 3) {
+                    const uint32_t x = a[j][n[j] - 1], y = a[j][n[j] - 2], z = a[j][n[j] - 3];
+                    if (j < 3) a[j + 1][n[j + 1]++] = (x & y) | (x & z) | (y & z);
+                    n[j] -= 2;
+                    a[j][n[j] - 1] = x ^ y ^ z;
+                } else if (n[j] == 2) {
+                    const uint32_t x = a[j][1], y = a[j][0];
+                    if (j < 3) a[j + 1][n[j + 1]++] = x & y;
+                    n[j] = 1;
+                    a[j][0] = x ^ y;
+                }
+            }
+            r.v[j] = n[j] ? a[j][0] : 0u;
+        }
     }
-    __syncthreads();
-    return rv;
+    return r;
 }
+
+// bits of `valid` whose pair has m mismatches
+__device__ __forceinline__ uint32_t level_mask(const Planes &p, int m, uint32_t valid)
+{
+    return valid & (m & 1 ? p.v[0] : ~p.v[0]) & (m & 2 ? p.v[1] : ~p.v[1]) & (m & 4 ? p.v[2] : ~p.v[2]) &
+           (m & 8 ? p.v[3] : ~p.v[3]);
+}
+
+// A row's bases as bit planes: x (forward) and y (reverse complement), two words
+// per 32 bases each, zero past the row.  Returns whether the packed windows are
+// not those of one sequence (all threads).
+__device__ __forceinline__ bool stage_planes(const uint32_t *frow, int n, int l, uint32_t *pl, int pw)
+{
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5, nb = n + l - 1;
+    const uint32_t low = (1u << (2 * (l - 1))) - 1u;
+    bool bad = false;
+    auto base = [&](int p) -> uint32_t {
+        return p < n ? frow[p] & 3u : (frow[n - 1] >> (2 * (p - n + 1))) & 3u;
+    };
+    for (int k = warp; k < pw; k += nw) {
+        const int p = k * 32 + lane;
+        const uint32_t x = n > 0 && p < nb ? base(p) : 0u, y = n > 0 && p < nb ? 3u - base(nb - 1 - p) : 0u;
+        if (p + 1 < n) bad |= (frow[p + 1] & low) != (frow[p] >> 2);
+        const uint32_t x0 = __ballot_sync(GKM_FULL, x & 1u), x1 = __ballot_sync(GKM_FULL, x & 2u);
+        const uint32_t y0 = __ballot_sync(GKM_FULL, y & 1u), y1 = __ballot_sync(GKM_FULL, y & 2u);
+        if (lane == 0) {
+            pl[k] = x0;
+            pl[pw + k] = x1;
+            pl[2 * pw + k] = y0;
+            pl[3 * pw + k] = y1;
+        }
+    }
+    return __syncthreads_or(bad);
+}
+
+// bit plane words of a row of W windows: the bases and three words past them
+__host__ __device__ inline int plane_words(int64_t W, int l) { return (int)((W + l - 1 + 31) / 32) + 3; }
 
 // Self-kernel of one row per block, optionally fused with the l-mer table sum
 // (svm.py:559-582: score = sum_i wt_i table[x_i] / sqrt(K(x, x)) + b).
-template <int NW>
+//
+// A pair of windows (i, i + s) compares the same positions as its neighbour on
+// the diagonal, shifted by one: along a diagonal the mismatches are a sliding sum
+// of the bits "bases p and p + s differ", which 32 pairs at a time take ~50
+// operations (a pair alone took 11 and a quarter-rate population count).  Forward x
+// RC pairs are the diagonals of the sequence against its reverse complement, each
+// symmetric about its middle: half of it is summed.  Bound by the integer pipe;
+// measured fused with the table sum (t=2): 8,192 rows of 50 .. 2,000 bp 4,516 us
+// pair by pair -> 633 us, 512 rows of 1,000 bp 544 -> 71 us.  Rows whose windows do not overlap (not one sequence's) or whose planes do
+// not fit shared memory are still taken pair by pair.
+template <int L, int NL, bool WT>
 __global__ void __launch_bounds__(SELF_THREADS) self_kernel(
     gkm_spec spec, const uint32_t *__restrict__ fwd, const uint32_t *__restrict__ rc,
     const int32_t *__restrict__ counts, int64_t W, double *__restrict__ diag,
     uint64_t *__restrict__ profile, const double *__restrict__ table, double bias, int normalize,
-    double *__restrict__ scores, double *__restrict__ raw_out, int sw)
+    double *__restrict__ scores, double *__restrict__ raw_out, int pw)
 {
-    constexpr int NL = 4 * NW;
-    extern __shared__ uint32_t sm[];
+    extern __shared__ uint32_t pl[];  // x0, x1, y0, y1, pw words each
     __shared__ uint64_t red[(SELF_THREADS / 32) * NL];
     __shared__ uint64_t sums[NL];
     __shared__ double dred[32];
     int64_t b = blockIdx.x;
-    int n = counts[b];
-    bool has_rc = spec.include_rc && rc != nullptr;
+    const int n = counts[b], l = L ? L : spec.l;
+    const bool has_rc = spec.include_rc && rc != nullptr;
     const uint32_t *frow = fwd + b * W;
-    RowView rv = stage_row(frow, has_rc ? rc + b * W : nullptr, W, n, has_rc, sm, sw);
+    const uint8_t *wd = spec.wd;
     uint64_t tot[NL];
 #pragma unroll
     for (int m = 0; m < NL; m++) tot[m] = 0;
-    self_pairs<NW>(rv, n, has_rc, spec.wd, spec.weighted, tot);
+    if (pw == 0 || stage_planes(frow, n, l, pl, pw)) {
+        RowView rv;
+        rv.f = frow;
+        rv.r = has_rc ? rc + b * W : nullptr;
+        rv.W = W;
+        rv.reversed = true;
+        self_pairs<NL / 4>(rv, n, has_rc, wd, WT, tot);
+    } else {
+        uint32_t cnt[NL], mid[NL];
+#pragma unroll
+        for (int m = 0; m < NL; m++) cnt[m] = mid[m] = 0;
+        // diagonal s of x against x (0), x against y (1) and y against x (2)
+        for (int t = threadIdx.x; t < (has_rc ? 3 * n : n); t += SELF_THREADS) {
+            const int mode = t >= 2 * n ? 2 : t >= n ? 1 : 0, s = t - mode * n, len = n - s;
+            if (s == 0 && mode != 1) continue;  // mode 0: a window with itself, below; mode 2: mode 1's
+            const int H = mode ? (len + 1) >> 1 : len;
+            const bool odd = mode && (len & 1);  // the last of the half is its own mirror image
+            const uint32_t *P = pl + (mode == 2 ? 2 * pw : 0), *Q = pl + (mode == 1 ? 2 * pw : 0) + (s >> 5);
+            uint32_t q0 = Q[0], q1 = Q[pw];
+            auto differ = [&](int w) -> uint32_t {  // words in turn
+                const uint32_t n0 = Q[w + 1], n1 = Q[pw + w + 1];
+                const uint32_t e = (P[w] ^ __funnelshift_r(q0, n0, s)) | (P[pw + w] ^ __funnelshift_r(q1, n1, s));
+                q0 = n0;
+                q1 = n1;
+                return e;
+            };
+            uint32_t e = differ(0);
+            const int nw = (H + 31) >> 5;
+            for (int w = 0; w < nw; w++) {
+                const uint32_t en = differ(w + 1);
+                const Planes pn = mismatch_planes<L>(e, en, l);
+                const bool last = w == nw - 1;
+                const uint32_t valid = last && (H & 31) ? (1u << (H & 31)) - 1u : GKM_FULL;
+                e = en;
+                uint32_t near = valid;
+                if (NL == 4) near &= ~pn.v[2] & ~pn.v[3];
+                if (WT) {
+#pragma unroll
+                    for (int m = 0; m < NL; m++) {
+                        if (m > spec.dmax) break;
+                        for (uint32_t h = level_mask(pn, m, near); h; h &= h - 1) {
+                            const int i = w * 32 + __ffs(h) - 1;
+                            // windows i and i + s; an RC window has its forward window's weight
+                            const int j = mode ? n - 1 - (i + s) : i + s, i2 = mode == 2 ? n - 1 - i : i,
+                                      j2 = mode == 2 ? i + s : j;
+                            tot[m] += (odd && i == H - 1 ? 1ull : 2ull) * gkm_wt(wd, n, i2) * gkm_wt(wd, n, j2);
+                        }
+                    }
+                } else {
+#pragma unroll
+                    for (int m = 0; m < NL; m++) {
+                        const uint32_t h = level_mask(pn, m, near);
+                        cnt[m] += __popc(h);
+                        if (last && odd) mid[m] += (h >> ((H - 1) & 31)) & 1u;
+                    }
+                }
+            }
+        }
+        if (WT) {
+            for (int i = threadIdx.x; i < n; i += SELF_THREADS) {
+                const uint64_t w = gkm_wt(wd, n, i);
+                tot[0] += w * w;
+            }
+        } else {
+#pragma unroll
+            for (int m = 0; m < NL; m++) tot[m] = 2ull * cnt[m] - mid[m];
+            if (threadIdx.x == 0) tot[0] += n;
+        }
+    }
     block_reduce_levels<NL>(tot, red, sums);
     double k = 0.0;
 #pragma unroll
@@ -203,7 +344,7 @@ __global__ void __launch_bounds__(SELF_THREADS) self_kernel(
         double t = 0.0;
         for (int i = threadIdx.x; i < n; i += blockDim.x) {
             double a = spec.weighted ? (double)gkm_wt(spec.wd, n, i) : 1.0;
-            t += a * table[rv.f[i]];
+            t += a * table[frow[i]];
         }
         t = gkm_block_sum(t, dred);
         if (threadIdx.x == 0) {
@@ -583,21 +724,28 @@ static int self_launch(const gkm_spec *spec, const uint32_t *fwd, const uint32_t
                        int normalize, double *scores, double *raw, cudaStream_t st)
 {
     if (B == 0) return GKM_OK;
-    const int sw = staged_windows(W);
-    size_t smem = (size_t)2 * sw * sizeof(uint32_t);
-    int nw = nw_for(spec->dmax);
-#define GKM_SELF(NW)                                                                                  \
-    do {                                                                                              \
-        cudaFuncSetAttribute(self_kernel<NW>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem); \
-        GKM_PREFER_SHARED(self_kernel<NW>);                                                            \
-        self_kernel<NW><<<(unsigned)B, SELF_THREADS, smem, st>>>(*spec, fwd, rc, counts, W, diag,      \
-                                                                 profile, table, bias, normalize,     \
-                                                                 scores, raw, sw);                    \
+    int pw = plane_words(W, spec->l);
+    size_t smem = (size_t)4 * pw * sizeof(uint32_t);
+    if (smem > 200 * 1024) smem = pw = 0;
+#define GKM_SELF_AS(L, NL, WT)                                                                                \
+    do {                                                                                                      \
+        cudaFuncSetAttribute(self_kernel<L, NL, WT>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem); \
+        GKM_PREFER_SHARED((self_kernel<L, NL, WT>));                                                          \
+        self_kernel<L, NL, WT><<<(unsigned)B, SELF_THREADS, smem, st>>>(                                      \
+            *spec, fwd, rc, counts, W, diag, profile, table, bias, normalize, scores, raw, pw);               \
     } while (0)
-    if (nw == 1) GKM_SELF(1);
-    else if (nw == 2) GKM_SELF(2);
-    else GKM_SELF(4);
+#define GKM_SELF(L)                                                       \
+    do {                                                                  \
+        if (spec->dmax < 4 && spec->weighted) GKM_SELF_AS(L, 4, true);    \
+        else if (spec->dmax < 4) GKM_SELF_AS(L, 4, false);                \
+        else if (spec->weighted) GKM_SELF_AS(L, 16, true);                \
+        else GKM_SELF_AS(L, 16, false);                                   \
+    } while (0)
+    if (spec->l == 11) GKM_SELF(11);
+    else if (spec->l == 10) GKM_SELF(10);
+    else GKM_SELF(0);
 #undef GKM_SELF
+#undef GKM_SELF_AS
     GKM_CHECK_LAUNCH("self_kernel");
     return GKM_OK;
 }
