@@ -123,6 +123,174 @@ __global__ void __launch_bounds__(EX_WARPS * 32) explain_windows(ExplainArgs a)
     }
 }
 
+// The same attributions from l-mer weights V, for neighbourhoods of at most XS_MAX
+// mismatches.  A mask is a subset of positions and a digit 1..3 at each: one block
+// takes a window, its threads the subsets (232 at l = 11, three mismatches), so that
+// a subset's 3^m neighbours are gathered at once and summed by digit in registers --
+// T, their sum, and D[j][d], those with digit d at the subset's j-th position: ~2 adds
+// per neighbour where the loop above makes 44 conditional ones.  Then one thread per
+// output adds its subsets in a fixed order: T of those that leave position k alone,
+// D of those that change it.  Bound by the L2 gathers of V (8 of 32 bytes used).
+// Measured: linear t=2 model, 512 x 1,000 bp, 330 (explain_windows) -> 45 ns a window;
+// RBF model of 72,000 SVs, 4 rows of 300 .. 600 bp, 166 us (and row_weights 328) where
+// explain_windows over the buckets took 4,318.
+constexpr int XS_MAX = 4;
+constexpr int XS_THREADS = 128;
+
+struct SubsetArgs {
+    const uint32_t *fwd;
+    const int32_t *cnt;
+    int64_t W;
+    int l;
+    const double *V;       // [4^l], or one per row
+    int64_t v_stride;      // 4^l, or 0
+    int weighted;
+    const uint8_t *wd;
+    const uint32_t *subs;  // [n_sub] positions (4 bits each) | size << 16, large ones first
+    const uint16_t *lists; // [l][n_sub]: the subsets with position k (subset | place << 12), then those without
+    const int32_t *n_with; // [l]
+    int n_sub;
+    const double *ta;
+    const double *tb;
+    int perturbation;
+    double *part;          // [B, W, 4, l]
+};
+
+// sums of the neighbours u ^ (digits at pos[0 .. M)) by digit
+template <int M>
+__device__ __forceinline__ void subset_sums(const double *__restrict__ V, uint32_t u, uint32_t pos, double *out)
+{
+    constexpr int N = M == 0 ? 1 : M == 1 ? 3 : M == 2 ? 9 : M == 3 ? 27 : 81;
+    constexpr int CH = N < 27 ? N : 27;  // gathers in flight
+    double t = 0.0, d[M ? M : 1][3];
+#pragma unroll
+    for (int j = 0; j < M; j++) d[j][0] = d[j][1] = d[j][2] = 0.0;
+#pragma unroll
+    for (int c = 0; c < N / CH; c++) {
+        double v[CH];
+#pragma unroll
+        for (int i = 0; i < CH; i++) {
+            uint32_t x = u;
+            int r = c * CH + i;
+#pragma unroll
+            for (int j = 0; j < M; j++) {
+                x ^= (uint32_t)(r % 3 + 1) << (2 * ((pos >> (4 * j)) & 15u));
+                r /= 3;
+            }
+            v[i] = __ldg(V + x);
+        }
+#pragma unroll
+        for (int i = 0; i < CH; i++) {
+            int r = c * CH + i;
+            t += v[i];
+#pragma unroll
+            for (int j = 0; j < M; j++) {
+                d[j][r % 3] += v[i];
+                r /= 3;
+            }
+        }
+    }
+    out[0] = t;
+#pragma unroll
+    for (int j = 0; j < M; j++)
+#pragma unroll
+        for (int k = 0; k < 3; k++) out[1 + 3 * j + k] = d[j][k];
+}
+
+__global__ void __launch_bounds__(XS_THREADS) explain_subsets(SubsetArgs a, int stride)
+{
+    extern __shared__ double sums[];  // [n_sub][stride]: T, D[j][d]
+    __shared__ double res[4][LMAX];
+    const int64_t b = blockIdx.y, win = blockIdx.x;
+    const int n = a.cnt[b], l = a.l;
+    double *out = a.part + ((b * a.W + win) * 4) * l;
+    if (win >= n) {  // PAD window: nothing
+        for (int k = threadIdx.x; k < 4 * l; k += XS_THREADS) out[k] = 0.0;
+        return;
+    }
+    const uint32_t u = a.fwd[b * a.W + win];
+    const double *V = a.V + b * a.v_stride;
+    for (int k = threadIdx.x; k < a.n_sub; k += XS_THREADS) {
+        const uint32_t sub = a.subs[k];
+        double *o = sums + k * stride;
+        switch (sub >> 16) {
+        case 4: subset_sums<4>(V, u, sub, o); break;
+        case 3: subset_sums<3>(V, u, sub, o); break;
+        case 2: subset_sums<2>(V, u, sub, o); break;
+        case 1: subset_sums<1>(V, u, sub, o); break;
+        default: subset_sums<0>(V, u, sub, o);
+        }
+    }
+    __syncthreads();
+    // output (k, d): d = 0 the neighbours that leave position k alone, else those
+    // with digit d there; two threads each
+    const int half = threadIdx.x & 1, o = threadIdx.x >> 1, k = o >> 2, d = o & 3;
+    double acc = 0.0;
+    if (k < l) {
+        const uint16_t *list = a.lists + k * a.n_sub;
+        const int nw = a.n_with[k], i0 = d ? 0 : nw, i1 = d ? nw : a.n_sub, im = i0 + ((i1 - i0 + 1) >> 1);
+        const double *t = d ? a.tb : a.ta;
+        for (int i = half ? im : i0; i < (half ? i1 : im); i++) {
+            const uint32_t e = list[i], s = e & 0xFFFu;
+            acc += __ldg(t + (a.subs[s] >> 16)) * sums[s * stride + (d ? 3 * (e >> 12) + d : 0)];
+        }
+    }
+    const double other = __shfl_xor_sync(GKM_FULL, acc, 1);
+    if (k < l && !half) res[d][k] = acc + other;
+    __syncthreads();
+    const double wx = a.weighted ? (double)gkm_wt(a.wd, n, (int)win) : 1.0;
+    for (int t = threadIdx.x; t < 4 * l; t += XS_THREADS) {
+        const int base = t / l, p = t - base * l, x = base ^ (int)((u >> (2 * p)) & 3u);
+        double v = x ? res[x][p] : 0.0;
+        if (a.perturbation ? x != 0 : x == 0) v += res[0][p];
+        out[t] = wx * v;
+    }
+}
+
+// V[r, v] = sum over the index entries of l-mer v of w[sv][r] times the entry's
+// window weight, R rows at once: a thread per (l-mer, row), so that an entry is
+// read once for its R lanes and its R weights are neighbours (R = 4: one 32-byte
+// sector).  With both strands indexed an l-mer and its reverse complement have the
+// same entries and are summed once (odd l: the one whose middle base is A or C, so
+// that every thread has work).  The RBF form of GkmExplain needs V of its own per
+// row; built once per row it costs one gather per index entry, where visiting the
+// buckets from every window costs windows x neighbours x entries per bucket (58,000
+// gathers a window at 72,000 SVs).  Bound by L2 sectors.  Measured (4 rows of 300 ..
+// 600 bp, 72,000 SVs): explain_windows over the buckets 4,318 us; a thread per l-mer
+// for its four rows, both strands, 527 us; this form 328 us.
+template <int R>
+__global__ void row_weights(const uint32_t *__restrict__ off, const uint32_t *__restrict__ ent,
+                            const uint16_t *__restrict__ ent16, int l, int strands, int tiles, int tile_svs, int weighted,
+                            const double *__restrict__ w, int rows, double *__restrict__ V)
+{
+    const int64_t n = (int64_t)1 << (2 * l), id = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    const int r = (int)(id % R);
+    int64_t v = id / R;
+    const bool half = strands == 2 && (l & 1);
+    if (v >= (half ? n / 2 : n)) return;
+    if (half) {  // skip the middle base's upper bit
+        const int64_t low = ((int64_t)2 << (l - 1)) - 1;
+        v = (v & low) | ((v & ~low) << 1);
+    }
+    const int64_t other = strands == 2 ? (int64_t)gkm_rc_word((uint32_t)v, l) : v;
+    if (other < v && !half) return;
+    double acc = 0.0;
+    for (int t = 0; t < tiles; t++) {
+        const uint32_t b = __ldg(off + t * n + v), e = __ldg(off + t * n + v + 1);
+        const double *wt = w + (int64_t)t * tile_svs * R + r;
+#pragma unroll 4
+        for (uint32_t k = b; k < e; k++) {
+            const uint32_t en = ent16 ? (uint32_t)__ldg(ent16 + k) | (1u << 24) : __ldg(ent + k);
+            const double x = __ldg(wt + (int64_t)R * (en & 0x00FFFFFFu));
+            acc += weighted ? x * (double)(en >> 24) : x;
+        }
+    }
+    if (r < rows) {
+        V[r * n + v] = acc;
+        V[r * n + other] = acc;
+    }
+}
+
 // out[b, base, p] = inv_dx[b] * sum over windows i covering p of part[b, i, base, p - i]
 // (nsplit > 1: part is [nsplit, B, W, 4, l], the splits added in order)
 __global__ void explain_gather(const double *__restrict__ part, const int32_t *__restrict__ cnt, int64_t B,
@@ -329,6 +497,75 @@ extern "C" int gkm_explain_lmer(const gkm_spec *spec, const uint32_t *fwd, const
     }
     cudaFreeAsync(part, st);
     return s;
+}
+
+extern "C" int gkm_index_row_weights(const gkm_index_t *ix, const double *w, int32_t width, int32_t rows, double *V,
+                                     gkm_stream_t stream)
+{
+    if (!ix || !w || !V) return gkm_fail(GKM_ERR_INVALID, "null argument");
+    if (width != 1 && width != 2 && width != 4) return gkm_fail(GKM_ERR_INVALID, "weights of 1, 2 or 4 rows, got %d", width);
+    if (rows < 1 || rows > width) return gkm_fail(GKM_ERR_INVALID, "%d of %d rows", rows, width);
+    const bool half = ix->strands == 2 && (ix->spec.l & 1);
+    const int64_t n = (half ? ix->n_lmers / 2 : ix->n_lmers) * width;
+    const unsigned grid = (unsigned)((n + 255) / 256);
+#define GKM_ROW_WEIGHTS(R)                                                                                     \
+    do {                                                                                                       \
+        GKM_PREFER_SHARED(row_weights<R>);                                                                     \
+        row_weights<R><<<grid, 256, 0, (cudaStream_t)stream>>>(ix->offsets, ix->ent, ix->ent16, ix->spec.l,    \
+                                                               ix->strands, ix->tiles, ix->tile_svs,           \
+                                                               ix->spec.weighted, w, rows, V);                 \
+    } while (0)
+    if (width == 1) GKM_ROW_WEIGHTS(1);
+    else if (width == 2) GKM_ROW_WEIGHTS(2);
+    else GKM_ROW_WEIGHTS(4);
+#undef GKM_ROW_WEIGHTS
+    GKM_CHECK_LAUNCH("row_weights");
+    return GKM_OK;
+}
+
+extern "C" int gkm_explain_subsets(const gkm_spec *spec, const uint32_t *fwd, const int32_t *counts, int64_t B, int64_t W,
+                                   int64_t L, const double *inv_dx, const double *V, int64_t v_stride,
+                                   const uint32_t *subsets, int32_t n_subsets, int32_t max_size, const uint16_t *lists,
+                                   const int32_t *n_with, const double *table_a, const double *table_b,
+                                   int32_t perturbation, double *part, double *out, gkm_stream_t stream)
+{
+    if (!spec || !fwd || !counts || !inv_dx || !V || !subsets || !lists || !n_with || !table_a || !table_b || !part || !out)
+        return gkm_fail(GKM_ERR_INVALID, "null argument");
+    if (spec->l < 1 || spec->l > LMAX) return gkm_fail(GKM_ERR_UNSUPPORTED, "GkmExplain l-mer path needs l <= %d", LMAX);
+    if (max_size < 0 || max_size > XS_MAX) return gkm_fail(GKM_ERR_UNSUPPORTED, "subsets of %d positions", max_size);
+    if (n_subsets < 1 || n_subsets > 4096) return gkm_fail(GKM_ERR_INVALID, "%d subsets", n_subsets);
+    if (B == 0 || W == 0 || L == 0) return GKM_OK;
+    if (B > 65535 || W > 0x7FFFFFFFLL) return gkm_fail(GKM_ERR_UNSUPPORTED, "too many rows or windows per launch");
+    cudaStream_t st = (cudaStream_t)stream;
+    SubsetArgs a = {};
+    a.fwd = fwd;
+    a.cnt = counts;
+    a.W = W;
+    a.l = spec->l;
+    a.V = V;
+    a.v_stride = v_stride;
+    a.weighted = spec->weighted;
+    a.wd = spec->wd;
+    a.subs = subsets;
+    a.lists = lists;
+    a.n_with = n_with;
+    a.n_sub = n_subsets;
+    a.ta = table_a;
+    a.tb = table_b;
+    a.perturbation = perturbation;
+    a.part = part;
+    const int stride = 1 + 3 * max_size;
+    const size_t smem = sizeof(double) * (size_t)n_subsets * stride;
+    if ((int64_t)smem > gkm_smem_limit() - 2048) return gkm_fail(GKM_ERR_UNSUPPORTED, "%d subsets do not fit", n_subsets);
+    cudaFuncSetAttribute(explain_subsets, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    GKM_PREFER_SHARED(explain_subsets);
+    explain_subsets<<<dim3((unsigned)W, (unsigned)B), XS_THREADS, smem, st>>>(a, stride);
+    GKM_CHECK_LAUNCH("explain_subsets");
+    const int64_t n = B * 4 * L;
+    GKM_PREFER_SHARED(explain_gather);
+    explain_gather<<<(unsigned)((n + 255) / 256), 256, 0, st>>>(part, counts, B, W, L, spec->l, inv_dx, out);
+    GKM_CHECK_LAUNCH("explain_gather");
+    return GKM_OK;
 }
 
 extern "C" int gkm_explain_pairs(const gkm_spec *spec, const uint32_t *fwd, const int32_t *counts, int64_t B,

@@ -23,7 +23,7 @@ import torch
 from . import engine
 from ._lib import call, ptr, stream_handle
 from .inputs import SeqBatch, allele_batches, device_codes, nan_rows, per_position
-from .kernels import INDEX_MAX_L, MAX_NEIGHBORS, RbfKernel, explain_tables, neighbor_count, neighbor_masks
+from .kernels import INDEX_MAX_L, MAX_NEIGHBORS, RbfKernel, explain_tables, neighbor_count, neighbor_masks, neighbor_subsets
 
 _MODE_ALIASES = {0: "importance", 1: "hypothetical", 2: "perturbation", "importance": "importance",
                  "hypothetical": "hypothetical", "perturbation": "perturbation"}
@@ -46,6 +46,46 @@ def _explain_masks(model, perturbation: bool, dev):
         c[key] = (torch.from_numpy(masks.view(np.int32).copy()).to(dev),
                   torch.from_numpy(a).to(dev), torch.from_numpy(b).to(dev))
     return c[key]
+
+
+# explain_subsets: at most this many mismatches (its register sums), and the
+# subsets that fit shared memory
+_SUBSET_MAX = 4
+_SUBSET_BYTES = 200 * 1024
+
+
+def _explain_subsets(model, perturbation: bool, dev):
+    """Device (subsets, lists, n_with), the largest subset's size, or None where
+    the neighbourhood is beyond explain_subsets."""
+    base = model.kernel.base
+    a, b, dmax = explain_tables(base, perturbation)
+    key = ("explain_subsets", perturbation)
+    c = model._sv_cache
+    if key not in c:
+        c[key] = None
+        if 0 <= dmax <= _SUBSET_MAX:
+            nonzero = tuple(bool(a[m] != 0 or b[m] != 0) for m in range(base.l + 1))
+            subs, lists, n_with = neighbor_subsets(base.l, nonzero, dmax)
+            if 8 * len(subs) * (1 + 3 * dmax) <= _SUBSET_BYTES:
+                c[key] = (torch.from_numpy(subs.view(np.int32).copy()).to(dev),
+                          torch.from_numpy(lists.view(np.int16).copy()).to(dev), torch.from_numpy(n_with).to(dev), dmax)
+    return c[key]
+
+
+# Seconds per bucket entry an RBF model's explain_windows visits from its windows,
+# and per index entry of a row_weights pass (four rows), measured on B200 at 72,000
+# SVs
+_BUCKET_VISIT_S = 4.1e-11
+_ROW_WEIGHTS_S = 5e-12
+# device memory of the rows' l-mer weights at a time
+_ROW_WEIGHTS_BYTES = 512 * 2**20
+
+
+def _row_weights_pay(model, index, n_windows: int, rows: int, n_masks: int) -> bool:
+    """Whether building each row's l-mer weights costs less than visiting the
+    buckets of its windows' neighbourhoods."""
+    visits = n_windows * n_masks * (index.entries / 4**model.kernel.base.l)
+    return visits * _BUCKET_VISIT_S > -(-rows // 4) * index.entries * _ROW_WEIGHTS_S + 4e-5
 
 
 def _explain_V(model) -> torch.Tensor:
@@ -102,9 +142,10 @@ def _explain_pair_tables(model, perturbation: bool, dev):
 
 
 # explain table limits and cost model ("auto"): build cost per entry of 4^l x l
-# and the direct l-mer path's cost per query window, measured on B200 at l=11
-# (a first call that builds V and the table: 0.17 s; the direct path: ~3e6
-# windows/s, the table ~3e7), so a call of ~300k windows pays for it
+# and the direct l-mer path's cost per query window with its launches, measured on
+# B200 at l=11 (a first call that builds V and the table: 0.17 s), so a call of ~300k
+# windows pays for it; the direct path of large calls has since become faster (45 ns
+# a window), but a built table serves later calls at 0.6 ns
 _EXPLAIN_TABLE_MAX_L = 12
 _EXPLAIN_TABLE_BYTES = 2 * 2**30
 _TABLE_BUILD_S_PER_ENTRY = 1e-9
@@ -199,8 +240,34 @@ def _explain_rows(model, x, lengths, mode, dev, table=None, check=True, work=Non
         w = w.contiguous()
     else:
         V = _explain_V(model)
+    masks = ta = tb = subsets = None
     if table is None and out is None:
         masks, ta, tb = _explain_masks(model, perturbation, dev)
+        subsets = _explain_subsets(model, perturbation, dev)
+        if index is not None and not _row_weights_pay(model, index, B * W, B, int(masks.numel())):
+            subsets = None
+    if subsets is not None:
+        subs, lists, n_with, size = subsets
+        n = 4**base.l
+        out = torch.empty((B, 4, L), dtype=torch.float64, device=dev)
+        step = B if V is not None else max(4, _ROW_WEIGHTS_BYTES // (8 * n) // 4 * 4)
+        part = torch.empty((min(B, step), W, 4, base.l), dtype=torch.float64, device=dev)
+        for s in range(0, B, step):
+            r = min(step, B - s)
+            if index is not None:
+                # (a captured pass: the workspace its K_raw rows are done with)
+                V = (torch.empty((r, n), dtype=torch.float64, device=dev) if work is None
+                     else work.get(8 * r * n, dev).view(torch.float64).view(r, n))
+                for g in range(0, r, 4):
+                    k = min(4, r - g)
+                    width = 4 if k == 3 else k
+                    ws = torch.zeros((index.S, width), dtype=torch.float64, device=dev)
+                    ws[:, :k] = w[s + g:s + g + k].T
+                    call("gkm_index_row_weights", index.handle, ptr(ws), width, k, ptr(V[g]), stream_handle())
+            call("gkm_explain_subsets", spec.ref, ptr(fwd[s]), ptr(counts[s:]), r, W, L, ptr(inv_dx[s:]), ptr(V),
+                 0 if index is None else n, ptr(subs), int(subs.numel()), size, ptr(lists), ptr(n_with), ptr(ta), ptr(tb),
+                 int(perturbation), ptr(part), ptr(out[s]), stream_handle())
+    elif table is None and out is None:
         out = torch.empty((B, 4, L), dtype=torch.float64, device=dev)
         call("gkm_explain_lmer", spec.ref, ptr(fwd), ptr(counts), B, W, L, ptr(inv_dx), ptr(V),
              None if index is None else index.handle, ptr(w), ptr(masks), int(masks.numel()), ptr(ta), ptr(tb),

@@ -153,6 +153,23 @@ def neighbor_masks(l: int, nonzero: tuple, dmax: int) -> np.ndarray:
     return np.array([x | (m << 24) for x, m in out], dtype=np.uint32)
 
 
+@lru_cache(maxsize=32)
+def neighbor_subsets(l: int, nonzero: tuple, dmax: int):
+    """The position subsets of neighbor_masks' masks, large ones first, packed
+    as positions (4 bits each) | size << 16 (uint32 [n]); per position the
+    subsets that hold it (subset | its place << 12), then those that do not
+    (uint16 [l, n]); how many hold it (int32 [l])."""
+    subs = [s for m in range(dmax, -1, -1) if nonzero[m] for s in combinations(range(l), m)]
+    packed = [sum(p << (4 * j) for j, p in enumerate(s)) | (len(s) << 16) for s in subs]
+    lists, n_with = [], []
+    for k in range(l):
+        held = [i | (s.index(k) << 12) for i, s in enumerate(subs) if k in s]
+        lists.append(held + [i for i, s in enumerate(subs) if k not in s])
+        n_with.append(len(held))
+    return (np.array(packed, dtype=np.uint32), np.array(lists, dtype=np.uint16).reshape(l, -1),
+            np.array(n_with, dtype=np.int32))
+
+
 def window_weight_table(M: int, H: float, n: int = 65537) -> np.ndarray:
     """[n] uint8 window weight by distance |W//2 - i| from the centre, with the
     reference's expression (kernels/weighted.py:38-43), so every weight is

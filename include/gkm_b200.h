@@ -290,6 +290,26 @@ int gkm_explain_lmer(const gkm_spec *spec, const uint32_t *fwd, const int32_t *c
                      const double *table_b, int32_t perturbation, double *out,
                      gkm_stream_t stream);
 
+/* V[r, v] [rows, 4^l] = sum over index entries of l-mer v of w[sv, r] times the
+ * entry's window weight; w [S, width], width 1, 2 or 4, rows <= width.  The l-mer
+ * weights of gkm_explain_subsets for rows with SV weights of their own (RBF).
+ * Replaces the bucket sums of _explain_index_cpu (explain/cpu.py:140-207). */
+int gkm_index_row_weights(const gkm_index_t *index, const double *w, int32_t width, int32_t rows, double *V,
+                          gkm_stream_t stream);
+
+/* gkm_explain_lmer's attributions from l-mer weights V [4^l] (v_stride 0) or
+ * [B, 4^l] (v_stride 4^l), for neighbourhoods of at most four mismatches:
+ * subsets [n_subsets] the position subsets (4 bits per position, the size in
+ * bits 16..) of every contributing level, lists [l, n_subsets] for each position
+ * the subsets that hold it (subset | its place in it << 12) and then those that
+ * do not, n_with [l] how many hold it.  part [B, W, 4, l] scratch.
+ * Replaces _explain_lmer_cpu (explain/cpu.py:69-139). */
+int gkm_explain_subsets(const gkm_spec *spec, const uint32_t *fwd, const int32_t *counts, int64_t B, int64_t W,
+                        int64_t L, const double *inv_dx, const double *V, int64_t v_stride,
+                        const uint32_t *subsets, int32_t n_subsets, int32_t max_size, const uint16_t *lists,
+                        const int32_t *n_with, const double *table_a, const double *table_b,
+                        int32_t perturbation, double *part, double *out, gkm_stream_t stream);
+
 /* GkmExplain by the per-SV pair loop, for models the l-mer path does not take
  * (l > 12, a neighbourhood larger than the SVs, no l-mer index): every query
  * window against every SV window by (SV s) forward and, with include_rc, RC
