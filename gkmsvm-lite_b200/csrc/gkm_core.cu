@@ -8,6 +8,8 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include <type_traits>
+
 #include "gkm_common.cuh"
 
 namespace {
@@ -618,6 +620,195 @@ __global__ void __launch_bounds__(MUT_THREADS) mutant_kernel(
     }
 }
 
+// The same for kernels of at most four levels, by bit-sliced diagonals: a block
+// takes MT_WINDOWS - l + 1 positions of a row and the windows that cover them.  Only
+// pairs within dmax + 1 mismatches can count after a substitution (~1 % of them), so
+// those are found 32 pairs at a time as in self_kernel -- every diagonal of the
+// tile's windows against the row and against its reverse complement -- queued per
+// warp and taken one per lane: the pair's l positions add to the counts of (position,
+// base, level).  Pairs whose second window covers the position, too, are the l x l
+// ones about it and are tested directly.  Bound by the integer pipe.  Measured (t=2,
+// 128 x 300 bp): mutant_kernel, every pair at every position, 685 us; this 76 us.
+// mutant_kernel stays for d >= 4 and for rows whose planes outgrow shared memory.
+constexpr int MT_THREADS = 256;
+constexpr int MT_WINDOWS = 128;
+
+// words of one plane: pw zeros, the row's pw, and what the last windows' partners
+// read past them (a tile's words and two more)
+__host__ __device__ inline int mutant_plane(int pw) { return 2 * pw + MT_WINDOWS / 32 + 4; }
+
+template <int L, bool WT>
+__global__ void __launch_bounds__(MT_THREADS) mutant_tiles(
+    gkm_spec spec, const uint32_t *__restrict__ fwd, const int32_t *__restrict__ counts, int64_t B,
+    int64_t W, int64_t len, const double *__restrict__ diag, double *__restrict__ mut_diag,
+    const double *__restrict__ table, const double *__restrict__ ref_raw, int normalize,
+    double *__restrict__ ism_out, int pw)
+{
+    typedef typename std::conditional<WT, unsigned long long, uint32_t>::type Acc;
+    // x0, x1, y0, y1: pw words of zeros, then the row's (and zeros past it)
+    extern __shared__ uint32_t pl[];
+    const int ps = mutant_plane(pw);
+    __shared__ Acc acc[MT_WINDOWS][4][4];  // position, base, level
+    __shared__ uint32_t queue[MT_THREADS / 32][64];
+    const int l = L ? L : spec.l, P = MT_WINDOWS - l + 1, D = spec.dmax;
+    const int64_t b = blockIdx.y;
+    const int n = counts[b], p0 = (int)(blockIdx.x * P), np = (int)min((int64_t)P, len - p0);
+    const int i0 = max(0, p0 - l + 1), i1 = min(n, p0 + np);  // the windows that cover the tile's positions
+    const double d0 = diag ? diag[b] : 0.0;
+    if (i0 >= i1) {  // past the row's windows: nothing changes
+        for (int t = threadIdx.x; t < 4 * np; t += MT_THREADS) {
+            const int v = t / np, p = p0 + t - v * np;
+            if (mut_diag) mut_diag[((int64_t)v * len + p) * B + b] = d0;
+            if (ism_out) ism_out[(b * 4 + v) * len + p] = 0.0;
+        }
+        return;
+    }
+    const uint32_t *F = fwd + b * W;
+    const bool has_rc = spec.include_rc != 0;
+    const uint8_t *wd = spec.wd;
+    for (int t = threadIdx.x; t < MT_WINDOWS * 16; t += MT_THREADS) (&acc[0][0][0])[t] = 0;
+    if (diag || mut_diag) {
+        const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+        for (int t = threadIdx.x; t < 4 * pw; t += MT_THREADS) pl[(t / pw) * ps + t % pw] = 0;
+        {
+            const int nb = n + l - 1;
+            auto base = [&](int p) -> uint32_t { return p < n ? F[p] & 3u : (F[n - 1] >> (2 * (p - n + 1))) & 3u; };
+            for (int k = warp; k < ps - pw; k += MT_THREADS / 32) {
+                const int p = k * 32 + lane;
+                const uint32_t x = p < nb ? base(p) : 0u, y = p < nb ? 3u - base(nb - 1 - p) : 0u;
+                const uint32_t x0 = __ballot_sync(GKM_FULL, x & 1u), x1 = __ballot_sync(GKM_FULL, x & 2u);
+                const uint32_t y0 = __ballot_sync(GKM_FULL, y & 1u), y1 = __ballot_sync(GKM_FULL, y & 2u);
+                if (lane == 0) {
+                    pl[pw + k] = x0;
+                    pl[ps + pw + k] = x1;
+                    pl[2 * ps + pw + k] = y0;
+                    pl[3 * ps + pw + k] = y1;
+                }
+            }
+        }
+        __syncthreads();
+        int nq = 0;  // queued pairs of this warp: window - i0 | RC << 8 | other window << 9
+        auto take = [&](int c) {
+            __syncwarp();
+            if (lane < c) {
+                const uint32_t e = queue[warp][lane];
+                const int i = i0 + (int)(e & 0xFFu), j = (int)(e >> 9);
+                const uint32_t fi = F[i], g = (e >> 8) & 1u ? gkm_rc_word(F[j], l) : F[j];
+                const uint32_t x = fi ^ g, differ = (x | (x >> 1)) & 0x55555555u;
+                const int m = __popc(differ);
+                const Acc w = WT ? (Acc)2 * gkm_wt(wd, n, i) * gkm_wt(wd, n, j) : (Acc)2;
+                for (int k = 0; k < l; k++) {
+                    const int p = i + k - p0, me = m - (int)((differ >> (2 * k)) & 1u);
+                    // me: mismatches away from p; a position j covers, too, is left to the pairs below
+                    if (me > D || p < 0 || p >= np || (unsigned)(i + k - j) < (unsigned)l) continue;
+                    const uint32_t same = (g >> (2 * k)) & 3u;
+                    atomicAdd(&acc[p][same][me], w);
+                    if (me < D)
+#pragma unroll
+                        for (uint32_t v = 0; v < 4; v++)
+                            if (v != same) atomicAdd(&acc[p][v][me + 1], w);
+                }
+            }
+            __syncwarp();
+            if (c == 32 && lane < nq - 32) queue[warp][lane] = queue[warp][32 + lane];
+            __syncwarp();
+            nq -= c;
+        };
+        // diagonals: shift s of the row (strand 0) and of its reverse complement (1)
+        const int nd = 2 * n - 1, nt = has_rc ? 2 * nd : nd, nwd = (i1 - i0 + 31) >> 5;
+        for (int t0 = 0; t0 < nt; t0 += MT_THREADS) {
+            const int t = t0 + threadIdx.x, st = t >= nd, s = t - st * nd - (n - 1);
+            // windows whose partner is one of the row's
+            const int lo = max(i0, -s), hi = min(i1, n - s);
+            const bool live = t < nt && (st || s != 0) && lo < hi;
+            // bit of the first window's partner, after the zeros: within n - 1 before
+            // and MT_WINDOWS after the row's bits
+            const int at = live ? pw * 32 + i0 + s : pw * 32;
+            const uint32_t *X = pl + pw + (i0 >> 5), *Q = pl + (live && st ? 2 * ps : 0) + (at >> 5);
+            auto differ = [&](int w) -> uint32_t {
+                const uint32_t x0 = __funnelshift_r(X[w], X[w + 1], i0), x1 = __funnelshift_r(X[ps + w], X[ps + w + 1], i0);
+                const uint32_t q0 = __funnelshift_r(Q[w], Q[w + 1], at), q1 = __funnelshift_r(Q[ps + w], Q[ps + w + 1], at);
+                return (x0 ^ q0) | (x1 ^ q1);
+            };
+            uint32_t e = differ(0);
+            for (int w = 0; w < nwd; w++) {
+                const uint32_t en = differ(w + 1);
+                const Planes pn = mismatch_planes<L>(e, en, l);
+                e = en;
+                const int a0 = max(lo - i0 - 32 * w, 0), a1 = min(hi - i0 - 32 * w, 32);
+                uint32_t h = live && a1 > a0 ? (a1 < 32 ? (1u << a1) - 1u : GKM_FULL) & ~((1u << a0) - 1u) : 0u;
+                // at most D + 1 <= 4 mismatches
+                uint32_t near = ~pn.v[3] & (~pn.v[2] | (~pn.v[0] & ~pn.v[1]));  // <= 4
+                if (D < 3) near &= ~pn.v[2] & (D == 2 ? GKM_FULL : D == 1 ? ~(pn.v[0] & pn.v[1]) : ~pn.v[1]);
+                h &= near;
+                while (__any_sync(GKM_FULL, h != 0)) {
+                    const uint32_t who = __ballot_sync(GKM_FULL, h != 0);
+                    if (h) {
+                        const int i = 32 * w + __ffs(h) - 1, q = i0 + i + s, j = st ? n - 1 - q : q;
+                        queue[warp][nq + __popc(who & ((1u << lane) - 1u))] = (uint32_t)i | (uint32_t)st << 8 | (uint32_t)j << 9;
+                        h &= h - 1;
+                    }
+                    nq += __popc(who);
+                    if (nq >= 32) take(32);
+                }
+            }
+        }
+        if (nq) take(nq);
+        __syncthreads();
+        // both windows cover the position: windows a_s .. a_e - 1, unordered pairs
+        // twice (a window with itself has no mismatch whatever the base)
+        for (int t = threadIdx.x; t < 4 * np; t += MT_THREADS) {
+            const int v = t & 3, p = p0 + (t >> 2), as = max(0, p - l + 1), ae = min(n, p + 1);
+            for (int i = as; i < ae; i++) {
+                const uint32_t sh = 2u * (uint32_t)(p - i), fi = (F[i] & ~(3u << sh)) | (uint32_t)v << sh;
+                const uint32_t wi = WT ? gkm_wt(wd, n, i) : 1u;
+                for (int j = i; j < ae; j++) {
+                    const uint32_t shj = 2u * (uint32_t)(p - j), fj = (F[j] & ~(3u << shj)) | (uint32_t)v << shj;
+                    const Acc w = (Acc)(i == j ? 1u : 2u) * wi * (WT ? gkm_wt(wd, n, j) : 1u);
+                    const int mf = gkm_mism(fi, fj);
+                    if (mf <= D) acc[p - p0][v][mf] += w;
+                    if (has_rc) {
+                        const int mr = gkm_mism(fi, gkm_rc_word(fj, l));
+                        if (mr <= D) acc[p - p0][v][mr] += w;
+                    }
+                }
+            }
+        }
+    }
+    __syncthreads();
+    for (int t = threadIdx.x; t < 4 * np; t += MT_THREADS) {
+        const int v = t / np, q = t - v * np, p = p0 + q;
+        const int as = max(0, p - l + 1), ae = min(n, p + 1);
+        const bool none = as >= ae;
+        const int xp = none ? v : (int)((F[as] >> (2 * (p - as))) & 3u);  // the row's base at p
+        double md = d0;
+        if (diag || mut_diag) {
+            double delta = 0.0;
+            for (int m = 0; m < 4 && m <= D; m++)
+                delta += spec.h[m] * (double)((int64_t)acc[q][v][m] - (int64_t)acc[q][xp][m]);
+            md = d0 + delta;
+            if (mut_diag) mut_diag[((int64_t)v * len + p) * B + b] = md;
+        }
+        if (ism_out) {
+            double out = 0.0;
+            if (!none) {
+                const double r = ref_raw[b];
+                double dt = 0.0;
+                if (v != xp)
+                    for (int i = as; i < ae; i++) {
+                        const uint32_t fi = F[i], sh = 2u * (uint32_t)(p - i);
+                        const uint32_t fn = (fi & ~(3u << sh)) | ((uint32_t)v << sh);
+                        const double a = WT ? (double)gkm_wt(wd, n, i) : 1.0;
+                        dt += a * (table[fn] - table[fi]);
+                    }
+                const double kn = r + dt;
+                out = normalize ? kn / sqrt(fmax(md, 1e-10)) - r / sqrt(fmax(d0, 1e-10)) : kn - r;
+            }
+            ism_out[(b * 4 + v) * len + p] = out;
+        }
+    }
+}
+
 // ---------------------------------------------------------------------------
 // Dense FP64 epilogues over materialised [rows, S] blocks
 // ---------------------------------------------------------------------------
@@ -852,6 +1043,29 @@ static int mutant_launch(const gkm_spec *spec, const uint32_t *fwd, const int32_
 {
     if (B == 0 || L == 0) return GKM_OK;
     if (B > 65535) return gkm_fail(GKM_ERR_UNSUPPORTED, "more than 65,535 rows per ISM launch");
+    // four levels, and rows whose bit planes fit shared memory: by diagonals
+    const int pw = plane_words(W, spec->l) + 1;
+    const size_t planes = (size_t)4 * mutant_plane(pw) * sizeof(uint32_t);
+    if (spec->dmax < 4 && planes <= 128 * 1024) {
+        const int P = MT_WINDOWS - spec->l + 1;
+        const dim3 grid((unsigned)((L + P - 1) / P), (unsigned)B);
+#define GKM_MUT_AS(LT, WT)                                                                                     \
+    do {                                                                                                       \
+        cudaFuncSetAttribute(mutant_tiles<LT, WT>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)planes);  \
+        GKM_PREFER_SHARED((mutant_tiles<LT, WT>));                                                             \
+        mutant_tiles<LT, WT><<<grid, MT_THREADS, planes, st>>>(*spec, fwd, counts, B, W, L, diag, mut_diag,    \
+                                                               table, ref_raw, normalize, out, pw);            \
+    } while (0)
+        if (spec->l == 11 && spec->weighted) GKM_MUT_AS(11, true);
+        else if (spec->l == 11) GKM_MUT_AS(11, false);
+        else if (spec->l == 10 && spec->weighted) GKM_MUT_AS(10, true);
+        else if (spec->l == 10) GKM_MUT_AS(10, false);
+        else if (spec->weighted) GKM_MUT_AS(0, true);
+        else GKM_MUT_AS(0, false);
+#undef GKM_MUT_AS
+        GKM_CHECK_LAUNCH("mutant_tiles");
+        return GKM_OK;
+    }
     const int sw = staged_windows(W);
     size_t smem = (size_t)2 * sw * sizeof(uint32_t);
     dim3 grid((unsigned)L, (unsigned)B);
@@ -863,7 +1077,7 @@ static int mutant_launch(const gkm_spec *spec, const uint32_t *fwd, const int32_
         mutant_kernel<NW><<<grid, MUT_THREADS, smem, st>>>(*spec, fwd, counts, B, W, L, diag, mut_diag,  \
                                                            table, ref_raw, normalize, out, sw);          \
     } while (0)
-    if (nw == 1) GKM_MUT(1);
+    if (nw == 1) GKM_MUT(1);  // (rows too long for mutant_tiles' planes)
     else if (nw == 2) GKM_MUT(2);
     else GKM_MUT(4);
 #undef GKM_MUT
