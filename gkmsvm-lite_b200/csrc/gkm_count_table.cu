@@ -17,13 +17,13 @@
 // and a table row read serves every query of the group: at 72,000 SVs and 300 bp
 // rows an index walk visits 16.7M entries per query by shared-memory atomics,
 // the gather reads 24.5M / 32 rows of 64 bytes.  Measured against the walk (with
-// its query self-kernels): 1,000 x 300 bp, t=3: 43.5 -> 9.2 ms; 2,048 rows of 50 ..
-// 2,000 bp: 135 -> 20.9 ms; 512 of them, weighted t=5: 77.8 -> 9.6 ms; one 300 bp
+// its query self-kernels): 1,000 x 300 bp, t=3: 43.5 -> 8.6 ms; 2,048 rows of 50 ..
+// 2,000 bp: 135 -> 20.4 ms; 512 of them, weighted t=5: 77.8 -> 8.4 ms; one 300 bp
 // row: 1.3 -> 0.2 ms.
 //
 // Entries are exact.  Unweighted entries take 16 bits (5, 4, 4 and 3 for levels
-// dmax, dmax - 1, ...: t = dmax - m indexes the fields), weighted ones four bytes,
-// one per level.  They are counted in shared memory in fields of those widths
+// dmax, dmax - 1, ...: t = dmax - m indexes the fields), weighted ones and those of
+// long unweighted rows (weights of 1) four bytes, one per level.  They are counted in shared memory in fields of those widths
 // (weighted: 9 / 8 / 8 / 7 bits).  A weighted count past its byte is clipped and
 // the excess added to the (SV, query) counts of that l-mer's SVs through the
 // index's buckets (spill_excess: C and its dirty bits, read back by the gather).
@@ -40,29 +40,42 @@
 
 namespace {
 
-constexpr int CT_ROWS = 4096;     // table rows per tile: six of the l-mer's positions
-constexpr int CT_THREADS = 1024;
+constexpr int CT_POS = 5;          // positions of a tile's suffix
+constexpr int CT_ROWS = 1 << (2 * CT_POS);  // table rows per tile
+constexpr int CT_THREADS = 512;
 constexpr int CT_WARPS = CT_THREADS / 32;
-constexpr int CT_SLOTS = 8;       // counter words per table row a block holds (128 KB)
-constexpr int CT_LIST = 512;      // entries of a tile a block queues for a second look
-constexpr int CT_RECS = 12288;    // window records of a pass a block keeps in shared memory
+constexpr int CT_BLOCKS = 2;      // count_tiles blocks per SM
+constexpr int CT_SLOTS = 16;      // counter words per table row a block holds (64 KB)
+constexpr int CT_LIST = 256;      // entries of a tile a block queues for a second look
+constexpr int CB_THREADS = 1024;  // ct_buckets
+constexpr int CT_PRE = 4096;      // most values of the other positions
 constexpr int64_t CT_EXC = 4096;   // clipped counts a group queues, per query (weighted)
 // unweighted counter halves (and entries): fields of 5 / 4 / 4 / 3 bits for t = 0
 // .. 3, placed so that two byte dot products sum all of them
 constexpr uint32_t CT_F0 = 0, CT_F1 = 8, CT_F2 = 12, CT_F3 = 5;
-constexpr int CT_R2 = 6, CT_R3 = 26;  // rounds of 32 lanes over the 154 / 694 neighbour masks of budgets 2 / 3
-constexpr int CT_BALL = 376;      // masks of up to five positions within three mismatches
+constexpr int CT_R2 = 4, CT_R3 = 20;  // rounds of 32 lanes over the 106 / 376 neighbour masks of budgets 2 / 3
+constexpr int CT_ROUNDS = 1 + CT_R2 + CT_R3;
+constexpr int CT_BALL = 694;      // masks of up to six positions within three mismatches
+constexpr int CT_LIST1 = 112, CT_LIST2 = 32;  // windows of budgets 1 and 2 a warp lists at a time
 constexpr int G_THREADS = 128;
 constexpr int G_BLOCKS = 4, G_BLOCKS_W = 6;   // gather blocks per SM, unweighted / weighted
 
-// Shared-memory position of the table row with suffix s (12 bits): a linear
-// bijection, its own inverse, chosen so that the masks of a budget spread evenly
-// over the 32 banks: lane b takes the masks of bank class b, so a warp's adds
-// around any one window hit 32 different banks.
-__host__ __device__ __forceinline__ uint32_t ct_phys(uint32_t s)
+// Shared-memory position of the table row with suffix s (10 bits): a linear
+// bijection, its own inverse, chosen so that the 16 masks of budget 1 lie on 16 of
+// the 32 banks, the 106 of budget 2 on all of them (at most 4 on one) and the 376 of
+// budget 3 at most 20 on one: lane b takes the masks of bank class b, so a warp's
+// adds around any one window hit different banks.
+__host__ __device__ constexpr __forceinline__ uint32_t ct_phys(uint32_t s)
 {
-    const uint32_t h = s >> 5;
-    return s ^ ((h ^ (h << 2) ^ (h >> 3)) & 31u);
+    return s ^ (((s >> 5) & 1u ? 15u : 0u) ^ ((s >> 6) & 1u ? 20u : 0u) ^ ((s >> 7) & 1u ? 10u : 0u) ^
+                ((s >> 8) & 1u ? 18u : 0u) ^ ((s >> 9) & 1u ? 5u : 0u));
+}
+
+// Counter plane j keeps its positions with bits 3 and 4 exchanged by its quarter, so
+// that the four lanes that write a table row's quarters read different banks.
+__device__ __forceinline__ uint32_t ct_swap(uint32_t plane)
+{
+    return (plane >> 2) << 3;
 }
 
 struct CtShape {
@@ -99,12 +112,11 @@ struct CtArgs {
     int nball[4];           // how many of each
     // windows of the call's rows by the bases outside the suffix (ct_buckets):
     // records [pass][rec_cap], bucket offsets [pass][n_pre + 1]
-    uint32_t *recs;
+    uint8_t *recs;
     uint32_t *roff;
     int64_t rec_cap;
     int n_pre;
     int pass0;  // pass of the group's first row
-    int words, rec_smem;  // count_tiles' counter words per row and staged records
     uint8_t *T;
     unsigned long long *exc;  // [cap_exc] clipped counts of the group: row | q << 22 | excess << 32
     unsigned int *nexc;       // how many (past cap_exc: added at once)
@@ -126,6 +138,7 @@ struct CtArgs {
     const uint32_t *goff;  // [S + 1] in gather order
     const uint32_t *perm;  // gather order: SVs by falling window count
     int64_t S;
+    int split;             // lane groups that share an SV's windows
     double h[4];           // by t
     int normalize;
     const double *inv_dx;  // [B] by row, or null: from self
@@ -169,7 +182,7 @@ __device__ void ct_excess(const CtArgs &a, uint32_t v, int q, const uint64_t *ex
             if (pal && ((k - b) & 1u)) continue;
             const uint32_t en = a.ent16 ? (uint32_t)a.ent16[k] | (1u << 24) : a.ent[k];
             const int64_t s = (int64_t)t * a.tile_svs + (en & 0x00FFFFFFu);
-            const uint64_t w = WT ? en >> 24 : 1;
+            const uint64_t w = WT && a.wd ? en >> 24 : 1;
             const int64_t at = s * a.qg + q;
             const unsigned long long c0 = w * ex[0] | (w * ex[1]) << 32, c1 = w * ex[2] | (w * ex[3]) << 32;
             if (c0) atomicAdd(a.C + 2 * at, c0);
@@ -179,10 +192,20 @@ __device__ void ct_excess(const CtArgs &a, uint32_t v, int q, const uint64_t *ex
     }
 }
 
-// plain add to shared memory (byte address), no value returned
-__device__ __forceinline__ void ct_add(uint32_t addr, uint32_t v)
+__device__ __forceinline__ void ct_fa(uint32_t &s, uint32_t &c, uint32_t a, uint32_t b)
 {
-    asm volatile("red.shared.add.u32 [%0], %1;" ::"r"(addr), "r"(v) : "memory");
+    const uint32_t x = s;
+    s = x ^ a ^ b;
+    c = (x & a) | (x & b) | (a & b);
+}
+
+// plain add to shared memory (byte address) where a < b, no value returned;
+// predicated rather than branched around
+__device__ __forceinline__ void ct_add(uint32_t a, uint32_t b, uint32_t addr, uint32_t v)
+{
+    asm volatile("{\n\t.reg .pred p;\n\tsetp.lt.u32 p, %0, %1;\n\t@p red.shared.add.u32 [%2], %3;\n\t}" ::"r"(a), "r"(b),
+                 "r"(addr), "r"(v)
+                 : "memory");
 }
 
 template <bool WT>
@@ -191,48 +214,54 @@ __host__ __device__ __forceinline__ uint32_t ct_shift(uint32_t t)
     return WT ? (t ? 8u * t + 1u : 0u) : t == 0 ? CT_F0 : t == 1 ? CT_F1 : t == 2 ? CT_F2 : CT_F3;
 }
 
-// Counter index (plane of the query, position of the suffix), half and weight of
-// a window: how ct_buckets hands it to count_tiles.
-//   bits 0..14 counter index, 15 upper half, 16.. weight
+// How ct_buckets hands a window to count_tiles: its counter (plane of the query,
+// position of the suffix) and above its 14 bits its weight or (unweighted: 16 bits)
+// the query's half of the word.
 template <bool WT>
-__device__ __forceinline__ uint32_t ct_record(const CtShape &sh, uint32_t v, int q, uint32_t w, uint32_t *pre)
+using ct_rec = std::conditional_t<WT, uint32_t, uint16_t>;
+
+template <bool WT>
+__device__ __forceinline__ ct_rec<WT> ct_record(const CtShape &sh, uint32_t v, int q, uint32_t w, uint32_t *pre)
 {
     uint32_t c = v;  // the l-mer without its middle base, which goes on top (fold)
     if (sh.fold) {
         const uint32_t low = (1u << (2 * sh.mid)) - 1u;
         c = (v & low) | ((v >> 2) & ~low & ((1u << (2 * (sh.l - 1))) - 1u)) | (((v >> (2 * sh.mid)) & 3u) << (2 * (sh.l - 1)));
     }
-    *pre = c >> 12;
+    *pre = c >> (2 * CT_POS);
     const uint32_t plane = WT ? (uint32_t)q : (uint32_t)q >> 1;
-    return plane * CT_ROWS + ct_phys(c & 0xFFFu) | (WT ? 0u : (uint32_t)(q & 1) << 15) | w << 16;
+    return (ct_rec<WT>)(plane * CT_ROWS + (ct_phys(c & (CT_ROWS - 1u)) ^ ct_swap(plane)) | (WT ? w : (uint32_t)(q & 1)) << 14);
 }
 
 // One block per pass of queries: their windows (both strands) sorted by the
-// bases outside the six suffix positions (counting sort in shared memory), so
+// bases outside the suffix (counting sort in shared memory), so
 // that a tile visits the buckets within D mismatches of it and tests nothing.
 template <bool WT>
-__global__ void __launch_bounds__(CT_THREADS) ct_buckets(CtArgs a, int64_t B)
+__global__ void __launch_bounds__(CB_THREADS) ct_buckets(CtArgs a, int64_t B)
 {
     constexpr int PASS = WT ? CT_SLOTS : 2 * CT_SLOTS;
-    __shared__ uint32_t hist[1024], wtot[32];
+    constexpr int EACH = CT_PRE / CB_THREADS;
+    __shared__ __align__(16) uint32_t hist[CT_PRE];
+    __shared__ uint32_t wtot[32];
     const int64_t pass = a.pass0 + blockIdx.x;
     const int64_t q0 = pass * PASS;
     const int nq = (int)min((int64_t)PASS, B - q0);
-    uint32_t *recs = a.recs + (int64_t)blockIdx.x * a.rec_cap, *roff = a.roff + (int64_t)blockIdx.x * (a.n_pre + 1);
+    ct_rec<WT> *recs = (ct_rec<WT> *)a.recs + (int64_t)blockIdx.x * a.rec_cap;
+    uint32_t *roff = a.roff + (int64_t)blockIdx.x * (a.n_pre + 1);
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    hist[threadIdx.x] = 0;
+    ((uint4 *)hist)[threadIdx.x] = make_uint4(0, 0, 0, 0);
     __syncthreads();
     for (int phase = 0; phase < 2; phase++) {
-        for (int q = warp; q < nq * 4; q += CT_WARPS) {  // four warps a row
+        for (int q = warp; q < nq * 4; q += CB_THREADS / 32) {  // four warps a row
             const int64_t r = a.order ? (int64_t)a.order[q0 + (q >> 2)] : q0 + (q >> 2);
             const int n = a.cx[r];
             for (int i = (q & 3) * 32 + lane; i < n; i += 128) {
                 uint32_t v = __ldg(a.bx + r * a.W + i);
-                const uint32_t w = WT ? gkm_wt(a.wd, n, i) : 1u;
+                const uint32_t w = WT && a.wd ? gkm_wt(a.wd, n, i) : 1u;
                 for (int st = 0; st < a.sh.strands; st++) {
                     if (st) v = gkm_rc_word(v, a.sh.l);
                     uint32_t pre;
-                    const uint32_t rec = ct_record<WT>(a.sh, v, q >> 2, w, &pre);
+                    const ct_rec<WT> rec = ct_record<WT>(a.sh, v, q >> 2, w, &pre);
                     const uint32_t at = atomicAdd(&hist[pre], 1u);
                     if (phase) recs[at] = rec;
                 }
@@ -240,9 +269,11 @@ __global__ void __launch_bounds__(CT_THREADS) ct_buckets(CtArgs a, int64_t B)
         }
         __syncthreads();
         if (phase) break;
-        // exclusive scan: the buckets' first records
-        const uint32_t c = hist[threadIdx.x];
-        uint32_t x = c;
+        // exclusive scan: the buckets' first records (four neighbours a thread)
+        const uint4 c = ((const uint4 *)hist)[threadIdx.x];
+        static_assert(EACH == 4, "four buckets a thread");
+        const uint32_t own = c.x + c.y + c.z + c.w;
+        uint32_t x = own;
 #pragma unroll
         for (int o = 1; o < 32; o <<= 1) {
             const uint32_t y = __shfl_up_sync(GKM_FULL, x, o);
@@ -260,42 +291,57 @@ __global__ void __launch_bounds__(CT_THREADS) ct_buckets(CtArgs a, int64_t B)
             wtot[lane] = t;
         }
         __syncthreads();
-        x = x - c + (warp ? wtot[warp - 1] : 0u);
-        hist[threadIdx.x] = x;
-        if ((int)threadIdx.x < a.n_pre) roff[threadIdx.x] = x;
-        if ((int)threadIdx.x == a.n_pre - 1) roff[a.n_pre] = x + c;
+        x = x - own + (warp ? wtot[warp - 1] : 0u);
+        const uint32_t first[EACH + 1] = {x, x + c.x, x + c.x + c.y, x + c.x + c.y + c.z, x + own};
+#pragma unroll
+        for (int k = 0; k < EACH; k++) {
+            const int pre = threadIdx.x * EACH + k;
+            hist[pre] = first[k];
+            if (pre < a.n_pre) roff[pre] = first[k];
+            if (pre == a.n_pre - 1) roff[a.n_pre] = first[k + 1];
+        }
         __syncthreads();
     }
 }
 
 // Items of (tile, pass of queries): a tile is the l-mers that agree outside the
-// six suffix positions.  Windows whose other positions differ from the tile's at
+// five suffix positions.  Windows whose other positions differ from the tile's at
 // dp <= D places reach the suffixes within budget D - dp of their own: one row
-// (budget 0), 19, 154 or 694.  Warps take buckets of windows of one budget:
-// budgets 0 and 1 a window per lane, budgets 2 and 3 a window per warp with a
-// lane on each bank (no two of its adds conflict).
+// (budget 0), 16, 106 or 376.  Their buckets are dealt to the warps; a warp copies
+// its buckets of budgets 1 and 2 to a list (they hold a few windows each) and adds a
+// window at a time with a lane on each bank (no two of its adds conflict), two of
+// budget 1.  Budget 0 is a bucket per lane.
 //
 // Shared counters: unweighted, one word per two queries (fields: CT_F0 ..);
 // weighted, one word per query with 9 / 8 / 8 / 7 bits (entry: a byte each).
+//
+// Bound by instruction issue and the latency of the short chains between barriers.  A
+// pass holds the 64 bytes of 32 unweighted (16 weighted) queries, so that rows are
+// written 64 bytes at a time, and two blocks share an SM, so that one counts while the
+// other writes.  Tiles of six positions and passes of half as many queries, one block
+// of 1,024 threads per SM, a window per lane for budget 1: 110 us a group of 32 x 300
+// bp, this 88 us (weighted: 268 and 190).
 template <bool WT>
-__global__ void __launch_bounds__(CT_THREADS, 1) count_tiles(CtArgs a)
+__global__ void __launch_bounds__(CT_THREADS, CT_BLOCKS) count_tiles(CtArgs a)
 {
     constexpr int PASS = WT ? CT_SLOTS : 2 * CT_SLOTS;
     extern __shared__ __align__(16) uint8_t ct_smem[];
     __shared__ uint2 l3[CT_R3 * 32];
-    __shared__ uint32_t off_s[1025];
     __shared__ uint16_t ball_s[CT_BALL];
+    constexpr int LIST = CT_LIST1 + 8 + CT_LIST2;  // (eight more of budget 1 are read)
+    __shared__ uint32_t list_s[CT_WARPS * LIST];
     // by tile parity: the entries that need a second look, and the fields' sum and
     // the adds made
     __shared__ uint16_t list_at[2][CT_LIST];
     __shared__ uint32_t list_w[2][CT_LIST];
     __shared__ int nlist[2];
-    __shared__ unsigned long long chk[2][2];
+    __shared__ uint32_t chk[2][2];
     // counters [words][CT_ROWS], aligned to a word's plane so that a neighbour's
     // address is an exclusive or
-    const uint32_t raw0 = (uint32_t)__cvta_generic_to_shared(ct_smem), cbase = (raw0 + 16383u) & ~16383u;
+    constexpr uint32_t PLANE = 4 * CT_ROWS;
+    const uint32_t raw0 = (uint32_t)__cvta_generic_to_shared(ct_smem), cbase = (raw0 + PLANE - 1u) & ~(PLANE - 1u);
     uint32_t *cnt = (uint32_t *)(ct_smem + (cbase - raw0));
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int lane = threadIdx.x & 31, warp = __shfl_sync(GKM_FULL, threadIdx.x >> 5, 0);  // (known to be uniform)
     const CtShape sh = a.sh;
     const int D = sh.D;
     // a mask: byte offset and increment (0: none in this round)
@@ -303,28 +349,27 @@ __global__ void __launch_bounds__(CT_THREADS, 1) count_tiles(CtArgs a)
         return (e >> 31) ? make_uint2((uint32_t)lane * 4u, 0u)
                          : make_uint2((e & 0xFFFu) * 4u, 1u << ct_shift<WT>((e >> 12) & 3u));
     };
+    const uint2 e1 = entry(a.lists[lane]);
     uint2 e2[CT_R2];
 #pragma unroll
-    for (int k = 0; k < CT_R2; k++) e2[k] = entry(a.lists[k * 32 + lane]);
-    for (int k = threadIdx.x; k < CT_R3 * 32; k += CT_THREADS) l3[k] = entry(a.lists[CT_R2 * 32 + k]);
+    for (int k = 0; k < CT_R2; k++) e2[k] = entry(a.lists[(1 + k) * 32 + lane]);
+    for (int k = threadIdx.x; k < CT_R3 * 32; k += CT_THREADS) l3[k] = entry(a.lists[(1 + CT_R2) * 32 + k]);
     const int pass = blockIdx.x % a.passes;  // grid: a multiple of passes
-    const uint32_t *recs = a.recs + (int64_t)pass * a.rec_cap;
-    uint32_t *recs_s = cnt + a.words * CT_ROWS;
-    const uint32_t n_rec = a.roff[(int64_t)pass * (a.n_pre + 1) + a.n_pre];
-    const bool staged = n_rec <= (uint32_t)a.rec_smem;
-    if (staged)
-        for (uint32_t k = threadIdx.x; k < n_rec; k += CT_THREADS) recs_s[k] = recs[k];
-    auto load_rec = [&](uint32_t k) -> uint32_t { return staged ? recs_s[k] : __ldg(recs + k); };
-    for (int k = threadIdx.x; k <= a.n_pre; k += CT_THREADS) off_s[k] = a.roff[(int64_t)pass * (a.n_pre + 1) + k];
+    const ct_rec<WT> *recs = (const ct_rec<WT> *)a.recs + (int64_t)pass * a.rec_cap;
+    const uint32_t *off = a.roff + (int64_t)pass * (a.n_pre + 1);
+    // A record in use: its counter's address (18 bits), and above it its weight or the
+    // shift of the query's half.  (The pass's records stay in L1.)
+    auto load_rec = [&](uint32_t k) -> uint32_t {
+        const uint32_t r = __ldg(recs + k);
+        return cbase + ((r & 0x3FFFu) << 2) + (r >> 14 << (WT ? 18 : 22));
+    };
     for (int k = threadIdx.x; k < CT_BALL; k += CT_THREADS) ball_s[k] = (uint16_t)a.ball[k];
     const int q0 = pass * PASS;
     const int nqp = min(PASS, a.nq - q0);
     const int words = WT ? nqp : (nqp + 1) >> 1;
-    // tasks: buckets of budget 3 (in 8 parts), 2 (in 4 parts), 1, 0; nb[b] of them,
-    // their masks from ball_s[sb[b]]
+    // buckets by budget, their masks in ball_s one budget after the other
     const int nb3 = D >= 3 ? a.nball[D - 3] : 0, nb2 = D >= 2 ? a.nball[D - 2] : 0, nb1 = D >= 1 ? a.nball[D - 1] : 0,
               nb0 = a.nball[D];
-    const int t3 = 8 * nb3, t2 = t3 + 4 * nb2, t1 = t2 + nb1, ntask = t1 + nb0;
     // the level-0 field (t = D) of a counter word; slow words have a window of the
     // query itself there, or (weighted) a count past its entry byte
     const uint32_t f0 = WT ? (D == 3 ? 0xFE000000u : D == 2 ? 0x01FE0000u : D == 1 ? 0x0001FE00u : 0x000001FFu)
@@ -372,7 +417,7 @@ __global__ void __launch_bounds__(CT_THREADS, 1) count_tiles(CtArgs a)
             if (lane == 0) base = atomicAdd(a.nexc, (unsigned)__popc(overs));
             const uint32_t pos = __shfl_sync(GKM_FULL, base, 0) + __popc(overs & ((1u << lane) - 1u));
             if (!over) return;
-            const uint32_t row = tl * CT_ROWS + ct_phys(at & (CT_ROWS - 1));
+            const uint32_t row = tl * CT_ROWS + ct_phys((at & (CT_ROWS - 1)) ^ ct_swap(j));
             ((uint32_t *)(a.T + (size_t)row * a.rb))[q0 + q] = clip(c, x);
             if (pos < a.cap_exc) {
                 a.exc[pos] = row | (unsigned long long)(q0 + q) << 22 | (unsigned long long)x[0] << 32;
@@ -393,7 +438,7 @@ __global__ void __launch_bounds__(CT_THREADS, 1) count_tiles(CtArgs a)
         }
     };
 
-    if (n_rec == 0) return;  // rows of length 0 pad a batch: the gather reads nothing of them
+    if (__ldg(off + a.n_pre) == 0) return;  // rows of length 0 pad a batch: the gather reads nothing of them
     const int tiles = a.items / a.passes;
     int par = 0, queued = -1;  // the tile whose queued entries wait for their second look
     for (int tile = blockIdx.x / a.passes; tile < tiles; tile += gridDim.x / a.passes, par ^= 1) {
@@ -405,158 +450,215 @@ __global__ void __launch_bounds__(CT_THREADS, 1) count_tiles(CtArgs a)
     __syncthreads();
     if (queued >= 0) look_queued(queued, par ^ 1);
 
-    // counts the windows of queries qa .. qb - 1 (safe: the recount of two
+    // counts the windows of queries qa .. qb - 1 (safe: the recount of four
     // queries with 32-bit counters, plane (q - qa) * 4 + t; else all)
-    auto count_buckets = [&](auto SAFE, int qa, int qb) -> unsigned long long {
+    auto count_buckets = [&](auto SAFE, int qa, int qb) -> uint32_t {
         constexpr bool safe = decltype(SAFE)::value;
-        unsigned long long adds = 0;
-        // counter address, increment of one window of weight 1 (0: not counted)
+        uint32_t adds = 0;
+        auto weight = [&](uint32_t rec) -> uint32_t { return WT ? rec >> 18 : 1u; };
+        // one window's counter address and what its increments are multiplied by
+        // (unweighted: shifted; safe: 0 if it is not counted)
         auto where = [&](uint32_t rec, uint32_t &sa, uint32_t &inc) {
-            const uint32_t at = rec & 0x7FFFu;
             if (safe) {
-                const int q = WT ? at / CT_ROWS : 2 * (at / CT_ROWS) + ((rec >> 15) & 1u);
+                const uint32_t at = (rec & 0x3FFFFu) - cbase, plane = at / PLANE;
+                const int q = WT ? plane : 2 * plane + (rec >> 22);
                 const bool in = q >= qa && q < qb;
-                sa = cbase + ((in ? (q - qa) * 4 * CT_ROWS + (at & (CT_ROWS - 1)) : 0u) << 2);
-                inc = in ? rec >> 16 : 0u;
+                sa = cbase + (in ? (q - qa) * 4 * PLANE + ((at & (PLANE - 1u)) ^ (ct_swap(plane) << 2)) : 0u);
+                inc = in ? weight(rec) : 0u;
             } else {
-                sa = cbase + (at << 2);
-                inc = WT ? rec >> 16 : 1u << ((rec >> 11) & 16u);
+                sa = rec & 0x3FFFFu;
+                inc = rec >> 18;
             }
         };
-        // add at the neighbour with byte offset x, field increment f = 1 << ct_shift(t)
-        auto add = [&](uint32_t sa, uint32_t x, uint32_t f, uint32_t inc) {
+        // add at the neighbour with byte offset x, field increment f = 1 << ct_shift(t),
+        // where i < n
+        auto add = [&](uint32_t sa, uint32_t x, uint32_t f, uint32_t inc, uint32_t i, uint32_t n) {
             if (safe) {
                 const uint32_t t = f == 1u ? 0u : f == 1u << ct_shift<WT>(1) ? 1u : f == 1u << ct_shift<WT>(2) ? 2u : 3u;
-                if (f && inc) ct_add((sa ^ x) + t * (4 * CT_ROWS), inc);
+                ct_add(i, f && inc ? n : 0u, (sa ^ x) + t * PLANE, inc);
             } else {
-                ct_add(sa ^ x, f * inc);
+                ct_add(i, n, sa ^ x, WT ? f * inc : f << inc);
             }
         };
-        // lane j: the warp's j-th task (at most 14), its bucket's records
-        uint32_t my_beg = 0, my_end = 0, my_kind = 0;
-        {
-            const int task = warp + CT_WARPS * lane;
-            if (task < ntask) {
-                int k;
-                if (task < t3) {
-                    my_kind = 3u | (task & 7) << 2;
-                    k = task >> 3;
-                } else if (task < t2) {
-                    my_kind = 2u | ((task - t3) & 3) << 2;
-                    k = nb3 + ((task - t3) >> 2);
-                } else {
-                    my_kind = task < t1 ? 1u : 0u;
-                    k = nb3 + nb2 + task - t2;
-                }
-                const uint32_t pre = (uint32_t)tile ^ ball_s[k];
-                my_beg = off_s[pre];
-                my_end = off_s[pre + 1];
-            }
-        }
-        uint32_t c = __shfl_sync(GKM_FULL, my_beg, 0), end = __shfl_sync(GKM_FULL, my_end, 0);
-        uint32_t rec = c + lane < end ? load_rec(c + lane) : 0u;
-        const int mine = (ntask - warp + CT_WARPS - 1) / CT_WARPS;
-        for (int j0 = 0; j0 < mine; j0++) {
-            const uint32_t kind = __shfl_sync(GKM_FULL, my_kind, j0);
-            const int b = kind & 3, part = kind >> 2;
-            // the next task's records, in flight while this one is counted
-            const int jn = j0 + 1 < mine ? j0 + 1 : j0;
-            const uint32_t nc = __shfl_sync(GKM_FULL, my_beg, jn), nend = __shfl_sync(GKM_FULL, my_end, jn);
-            const uint32_t nrec = nc + lane < nend ? load_rec(nc + lane) : 0u;
-            while (c < end) {
-                const int n = min(32u, end - c);
+        auto bucket = [&](int k, uint32_t &beg, uint32_t &end) {
+            const uint32_t pre = (uint32_t)tile ^ ball_s[k];
+            beg = __ldg(off + pre);
+            end = __ldg(off + pre + 1);
+        };
+        // budget 3: a warp takes every CT_WARPS-th window of the bucket
+        if (nb3) {
+            uint32_t r, e;
+            bucket(0, r, e);
+            for (r += warp; r < e; r += CT_WARPS) {
+                const uint32_t rec = load_rec(r);
                 uint32_t sa, inc;
                 where(rec, sa, inc);
-                const uint32_t w = rec >> 16;
-                if (b <= 1) {
-                    if (lane < n) {
-                        if (b == 0) {
-                            add(sa, 0u, 1u, inc);
-                            adds += w;
-                        } else {
-                            add(sa, 0u, 1u << ct_shift<WT>(1), inc);
+                if (lane == 0) adds += 376u * weight(rec);
+#pragma unroll 10
+                for (int k = 0; k < CT_R3; k++) {
+                    const uint2 x = l3[k * 32 + lane];
+                    add(sa, x.x, x.y, inc, r, e);
+                }
+            }
+        }
+        // budget 0: a bucket per lane
+        const int near = nb3 + nb2 + nb1;
+        for (int b = CT_WARPS - 1 - warp; b * 32 < nb0; b += CT_WARPS) {
+            uint32_t r = 0, e = 0;
+            if (b * 32 + lane < nb0) bucket(near + b * 32 + lane, r, e);
+            auto zero = [&](uint32_t rec, uint32_t i, uint32_t n) {
+                uint32_t sa, inc;
+                where(rec, sa, inc);
+                add(sa, 0u, 1u, inc, i, n);
+                if (WT && i < n) adds += weight(rec);
+            };
+            if (!WT) adds += e - r;
+            const uint32_t some = min(e, r + 128u);
+            for (; r < some; r += 4) {
+                uint32_t x[4];
 #pragma unroll
-                            for (int pos = 0; pos < 6; pos++)
+                for (int k = 0; k < 4; k++) x[k] = load_rec(r + k);
 #pragma unroll
-                                for (uint32_t d = 1; d < 4; d++) add(sa, ct_phys(d << (2 * pos)) << 2, 1u, inc);
-                            adds += 19u * w;
+                for (int k = 0; k < 4; k++) zero(x[k], r + k, some);
+            }
+            r = some;
+            // the rest of a crowded bucket (low-complexity rows) by all lanes
+            for (uint32_t rest = __ballot_sync(GKM_FULL, r < e); rest; rest &= rest - 1) {
+                const int j = __ffs(rest) - 1;
+                const uint32_t re = __shfl_sync(GKM_FULL, e, j);
+                for (uint32_t k = __shfl_sync(GKM_FULL, r, j) + lane; k < re; k += 32) zero(load_rec(k), k, re);
+            }
+        }
+        // budgets 1 and 2: lanes 0 .. n1 - 1 and n1 .. n1 + n2 - 1 have the warp's
+        // buckets of each and list up to cap windows of them at a time
+        if (nb1) {
+            const int n1 = (nb1 + CT_WARPS - 1) / CT_WARPS, n2 = (nb2 + CT_WARPS - 1) / CT_WARPS;
+            const bool is1 = lane < n1;
+            const int k = is1 ? nb3 + nb2 + warp + CT_WARPS * lane : nb3 + warp + CT_WARPS * (lane - n1);
+            uint32_t r = 0, e = 0;
+            if (k < (is1 ? near : nb3 + nb2)) bucket(k, r, e);
+            if (!WT) adds += (is1 ? 16u : 106u) * (e - r);
+            const uint32_t cap = is1 ? CT_LIST1 / n1 : n2 ? CT_LIST2 / n2 : 0;
+            uint32_t *list = list_s + warp * LIST;
+            while (__any_sync(GKM_FULL, r < e)) {
+                const uint32_t m = min(cap, e - r), v = is1 ? m : m << 16;
+                uint32_t x = v;
+#pragma unroll
+                for (int o = 1; o < 16; o <<= 1) {
+                    const uint32_t y = __shfl_up_sync(GKM_FULL, x, o);
+                    if (lane >= o) x += y;
+                }
+                const uint32_t all = __shfl_sync(GKM_FULL, x, 15), n_1 = all & 0xFFFFu, n_2 = all >> 16;
+                uint32_t *to = list + (is1 ? (x - v) & 0xFFFFu : CT_LIST1 + 8 + ((x - v) >> 16));
+                uint32_t w = 0;
+                for (uint32_t c = 0; c < m; c += 4) {
+                    uint32_t y[4];
+#pragma unroll
+                    for (int i = 0; i < 4; i++) y[i] = load_rec(r + c + i);
+#pragma unroll
+                    for (int i = 0; i < 4; i++)
+                        if (c + i < m) {
+                            to[c + i] = y[i];
+                            if (WT) w += weight(y[i]);
                         }
-                    }
-                } else if (b == 2) {
-                    if (part == 0 && lane < n) adds += 154u * w;
-                    for (int j = part; j < n; j += 4) {
-                        const uint32_t ss = __shfl_sync(GKM_FULL, sa, j), si = __shfl_sync(GKM_FULL, inc, j);
+                }
+                if (WT) adds += (is1 ? 16u : 106u) * w;
+                r += m;
+                __syncwarp();
+                for (uint32_t j = lane >> 4; j < n_1 + (lane >> 4); j += 8) {  // half a warp per window
 #pragma unroll
-                        for (int k = 0; k < CT_R2; k++) add(ss, e2[k].x, e2[k].y, si);
-                    }
-                } else {
-                    if (part == 0 && lane < n) adds += 694u * w;
-                    for (int j = part; j < n; j += 8) {
-                        const uint32_t ss = __shfl_sync(GKM_FULL, sa, j), si = __shfl_sync(GKM_FULL, inc, j);
-#pragma unroll 2
-                        for (int k = 0; k < CT_R3; k++) {
-                            const uint2 e = l3[k * 32 + lane];
-                            add(ss, e.x, e.y, si);
-                        }
+                    for (int i = 0; i < 4; i++) {
+                        uint32_t sa, inc;
+                        where(list[j + 2 * i], sa, inc);
+                        add(sa, e1.x, e1.y, inc, j + 2 * i, n_1);
                     }
                 }
-                c += 32;
-                if (c < end) rec = c + lane < end ? load_rec(c + lane) : 0u;
+#pragma unroll 2
+                for (uint32_t j = 0; j < n_2; j++) {
+                    uint32_t sa, inc;
+                    where(list[CT_LIST1 + 8 + j], sa, inc);
+#pragma unroll
+                    for (int i = 0; i < CT_R2; i++) add(sa, e2[i].x, e2[i].y, inc, j, n_2);
+                }
+                __syncwarp();
             }
-            c = nc, end = nend, rec = nrec;
         }
         return adds;
     };
 
-    unsigned long long adds = count_buckets(std::false_type{}, 0, nqp);
+    const uint32_t adds = count_buckets(std::false_type{}, 0, nqp);
     __syncthreads();
-    // The tile's entries (row by row; a thread takes four neighbouring counters
-    // of every word), the words that need more queued, and the fields' sum: it
-    // equals the adds made unless some field carried into the next.
-    uint8_t *T = a.T + (size_t)tile * CT_ROWS * a.rb + q0 * (WT ? 4 : 2);
-    {
-        uint32_t fa = 0, fb = 0;
+    // The tile's entries, the words that need more queued, and the fields' sum: it
+    // equals the adds made unless some field carried into the next.  Four lanes, eight
+    // apart, write the quarters of a row, so that a store writes eight rows side by
+    // side.  The words are summed by carry-save adders (two logic operations a word)
+    // and the fields of the six sums added up.
+    auto write_tile = [&](auto FULL) {
+        constexpr bool full = decltype(FULL)::value;  // every word of a row is counted and stored
+        const int part = (lane >> 3) & 3, j0 = 4 * part;
+        uint8_t *T = a.T + (size_t)tile * CT_ROWS * a.rb + q0 * (WT ? 4 : 2) + 16 * part;
+        const bool write = full || 16 * part < a.rb;  // (narrow rows: fewer quarters)
+        const uint32_t row0 = ct_phys(threadIdx.x & ~24u) * a.rb;
+        const uint32_t *mine = cnt + j0 * CT_ROWS;
+        uint32_t ones = 0, twos = 0, fours = 0, e[4];
+        static_assert(CT_ROWS == 2 * CT_THREADS && CT_SLOTS == 16, "32 words per thread");
 #pragma unroll
-        for (int i = 0; i < CT_ROWS / CT_THREADS; i++) {
-            const uint32_t p = i * CT_THREADS + threadIdx.x;
-            uint32_t o[CT_SLOTS], slow = 0;
+        for (int i = 0; i < 4; i++) {
+            uint32_t t[4], f[2];
 #pragma unroll
-            for (int j = 0; j < CT_SLOTS; j++) {
-                const uint32_t w = j < words ? cnt[j * CT_ROWS + p] : 0u;
-                if (WT) {
-                    fa = __dp4a(w >> 9, 0x00010101u, fa) + (w & 0x1FFu);
-                    o[j] = (w & 0xFFu) | ((w >> 1) & 0xFFFFFF00u);
-                } else {
-                    // t = 0 and 1 are the bytes' low fields; t = 3 and 2 the high
-                    // ones, 32 and 16 times too large
-                    fa = __dp4a(w & 0x0F1F0F1Fu, 0x01010101u, fa);
-                    fb = __dp4a(w & 0xF0E0F0E0u, 0x02010201u, fb);
-                    o[j] = w;
-                }
-                slow |= (uint32_t)((w & slow_mask) != 0) << j;
+            for (int g = 0; g < 2; g++) {
+                // the row of position (i / 2) * CT_THREADS + threadIdx.x with bits 3 and 4 = h
+                const uint32_t h = (i & 1) * 2 + g, at = (i >> 1) * CT_THREADS;
+                uint32_t w[4];
+#pragma unroll
+                for (int j = 0; j < 4; j++) w[j] = full || j0 + j < words ? mine[j * CT_ROWS + ((at + threadIdx.x) ^ (8u * h))] : 0u;
+                ct_fa(ones, t[2 * g], w[0], w[1]);
+                ct_fa(ones, t[2 * g + 1], w[2], w[3]);
+                if (WT)
+#pragma unroll
+                    for (int j = 0; j < 4; j++) w[j] = (w[j] & 0xFFu) | ((w[j] >> 1) & 0xFFFFFF00u);
+                const uint32_t row = row0 ^ ((ct_phys(at) ^ (8u * h)) * a.rb);
+                if (write) *(uint4 *)(T + row) = make_uint4(w[0], w[1], w[2], w[3]);
             }
-            uint4 *out = (uint4 *)(T + (size_t)ct_phys(p) * a.rb);
-            out[0] = make_uint4(o[0], o[1], o[2], o[3]);
-            out[1] = make_uint4(o[4], o[5], o[6], o[7]);
-            for (; slow; slow &= slow - 1) {
-                const int j = __ffs(slow) - 1, n = atomicAdd(&nlist[par], 1);
-                if (n < CT_LIST) {
-                    list_at[par][n] = (uint16_t)(j * CT_ROWS + p);
-                    list_w[par][n] = cnt[j * CT_ROWS + p];
-                }
+            ct_fa(twos, f[0], t[0], t[1]);
+            ct_fa(twos, f[1], t[2], t[3]);
+            ct_fa(fours, e[i], f[0], f[1]);
+        }
+        uint32_t eights = 0, s0, s1;
+        ct_fa(eights, s0, e[0], e[1]);
+        ct_fa(eights, s1, e[2], e[3]);
+        const uint32_t sums[6] = {ones, twos, fours, eights, s0 ^ s1, s0 & s1};
+        uint32_t sum = 0, any = 0;
+#pragma unroll
+        for (int k = 0; k < 6; k++) {
+            const uint32_t w = sums[k];
+            any |= w;
+            // (unweighted: t = 0 and 1 are the bytes' low fields, t = 3 and 2 the high
+            // ones, 32 and 16 times too large)
+            sum += (WT ? __dp4a(w >> 9, 0x00010101u, w & 0x1FFu)
+                       : __dp4a(w & 0x0F1F0F1Fu, 0x01010101u, __dp4a(w & 0xF0E0F0E0u, 0x02010201u, 0u) >> 5)) << k;
+        }
+        // a lane that saw such a word: its 32 words again, one per lane
+        for (uint32_t some = __ballot_sync(GKM_FULL, (any & slow_mask) != 0); some; some &= some - 1) {
+            const int from = __ffs(some) - 1;
+            const int j = ((from >> 3) & 3) * 4 + (lane & 3),
+                      pos = ((lane >> 4) * CT_THREADS + warp * 32 + from) ^ (2 * (lane & 12));
+            const uint32_t w = j < words ? cnt[j * CT_ROWS + pos] : 0u;
+            if (!(w & slow_mask)) continue;
+            const int n = atomicAdd(&nlist[par], 1);
+            if (n < CT_LIST) {
+                list_at[par][n] = (uint16_t)(j * CT_ROWS + pos);
+                list_w[par][n] = w;
             }
         }
-        unsigned long long sum = fa + (fb >> 5);
-#pragma unroll
-        for (int o2 = 16; o2; o2 >>= 1) {
-            sum += __shfl_xor_sync(GKM_FULL, sum, o2);
-            adds += __shfl_xor_sync(GKM_FULL, adds, o2);
-        }
+        const uint32_t wsum = __reduce_add_sync(GKM_FULL, sum), wadds = __reduce_add_sync(GKM_FULL, adds);
         if (lane == 0) {
-            atomicAdd(&chk[par][0], sum);
-            atomicAdd(&chk[par][1], adds);
+            atomicAdd(&chk[par][0], wsum);
+            atomicAdd(&chk[par][1], wadds);
         }
-    }
+    };
+    if (words == CT_SLOTS && a.rb >= 4 * CT_SLOTS) write_tile(std::true_type{});
+    else write_tile(std::false_type{});
     __syncthreads();
 
     queued = -1;
@@ -571,9 +673,9 @@ __global__ void __launch_bounds__(CT_THREADS, 1) count_tiles(CtArgs a)
             __syncthreads();
         }
     } else {
-        // a field overflowed: 32-bit counters, two queries x four levels at a time
-        for (int qa = 0; qa < nqp; qa += 2) {
-            const int nb = min(2, nqp - qa);
+        // a field overflowed: 32-bit counters, four queries x four levels at a time
+        for (int qa = 0; qa < nqp; qa += 4) {
+            const int nb = min(4, nqp - qa);
             __syncthreads();
             for (int k = threadIdx.x; k < 4 * nb * CT_ROWS; k += CT_THREADS) cnt[k] = 0;
             __syncthreads();
@@ -581,6 +683,7 @@ __global__ void __launch_bounds__(CT_THREADS, 1) count_tiles(CtArgs a)
             __syncthreads();
             for (int p = threadIdx.x; p < CT_ROWS; p += CT_THREADS) {
                 const uint32_t suf = ct_phys(p);
+                uint8_t *T = a.T + ((size_t)tile * CT_ROWS + suf) * a.rb + q0 * (WT ? 4 : 2);
                 for (int q = 0; q < nb; q++) {
                     const uint32_t *cq = cnt + q * 4 * CT_ROWS + p;
                     const uint32_t c[4] = {cq[0], cq[CT_ROWS], cq[2 * CT_ROWS], cq[3 * CT_ROWS]};
@@ -588,9 +691,9 @@ __global__ void __launch_bounds__(CT_THREADS, 1) count_tiles(CtArgs a)
                     uint32_t x[4];
                     const uint32_t v = clip(c, x);
                     if (WT)
-                        ((uint32_t *)(T + (size_t)suf * a.rb))[qa + q] = v;
+                        ((uint32_t *)T)[qa + q] = v;
                     else
-                        ((uint16_t *)(T + (size_t)suf * a.rb))[qa + q] = (uint16_t)v;
+                        ((uint16_t *)T)[qa + q] = (uint16_t)v;
                     const uint64_t ex[4] = {x[0], x[1], x[2], x[3]};
                     if (x[0] | x[1] | x[2] | x[3]) ct_excess<WT>(a, sh.lmer(tile * CT_ROWS + suf), q0 + qa + q, ex, 0, 1);
                 }
@@ -616,13 +719,6 @@ __global__ void spill_excess(CtArgs a)
 // ---------------------------------------------------------------------------
 // 2. gather
 // ---------------------------------------------------------------------------
-
-__device__ __forceinline__ void ct_fa(uint32_t &s, uint32_t &c, uint32_t a, uint32_t b)
-{
-    const uint32_t x = s;
-    s = x ^ a ^ b;
-    c = (x & a) | (x & b) | (a & b);
-}
 
 // acc[t] (two 16-bit sums, a query each) += the fields of entry word x times 2^p
 __device__ __forceinline__ void ct_unpack(uint32_t *acc, uint32_t x, int p)
@@ -673,21 +769,24 @@ __device__ __forceinline__ void ct_finish(const CtArgs &a, int64_t s, int j0, co
 }
 
 // RB-byte rows, 16 bytes per lane, RB / 16 lanes per SV; persistent blocks take
-// SVs round robin in gather order (long SVs first).  Bound by L2 and HBM latency
+// SVs round robin in gather order (long SVs first); where there are fewer SVs than
+// lane groups, `split` groups share an SV's windows.  Bound by L2 and HBM latency
 // times bandwidth: every lane keeps two stages of eight row pieces in flight in
 // its own slots of shared memory (asynchronous copies; nothing is shared between
 // lanes, so no barriers) while it adds a third.
-template <int RB, bool WT, bool RAW>
+template <int RB, bool WT, bool RAW, bool SPLIT>
 __global__ void __launch_bounds__(G_THREADS, WT ? G_BLOCKS_W : G_BLOCKS) gather_kernel(CtArgs a)
 {
     constexpr int NQ = WT ? 4 : 8;  // queries a lane owns
-    constexpr int LPG = RB / 16, GPB = G_THREADS / LPG, QG = LPG * NQ;
+    constexpr int LPG = RB / 16, QG = LPG * NQ;
+    const int split = SPLIT ? a.split : 1, lanes = LPG * split, GPB = G_THREADS / lanes;  // lanes per SV, SVs per block
     __shared__ uint4 rows_s[4 * G_THREADS];
     __shared__ double inv_dx[QG];
     __shared__ uint32_t empty_s[QG];  // a query without windows (its columns may hold another group's counts)
     __shared__ double part_s[G_THREADS / 32][QG];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int sub = threadIdx.x % LPG, j0 = sub * NQ;
+    const uint32_t turn = SPLIT ? threadIdx.x / LPG % split : 0;  // the lane group's stages: turn, turn + split, ..
     bool some = false;
     for (int j = threadIdx.x; j < QG; j += G_THREADS) {
         inv_dx[j] = 0.0;
@@ -709,8 +808,8 @@ __global__ void __launch_bounds__(G_THREADS, WT ? G_BLOCKS_W : G_BLOCKS) gather_
     const uint8_t *base = a.T + sub * 16;
     const int64_t rounds = (a.S + (int64_t)gridDim.x * GPB - 1) / ((int64_t)gridDim.x * GPB);
     for (int64_t it = 0; it < rounds; it++) {
-        const int64_t g = (it * gridDim.x + blockIdx.x) * GPB + threadIdx.x / LPG;
-        const bool live = g < a.S;
+        const int64_t g = (it * gridDim.x + blockIdx.x) * GPB + threadIdx.x / lanes;
+        bool live = g < a.S;
         const int64_t s = live ? a.perm[g] : 0;
         const uint32_t p0 = live ? a.goff[g] : 0;
         uint32_t nst = live ? (a.goff[g + 1] - p0) >> 3 : 0;
@@ -723,7 +822,7 @@ __global__ void __launch_bounds__(G_THREADS, WT ? G_BLOCKS_W : G_BLOCKS) gather_
             id[0] = i0.x, id[1] = i0.y, id[2] = i0.z, id[3] = i0.w;
             id[4] = i1.x, id[5] = i1.y, id[6] = i1.z, id[7] = i1.w;
         };
-        load_ids(0);
+        load_ids(turn);
         uint32_t acc[16];  // WT: [query][t]; else [word][t], two 16-bit sums each
 #pragma unroll
         for (int k = 0; k < 16; k++) acc[k] = 0;
@@ -732,13 +831,13 @@ __global__ void __launch_bounds__(G_THREADS, WT ? G_BLOCKS_W : G_BLOCKS) gather_
         // carries of weight 32 are added field by field into 16-bit sums (31 x 2,048
         // rows < 2^16).  (p8, p16: carries waiting for the second of a pair)
         uint32_t ones[4] = {}, twos[4] = {}, fours[4] = {}, eights[4] = {}, s16[4] = {}, p8[4] = {}, p16[4] = {};
-        for (uint32_t k = 0; k < nst; k++) {
+        for (uint32_t k = turn, n = 0; k < nst; k += split, n++) {
             uint4 r[8];
 #pragma unroll
             for (int j = 0; j < 8; j++) r[j] = __ldg((const uint4 *)(base + (size_t)id[j] * RB));
-            uint2 wt = make_uint2(0, 0);
-            if (WT) wt = __ldg((const uint2 *)(a.wts + p0) + k);
-            load_ids(k + 1);
+            uint2 wt = make_uint2(0x01010101u, 0x01010101u);
+            if (WT && a.wts) wt = __ldg((const uint2 *)(a.wts + p0) + k);
+            load_ids(k + split);
             if constexpr (!WT) {
                 uint32_t f[2][4];
 #pragma unroll
@@ -758,14 +857,14 @@ __global__ void __launch_bounds__(G_THREADS, WT ? G_BLOCKS_W : G_BLOCKS) gather_
                 for (int w = 0; w < 4; w++) {
                     uint32_t e;
                     ct_fa(fours[w], e, f[0][w], f[1][w]);
-                    if ((k & 1) == 0) {
+                    if ((n & 1) == 0) {
                         p8[w] = e;
                         continue;
                     }
                     uint32_t c;
                     ct_fa(eights[w], c, p8[w], e);
                     p8[w] = 0;
-                    if ((k & 2) == 0) {
+                    if ((n & 2) == 0) {
                         p16[w] = c;
                     } else {
                         uint32_t x;
@@ -812,6 +911,12 @@ __global__ void __launch_bounds__(G_THREADS, WT ? G_BLOCKS_W : G_BLOCKS) gather_
                 ct_unpack(acc + 4 * w, eights[w], 3);
                 ct_unpack(acc + 4 * w, s16[w], 4);
             }
+        }
+        if (SPLIT) {  // the groups' sums, in the first
+#pragma unroll
+            for (int k = 0; k < 16; k++)
+                for (int o = LPG; o < lanes; o <<= 1) acc[k] += __shfl_xor_sync(GKM_FULL, acc[k], o);
+            live = live && turn == 0;
         }
         // epilogue, four queries at a time (the sums wait in the lane's slots, so
         // that the loop above has the registers).  Weighted: two lanes share a byte
@@ -973,25 +1078,32 @@ static int64_t ct_table_rows(const gkm_index *ix)
     return sh.fold ? (int64_t)1 << (2 * sh.l - 1) : (int64_t)1 << (2 * sh.l);
 }
 
-// Neighbour masks of the six suffix positions with 0 .. b mismatches for b = 2,
-// 3, arranged so that lane k of every round holds a mask of bank class k:
-// position | t << 12, or bit 31.
+// Neighbour masks of the suffix positions with 0 .. b mismatches for b = 1 ..
+// 3, arranged so that lane k of every round holds a mask of bank class k (budget 1:
+// the 16 masks twice): position | t << 12, or bit 31.
 static void ct_lists(uint32_t *out)
 {
-    const int rounds[4] = {0, 0, CT_R2, CT_R3};
+    const int rounds[4] = {0, 1, CT_R2, CT_R3};
     uint32_t *p = out;
-    for (int b = 2; b <= 3; b++) {
-        int used[32] = {0};
+    for (int b = 1; b <= 3; b++) {
+        int used[32] = {0}, n = 0;
         for (int k = 0; k < rounds[b] * 32; k++) p[k] = 0x80000000u;
         for (uint32_t x = 0; x < CT_ROWS; x++) {
-            const int m = __builtin_popcount((x | (x >> 1)) & 0x555u), cls = ct_phys(x) & 31;
-            if (m <= b) p[32 * used[cls]++ + cls] = ct_phys(x) | (uint32_t)(b - m) << 12;
+            const int m = __builtin_popcount((x | (x >> 1)) & 0x55555555u), cls = ct_phys(x) & 31;
+            const uint32_t e = ct_phys(x) | (uint32_t)(b - m) << 12;
+            if (m > b) continue;
+            if (b == 1) {
+                p[n] = p[n + 16] = e;
+                n++;
+            } else {
+                p[32 * used[cls]++ + cls] = e;
+            }
         }
         p += rounds[b] * 32;
     }
 }
 
-// Masks of n positions (l - 6 of them) with m mismatches; returns how many.
+// Masks of n positions (l - CT_POS of them) with m mismatches; returns how many.
 static int ct_ball(int n, int m, uint32_t *out)
 {
     int k = 0;
@@ -1017,16 +1129,16 @@ int gkm_ct_build(gkm_index *ix, const uint32_t *fwd, const int32_t *counts, cuda
     do {
         if (cudaMalloc(&ix->ct_perm, sizeof(uint32_t) * S) != cudaSuccess ||
             cudaMalloc(&ix->ct_off, sizeof(uint32_t) * (S + 1)) != cudaSuccess ||
-            cudaMalloc(&ix->ct_lists, sizeof(uint32_t) * (32 * (CT_R2 + CT_R3) + CT_BALL)) != cudaSuccess ||
+            cudaMalloc(&ix->ct_lists, sizeof(uint32_t) * (32 * CT_ROUNDS + CT_BALL)) != cudaSuccess ||
             cudaMallocAsync(&k0, sizeof(uint32_t) * (S + 1), st) != cudaSuccess ||
             cudaMallocAsync(&k1, sizeof(uint32_t) * (S + 1), st) != cudaSuccess ||
             cudaMallocAsync(&v1, sizeof(uint32_t) * (S + 1), st) != cudaSuccess) {
             s = gkm_fail(GKM_ERR_OOM, "gather lists");
             break;
         }
-        uint32_t lists[32 * (CT_R2 + CT_R3) + CT_BALL] = {};
+        uint32_t lists[32 * CT_ROUNDS + CT_BALL] = {};
         ct_lists(lists);
-        for (int m = 0, k = 32 * (CT_R2 + CT_R3); m <= sh.D; m++) k += ct_ball(sh.l - 6, m, lists + k);
+        for (int m = 0, k = 32 * CT_ROUNDS; m <= sh.D; m++) k += ct_ball(sh.l - CT_POS, m, lists + k);
         if (cudaMemcpyAsync(ix->ct_lists, lists, sizeof(lists), cudaMemcpyHostToDevice, st) != cudaSuccess) {
             s = gkm_cuda_status(cudaGetLastError(), "mask lists");
             break;
@@ -1076,7 +1188,8 @@ void gkm_ct_free(gkm_index *ix)
 // The row width of a call: 32 bytes for batches that fit a few groups of them,
 // else 128.
 struct CtPlan {
-    int rb, qg, blocks;
+    bool wide;                // four bytes per query (weighted kernels, dense rows), else two
+    int rb, qg, blocks, split;
     int64_t groups, rows, table, c, dirty, self, nexc, exc, partial, bytes;
     int pass, passes;         // queries of a count_tiles pass, passes of a full group
     int64_t rec_cap, chunk;   // window records of a pass, groups bucketed at a time
@@ -1084,10 +1197,29 @@ struct CtPlan {
     int n_pre;
 };
 
-static CtPlan ct_plan(const gkm_index *ix, int64_t B, int64_t W)
+// Known average rows past this mean take wide entries: below it two bytes a query cost
+// less (l = 10, 72,000 SVs: 10.2 against 13.5 us a 500 bp row; l = 11: 18.2 against 22.3
+// at 1,800 bp), above it most tiles are counted twice (600 bp: 19.8 against 14.2; 2,000
+// bp: 29.9 against 23.2).
+constexpr double WIDE_MEAN = 3.4;
+
+// The mean count of a table row at level dmax for rows of W window slots.
+static double ct_mean(const gkm_index *ix, int64_t W)
+{
+    double reach = 1.0;
+    for (int m = 0; m < ix->spec.dmax; m++) reach *= 3.0 * (ix->spec.l - m) / (m + 1);
+    const double wx = ix->spec.weighted ? (double)gkm_weight_sum(ix, W) : (double)W;
+    return (double)ix->strands * wx * reach / (double)ix->n_lmers;
+}
+
+static CtPlan ct_plan(const gkm_index *ix, int64_t B, int64_t W, int64_t windows)
 {
     CtPlan p = {};
-    const int wt = ix->spec.weighted ? 4 : 2;
+    // fields of 5 bits hold the AT-rich rows of five times a mean of 4.6 (a tile with a
+    // larger count is counted again); past it, and for average rows past WIDE_MEAN,
+    // unweighted rows, too, take the weighted ones' bytes, all weights 1
+    p.wide = ix->spec.weighted || ct_mean(ix, W) > 4.6 || (windows > 0 && ct_mean(ix, windows / B < W ? windows / B : W) > WIDE_MEAN);
+    const int wt = p.wide ? 4 : 2;
     // 32 queries a group: 64- or (weighted) 128-byte rows; the narrowest rows that
     // hold a smaller batch
     p.rb = wt * 32;
@@ -1095,37 +1227,44 @@ static CtPlan ct_plan(const gkm_index *ix, int64_t B, int64_t W)
     p.qg = p.rb / wt;
     p.groups = (B + p.qg - 1) / p.qg;
     p.rows = ct_table_rows(ix);
-    const int per_sm = ix->spec.weighted ? G_BLOCKS_W : G_BLOCKS;
+    const int per_sm = p.wide ? G_BLOCKS_W : G_BLOCKS;
     p.blocks = gkm_query_blocks() * per_sm;
+    // few SVs: a power of two of lane groups within a warp for each (2,000 SVs of 200 ..
+    // 500 bp: 94 -> 47 us per group of 32 weighted queries, 36 -> 12 us unweighted)
+    p.split = 1;
+    while (p.rb / 16 * p.split < 32 && ix->S * (p.rb / 16) * p.split * 2 <= (int64_t)p.blocks * G_THREADS) p.split *= 2;
     auto up = [](int64_t n) { return (n + 255) & ~(int64_t)255; };
     p.table = up((p.rows + 2) * p.rb);
     p.self = up(B * 4 * 8);
     p.nexc = up(p.groups * 4);
-    p.exc = ix->spec.weighted ? up(8 * CT_EXC * (B < p.qg ? B : p.qg)) : 0;
+    p.exc = p.wide ? up(8 * CT_EXC * (B < p.qg ? B : p.qg)) : 0;
     p.dirty = up(ix->S * p.qg / 8 + 8);
     p.c = up(ix->S * p.qg * 16);
     p.partial = up(p.groups * gkm_sm_count() * per_sm * p.qg * 8);  // (a grid limit only lowers p.blocks)
     // windows by bucket: the groups whose records fit 64 MB, at least one
-    p.pass = ix->spec.weighted ? CT_SLOTS : 2 * CT_SLOTS;
+    p.pass = p.wide ? CT_SLOTS : 2 * CT_SLOTS;
     p.passes = p.qg / p.pass > 0 ? p.qg / p.pass : 1;
-    p.n_pre = 1 << (2 * (ix->spec.l - 6));
+    p.n_pre = 1 << (2 * (ix->spec.l - CT_POS));
     p.rec_cap = (int64_t)p.pass * W * ix->strands;
-    p.chunk = (64LL << 20) / (4 * p.rec_cap * p.passes);
+    const int64_t rec = p.wide ? sizeof(ct_rec<true>) : sizeof(ct_rec<false>);
+    p.chunk = (64LL << 20) / (rec * p.rec_cap * p.passes);
     if (p.chunk < 1) p.chunk = 1;
     if (p.chunk > p.groups) p.chunk = p.groups;
-    p.recs = up(4 * p.rec_cap * p.passes * p.chunk);
+    p.recs = up(rec * (p.rec_cap * p.passes * p.chunk + 8));  // (count_tiles reads up to eight past a bucket)
     p.roff = up(4 * (int64_t)(p.n_pre + 1) * p.passes * p.chunk);
     p.bytes = p.table + p.self + p.nexc + p.dirty + p.c + p.partial + p.recs + p.roff + p.exc;
     return p;
 }
 
-// Microseconds of a query, measured on B200 (l = 11, 300 .. 72,000 SVs of 200 ..
-// 500 bp, 1 .. 1,024 rows of 30 .. 2,000 bp).  Count tables: a tile pass on one SM
-// costs CT_ITEM_US plus CT_WINDOW_US per window of its longest row, the gather
-// reads the SVs' table rows at CT_GATHER_BYTES_US.  Index walk: its lookups and
-// hits, at least WALK_FLOOR_US (a few rows leave most SMs idle and a row's masks
-// are a serial walk).
-constexpr double CT_CALL_US = 60.0, CT_ITEM_US = 12.8, CT_WINDOW_US = 0.0125, CT_GATHER_BYTES_US = 9.0e6;
+// Microseconds of a query, measured on B200 (l = 10 and 11, 300 .. 72,000 SVs of 200
+// .. 500 bp, 1 .. 1,024 rows of 30 .. 1,000 bp; 90 % of 322 shapes within 27 %, and
+// none that takes the tables by them is slower than the walk).  Count tables: a wave of
+// tile passes costs CT_ITEM_US plus CT_WINDOW_US per window of the pass's rows, the
+// gather reads the SVs' table rows at CT_GATHER_BYTES_US.  Index walk: its lookups and
+// hits, at least WALK_FLOOR_US (a few rows leave most SMs idle and a row's masks are a
+// serial walk).  At 72,000 SVs, t=3, the tables win from one 300 bp row (1.3 -> 0.2 ms)
+// on; at 30 bp rows from 64 at a time the walk does (1,024 rows: 7.5 against 4.0 ms).
+constexpr double CT_CALL_US = 45.0, CT_ITEM_US = 12.0, CT_WINDOW_US = 8.5e-4, CT_GATHER_BYTES_US = 8.0e6;
 constexpr double WALK_FLOOR_US = 400.0, WALK_LOOKUP_US[2] = {8.0e-6, 5.8e-6}, WALK_HIT_US[2] = {1.1e-6, 2.0e-6};
 
 // Whether a query over B rows of W window slots, `windows` windows in all, may
@@ -1139,17 +1278,15 @@ static bool ct_applies(const gkm_index *ix, int64_t B, int64_t W, int64_t window
     // (row, SV) weight products summed over every pair of windows
     const uint64_t wx = wt ? gkm_weight_sum(ix, W) : (uint64_t)W, wy = wt ? gkm_weight_sum(ix, ix->W) : (uint64_t)ix->W;
     if (!wx || !wy || wx >= (1ull << 32) / ((uint64_t)ix->strands * wy)) return false;
-    // the mean count of a table row at level dmax: fields of 31 (unweighted, over
-    // which a tile is recounted) hold the AT-rich rows of five times the mean
-    double reach = 1.0;
-    for (int m = 0; m < ix->spec.dmax; m++) reach *= 3.0 * (ix->spec.l - m) / (m + 1);
-    const double mean = (double)ix->strands * (double)wx * reach / (double)ix->n_lmers;
-    if (mean > (wt ? 80.0 : 4.6)) return false;
+    // bytes hold the AT-rich rows of three times this mean
+    if (ct_mean(ix, W) > 80.0) return false;
+    const int64_t known = windows;
     if (windows <= 0) windows = B * W / 2;  // lengths unknown: rows padded to W
-    const CtPlan p = ct_plan(ix, B, W);
+    const CtPlan p = ct_plan(ix, B, W, known);
     const int64_t items = p.rows / CT_ROWS * p.passes;
-    const double row = (double)windows / B < W ? (double)windows / B : (double)W, waves = (double)((items + gkm_sm_count() - 1) / gkm_sm_count());
-    const double table = CT_CALL_US + p.groups * (waves * (CT_ITEM_US + CT_WINDOW_US * row) +
+    const double row = (double)windows / B < W ? (double)windows / B : (double)W, waves = (double)((items + gkm_sm_count() * CT_BLOCKS - 1) / (gkm_sm_count() * CT_BLOCKS));
+    const double queries = (double)(B < p.pass ? B : p.pass);
+    const double table = CT_CALL_US + p.groups * (waves * (CT_ITEM_US + CT_WINDOW_US * row * queries) +
                                                   (double)ix->ct_entries * p.rb / CT_GATHER_BYTES_US);
     double walk = (double)windows * (ix->n_masks * (double)ix->tiles * WALK_LOOKUP_US[wt] +
                                      (double)ix->entries * ix->n_masks / ix->n_lmers * WALK_HIT_US[wt]);
@@ -1160,13 +1297,13 @@ static bool ct_applies(const gkm_index *ix, int64_t B, int64_t W, int64_t window
 extern "C" int gkm_count_table_workspace(const gkm_index_t *ix, int64_t B, int64_t W, int64_t windows, int64_t *bytes)
 {
     if (!ix || !bytes) return gkm_fail(GKM_ERR_INVALID, "null argument");
-    *bytes = ct_applies(ix, B, W, windows) ? ct_plan(ix, B, W).bytes : 0;
+    *bytes = ct_applies(ix, B, W, windows) ? ct_plan(ix, B, W, windows).bytes : 0;
     return GKM_OK;
 }
 
 extern "C" int gkm_count_table_query(const gkm_index_t *ix, const uint32_t *bx, const int32_t *cx, int64_t B,
-                                     int64_t W, const int32_t *order, int32_t normalize, const double *inv_dx,
-                                     double *diag, int64_t diag_offset, double *raw, const double *inv_ds,
+                                     int64_t W, int64_t windows, const int32_t *order, int32_t normalize,
+                                     const double *inv_dx, double *diag, int64_t diag_offset, double *raw, const double *inv_ds,
                                      const double *coef, double gamma, int32_t rbf, double bias, double *scores,
                                      void *workspace, int64_t workspace_bytes, gkm_stream_t stream)
 {
@@ -1179,11 +1316,11 @@ extern "C" int gkm_count_table_query(const gkm_index_t *ix, const uint32_t *bx, 
     if (B == 0) return GKM_OK;
     // (counts stay below 2^32 only where gkm_count_table_workspace says so)
     if (!ix->ct_ids || W > 60000) return gkm_fail(GKM_ERR_UNSUPPORTED, "this index or shape has no count tables");
-    const CtPlan p = ct_plan(ix, B, W);
+    const CtPlan p = ct_plan(ix, B, W, windows);
     if (!workspace || ((uintptr_t)workspace & 255) || workspace_bytes < p.bytes)
         return gkm_fail(GKM_ERR_CAPACITY, "count tables need a 256-byte aligned workspace of %lld bytes", (long long)p.bytes);
     cudaStream_t st = (cudaStream_t)stream;
-    const bool wt = ix->spec.weighted != 0;
+    const bool wt = p.wide;
     CtArgs a = {};
     a.bx = bx;
     a.cx = cx;
@@ -1208,7 +1345,7 @@ extern "C" int gkm_count_table_query(const gkm_index_t *ix, const uint32_t *bx, 
     w += p.c;
     double *partial = (double *)w;
     w += p.partial;
-    uint32_t *recs = (uint32_t *)w;
+    uint8_t *recs = w;
     w += p.recs;
     uint32_t *roff = (uint32_t *)w;
     w += p.roff;
@@ -1216,7 +1353,7 @@ extern "C" int gkm_count_table_query(const gkm_index_t *ix, const uint32_t *bx, 
     a.cap_exc = (unsigned)(p.exc / 8);
     cudaError_t e = cudaMemsetAsync(z0, 0, (size_t)((uint8_t *)partial - z0), st);
     if (e != cudaSuccess) return gkm_cuda_status(e, "count table workspace");
-    a.wd = ix->spec.wd;
+    a.wd = ix->spec.weighted ? ix->spec.wd : nullptr;
     a.off = ix->offsets;
     a.ent = ix->ent;
     a.ent16 = ix->ent16;
@@ -1228,6 +1365,7 @@ extern "C" int gkm_count_table_query(const gkm_index_t *ix, const uint32_t *bx, 
     a.goff = ix->ct_off;
     a.perm = ix->ct_perm;
     a.S = ix->S;
+    a.split = p.split;
     for (int t = 0; t < 4; t++) a.h[t] = t <= a.sh.D ? ix->spec.h[a.sh.D - t] : 0.0;
     a.normalize = normalize;
     a.inv_dx = inv_dx;
@@ -1238,8 +1376,8 @@ extern "C" int gkm_count_table_query(const gkm_index_t *ix, const uint32_t *bx, 
     a.rbf = rbf;
     a.raw = raw;
     a.diag_offset = diag_offset;
-    a.ball = ix->ct_lists + 32 * (CT_R2 + CT_R3);
-    for (int m = 0; m < 4; m++) a.nball[m] = m <= a.sh.D ? ct_ball(a.sh.l - 6, m, nullptr) : 0;
+    a.ball = ix->ct_lists + 32 * CT_ROUNDS;
+    for (int m = 0; m < 4; m++) a.nball[m] = m <= a.sh.D ? ct_ball(a.sh.l - CT_POS, m, nullptr) : 0;
     a.n_pre = p.n_pre;
     a.rec_cap = p.rec_cap;
     for (int64_t g = 0; g < p.groups; g++) {
@@ -1253,33 +1391,28 @@ extern "C" int gkm_count_table_query(const gkm_index_t *ix, const uint32_t *bx, 
             a.pass0 = (int)(g * p.passes);
             const int64_t rows = B - a.r0 < p.chunk * p.qg ? B - a.r0 : p.chunk * p.qg;
             const unsigned n = (unsigned)((rows + p.pass - 1) / p.pass);
-            if (wt) ct_buckets<true><<<n, CT_THREADS, 0, st>>>(a, B);
-            else ct_buckets<false><<<n, CT_THREADS, 0, st>>>(a, B);
+            if (wt) ct_buckets<true><<<n, CB_THREADS, 0, st>>>(a, B);
+            else ct_buckets<false><<<n, CB_THREADS, 0, st>>>(a, B);
             GKM_CHECK_LAUNCH("ct_buckets");
         }
-        a.recs = recs + (g % p.chunk) * p.passes * p.rec_cap;
+        a.recs = recs + (g % p.chunk) * p.passes * p.rec_cap * (wt ? sizeof(ct_rec<true>) : sizeof(ct_rec<false>));
         a.roff = roff + (g % p.chunk) * p.passes * (p.n_pre + 1);
         const int nqp = a.nq < p.pass ? a.nq : p.pass;
-        // two queries (or the one there is) x four levels for the 32-bit recount
+        // four queries (or those there are) x four levels for the 32-bit recount
         int words = wt ? nqp : (nqp + 1) / 2;
-        if (words < 4 * (nqp < 2 ? nqp : 2)) words = 4 * (nqp < 2 ? nqp : 2);
-        a.words = words;
-        a.rec_smem = (int)(p.rec_cap < CT_RECS ? p.rec_cap : CT_RECS);
-        const size_t smem = sizeof(uint32_t) * ((size_t)CT_ROWS * (words + 1) + a.rec_smem);  // + alignment
+        if (words < 4 * (nqp < 4 ? nqp : 4)) words = 4 * (nqp < 4 ? nqp : 4);
+        const size_t smem = sizeof(uint32_t) * (size_t)CT_ROWS * (words + 1);  // + alignment
         a.passes = (a.nq + p.pass - 1) / p.pass;
         a.items = (int)(p.rows / CT_ROWS) * a.passes;
         // a block keeps its pass (its windows stay in L1), the passes of a tile
         // run side by side (their parts of a table row meet in L2)
-        const int sms = gkm_query_blocks();
-        const int fit = sms / a.passes > 0 ? sms / a.passes * a.passes : a.passes;
-        const unsigned grid = (unsigned)(a.items < fit ? a.items : fit);
-        if (wt) {
-            cudaFuncSetAttribute(count_tiles<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-            count_tiles<true><<<grid, CT_THREADS, smem, st>>>(a);
-        } else {
-            cudaFuncSetAttribute(count_tiles<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-            count_tiles<false><<<grid, CT_THREADS, smem, st>>>(a);
-        }
+        const int fit = gkm_query_blocks() * CT_BLOCKS / a.passes * a.passes;
+        const unsigned grid = (unsigned)(a.items < fit ? a.items : fit > 0 ? fit : a.passes);
+        auto count = wt ? count_tiles<true> : count_tiles<false>;
+        // two blocks' shared memory, the rest of the SM's for L1
+        cudaFuncSetAttribute(count, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+        cudaFuncSetAttribute(count, cudaFuncAttributePreferredSharedMemoryCarveout, 86);
+        count<<<grid, CT_THREADS, smem, st>>>(a);
         GKM_CHECK_LAUNCH("count_tiles");
         if (wt) {
             spill_excess<<<(unsigned)gkm_sm_count() * 4, 256, 0, st>>>(a);
@@ -1287,7 +1420,8 @@ extern "C" int gkm_count_table_query(const gkm_index_t *ix, const uint32_t *bx, 
         }
 #define GKM_GATHER_AS(RB, WT, RAW)                                                                        \
     do {                                                                                                  \
-        gather_kernel<RB, WT, RAW><<<p.blocks, G_THREADS, 0, st>>>(a);                                   \
+        if (p.split > 1) gather_kernel<RB, WT, RAW, true><<<p.blocks, G_THREADS, 0, st>>>(a);             \
+        else gather_kernel<RB, WT, RAW, false><<<p.blocks, G_THREADS, 0, st>>>(a);                        \
     } while (0)
 #define GKM_GATHER(RB, WT)                                                                                \
     do {                                                                                                  \

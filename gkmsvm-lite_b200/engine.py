@@ -345,13 +345,13 @@ class DeviceIndex:
         return n.value
 
     def table_query(self, bx, cx, *, work, order=None, normalize=True, inv_dx=None, diag=None, diag_offset=None,
-                    raw=None, inv_ds=None, coef=None, gamma=0.0, rbf=False, bias=0.0, scores=None):
+                    raw=None, inv_ds=None, coef=None, gamma=0.0, rbf=False, bias=0.0, scores=None, windows=0):
         """Scores [B] or K_raw [B, S] (into scores / raw) through count tables,
         exact with no check to settle; diag (nullable) gets the rows' K(x, x).
-        work: a uint8 tensor of table_bytes(B, W)."""
+        work: a uint8 tensor of table_bytes(B, W, windows)."""
         B, W = bx.shape
-        call("gkm_count_table_query", self.handle, ptr(bx), ptr(cx), B, W, ptr(order), int(bool(normalize)),
-             ptr(inv_dx), ptr(diag), -1 if diag_offset is None else int(diag_offset), ptr(raw), ptr(inv_ds),
+        call("gkm_count_table_query", self.handle, ptr(bx), ptr(cx), B, W, int(windows), ptr(order),
+             int(bool(normalize)), ptr(inv_dx), ptr(diag), -1 if diag_offset is None else int(diag_offset), ptr(raw), ptr(inv_ds),
              ptr(coef), float(gamma), int(rbf), float(bias), ptr(scores), ptr(work), int(work.numel()), _st())
 
     def rows(self, bx, rx, cx, normalize, *, diag_offset=None, out=None, check=True, windows=0, work=None):
@@ -367,7 +367,7 @@ class DeviceIndex:
         if out is None:
             out = torch.empty((B, self.S), dtype=torch.float64, device=bx.device)
         diag = torch.empty(B, dtype=torch.float64, device=bx.device) if normalize else None
-        self.table_query(bx, cx, work=tw, diag=diag, diag_offset=diag_offset, raw=out)
+        self.table_query(bx, cx, work=tw, diag=diag, diag_offset=diag_offset, raw=out, windows=windows)
         return out, diag
 
     def scores(self, bx, rx, cx, normalize, inv_ds, coef, gamma, rbf, bias, order=None, *, windows=0, work=None):
@@ -379,7 +379,7 @@ class DeviceIndex:
             return None
         out = torch.empty(B, dtype=torch.float64, device=bx.device)
         self.table_query(bx, cx, work=tw, order=order, normalize=normalize, inv_ds=inv_ds, coef=coef, gamma=gamma,
-                         rbf=rbf, bias=bias, scores=out)
+                         rbf=rbf, bias=bias, scores=out, windows=windows)
         return out
 
     def count(self, bx, cx):

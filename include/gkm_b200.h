@@ -183,7 +183,8 @@ int gkm_index_count(const gkm_index_t *index, const uint32_t *bx, const int32_t 
  * every l-mer, then per SV the sum of its windows' table rows; exact (no event
  * counts to read).  gkm_count_table_workspace: *bytes of device workspace a
  * call over B rows of W window slots needs, 0 where the walk serves it
- * (windows: all rows' windows, <= 0 unknown).  order (nullable): the order
+ * (windows: all rows' windows, <= 0 unknown; the query's must be the same, or
+ * unknown).  order (nullable): the order
  * rows are grouped in (longest first).  diag [B] (nullable): the rows'
  * K(x, x).  Either raw [B, S], with diag_offset as in gkm_index_pairwise (order
  * then null), or scores [B] as in gkm_index_score, normalised by inv_dx [B] or,
@@ -193,10 +194,10 @@ int gkm_index_count(const gkm_index_t *index, const uint32_t *bx, const int32_t 
  * raw_diag_packed of the query rows (kernels/direct.py:109-137). */
 int gkm_count_table_workspace(const gkm_index_t *index, int64_t B, int64_t W, int64_t windows, int64_t *bytes);
 int gkm_count_table_query(const gkm_index_t *index, const uint32_t *bx, const int32_t *cx, int64_t B, int64_t W,
-                          const int32_t *order, int32_t normalize, const double *inv_dx, double *diag,
-                          int64_t diag_offset, double *raw, const double *inv_ds, const double *coef, double gamma,
-                          int32_t rbf, double bias, double *scores, void *workspace, int64_t workspace_bytes,
-                          gkm_stream_t stream);
+                          int64_t windows, const int32_t *order, int32_t normalize, const double *inv_dx,
+                          double *diag, int64_t diag_offset, double *raw, const double *inv_ds, const double *coef,
+                          double gamma, int32_t rbf, double bias, double *scores, void *workspace,
+                          int64_t workspace_bytes, gkm_stream_t stream);
 
 /* V[v] = sum over index entries of l-mer v of c_sv[sv] times the entry's
  * window weight, [4^l].
