@@ -75,6 +75,8 @@ SIGNATURES = {
     "gkm_mutant_diag": [SPEC, P, P, I64, I64, I64, P, P, P],
     "gkm_ism_table": [SPEC, P, P, P, I64, I64, I64, P, P, P, I32, P, P],
     "gkm_index_mutants_workspace": [P, I64, I64, P, P],
+    "gkm_ism_pairs_workspace": [P, I64, I64, P],
+    "gkm_ism_pairs": [P, P, P, I64, I64, I64, P, P, P, P, P, D, I32, P, P, I64, P],
     "gkm_index_mutants": [P, P, P, I64, I64, I64, P, P, P, P, P, P, D, I32, P, P, I64, P],
     "gkm_raw_score": [P, I64, I64, P, P, P, D, I32, D, P, P],
     "gkm_impact": [P, I64, I64, P, P, P, D, I32, P, P],

@@ -136,6 +136,43 @@ struct gkm_index {
     int64_t ct_entries;
 };
 
+// Rows of a table over l-mers (count tables, pair lists): odd l with both strands
+// folds a window and its reverse complement into one row.
+struct gkm_rows {
+    int l, D, fold, strands, mid;
+    // l-mer -> table row.  fold: the middle position keeps one bit (A / C),
+    // moved to the top; the other positions stay in order.
+    __host__ __device__ __forceinline__ uint32_t row(uint32_t u) const
+    {
+        if (!fold) return u;
+        const uint32_t low = (1u << (2 * mid)) - 1u;
+        return (u & low) | ((u >> 2) & ~low & ((1u << (2 * (l - 1))) - 1u)) | (((u >> (2 * mid)) & 1u) << (2 * (l - 1)));
+    }
+    __host__ __device__ __forceinline__ uint32_t lmer(uint32_t r) const
+    {
+        if (!fold) return r;
+        const uint32_t low = (1u << (2 * mid)) - 1u, top = (1u << (2 * (l - 1))) - 1u;
+        return (r & low) | (((r & top) & ~low) << 2) | ((r >> (2 * (l - 1))) << (2 * mid));
+    }
+};
+
+inline gkm_rows gkm_rows_of(const gkm_index *ix)
+{
+    gkm_rows sh;
+    sh.l = ix->spec.l;
+    sh.D = ix->spec.dmax;
+    sh.strands = ix->strands;
+    sh.fold = ix->strands == 2 && (sh.l & 1);
+    sh.mid = sh.l / 2;
+    return sh;
+}
+
+inline int64_t gkm_row_count(const gkm_index *ix)
+{
+    const gkm_rows sh = gkm_rows_of(ix);
+    return sh.fold ? (int64_t)1 << (2 * sh.l - 1) : (int64_t)1 << (2 * sh.l);
+}
+
 // Built with the index / freed with it (gkm_count_table.cu).
 int gkm_ct_build(gkm_index *ix, const uint32_t *fwd, const int32_t *counts, cudaStream_t st);
 void gkm_ct_free(gkm_index *ix);

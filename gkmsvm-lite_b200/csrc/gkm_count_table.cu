@@ -78,24 +78,6 @@ __device__ __forceinline__ uint32_t ct_swap(uint32_t plane)
     return (plane >> 2) << 3;
 }
 
-struct CtShape {
-    int l, D, fold, strands, mid;
-    // l-mer -> table row.  fold: the middle position keeps one bit (A / C),
-    // moved to the top; the other positions stay in order.
-    __host__ __device__ __forceinline__ uint32_t row(uint32_t u) const
-    {
-        if (!fold) return u;
-        const uint32_t low = (1u << (2 * mid)) - 1u;
-        return (u & low) | ((u >> 2) & ~low & ((1u << (2 * (l - 1))) - 1u)) | (((u >> (2 * mid)) & 1u) << (2 * (l - 1)));
-    }
-    __host__ __device__ __forceinline__ uint32_t lmer(uint32_t r) const
-    {
-        if (!fold) return r;
-        const uint32_t low = (1u << (2 * mid)) - 1u, top = (1u << (2 * (l - 1))) - 1u;
-        return (r & low) | (((r & top) & ~low) << 2) | ((r >> (2 * (l - 1))) << (2 * mid));
-    }
-};
-
 struct CtArgs {
     const uint32_t *bx;
     const int32_t *cx;
@@ -106,7 +88,7 @@ struct CtArgs {
     int qg;      // queries a table row holds
     int rb;      // bytes of a table row
     int items, passes;  // (tile, pass of queries) items of the group, passes per tile
-    CtShape sh;
+    gkm_rows sh;
     const uint32_t *lists;  // neighbour masks of the six suffix positions by bank class
     const uint32_t *ball;   // masks of the other positions by mismatches
     int nball[4];           // how many of each
@@ -221,7 +203,7 @@ template <bool WT>
 using ct_rec = std::conditional_t<WT, uint32_t, uint16_t>;
 
 template <bool WT>
-__device__ __forceinline__ ct_rec<WT> ct_record(const CtShape &sh, uint32_t v, int q, uint32_t w, uint32_t *pre)
+__device__ __forceinline__ ct_rec<WT> ct_record(const gkm_rows &sh, uint32_t v, int q, uint32_t w, uint32_t *pre)
 {
     uint32_t c = v;  // the l-mer without its middle base, which goes on top (fold)
     if (sh.fold) {
@@ -342,7 +324,7 @@ __global__ void __launch_bounds__(CT_THREADS, CT_BLOCKS) count_tiles(CtArgs a)
     const uint32_t raw0 = (uint32_t)__cvta_generic_to_shared(ct_smem), cbase = (raw0 + PLANE - 1u) & ~(PLANE - 1u);
     uint32_t *cnt = (uint32_t *)(ct_smem + (cbase - raw0));
     const int lane = threadIdx.x & 31, warp = __shfl_sync(GKM_FULL, threadIdx.x >> 5, 0);  // (known to be uniform)
-    const CtShape sh = a.sh;
+    const gkm_rows sh = a.sh;
     const int D = sh.D;
     // a mask: byte offset and increment (0: none in this round)
     auto entry = [&](uint32_t e) -> uint2 {
@@ -1014,7 +996,7 @@ __global__ void ct_padded(const int32_t *__restrict__ counts, const uint32_t *__
 // One SV per block: its windows' table rows in rising order (neighbouring SVs
 // then sweep the table together, which keeps the rows they share in L2), padded
 // with the zero row.
-__global__ void ct_rows(CtShape sh, const uint32_t *__restrict__ fwd, const int32_t *__restrict__ counts, int64_t W,
+__global__ void ct_rows(gkm_rows sh, const uint32_t *__restrict__ fwd, const int32_t *__restrict__ counts, int64_t W,
                         const uint32_t *__restrict__ perm, const uint32_t *__restrict__ goff, uint32_t zero_row,
                         const uint8_t *__restrict__ wd, uint32_t *__restrict__ ids, uint8_t *__restrict__ wts)
 {
@@ -1061,23 +1043,6 @@ __global__ void ct_rows(CtShape sh, const uint32_t *__restrict__ fwd, const int3
 // Host side
 // ---------------------------------------------------------------------------
 
-static CtShape ct_shape(const gkm_index *ix)
-{
-    CtShape sh;
-    sh.l = ix->spec.l;
-    sh.D = ix->spec.dmax;
-    sh.strands = ix->strands;
-    sh.fold = ix->strands == 2 && (sh.l & 1);
-    sh.mid = sh.l / 2;
-    return sh;
-}
-
-static int64_t ct_table_rows(const gkm_index *ix)
-{
-    const CtShape sh = ct_shape(ix);
-    return sh.fold ? (int64_t)1 << (2 * sh.l - 1) : (int64_t)1 << (2 * sh.l);
-}
-
 // Neighbour masks of the suffix positions with 0 .. b mismatches for b = 1 ..
 // 3, arranged so that lane k of every round holds a mask of bank class k (budget 1:
 // the 16 masks twice): position | t << 12, or bit 31.
@@ -1118,7 +1083,7 @@ static int ct_ball(int n, int m, uint32_t *out)
 int gkm_ct_build(gkm_index *ix, const uint32_t *fwd, const int32_t *counts, cudaStream_t st)
 {
     ix->ct_ids = nullptr;
-    const CtShape sh = ct_shape(ix);
+    const gkm_rows sh = gkm_rows_of(ix);
     // 16-bit gather sums (31 x windows) and the in-block sort bound the SV rows;
     // weighted entries are bytes: three windows of the largest weight fit
     if (sh.l < 8 || sh.l > 11 || sh.D < 0 || sh.D > 3 || ix->W > 2048 || ix->S < 64 || ix->wmax > 85) return GKM_OK;
@@ -1164,7 +1129,7 @@ int gkm_ct_build(gkm_index *ix, const uint32_t *fwd, const int32_t *counts, cuda
         int m = 1;
         while (m < ix->W) m <<= 1;
         ct_rows<<<(unsigned)S, m >= 512 ? 256 : m >= 64 ? m / 2 : 32, sizeof(uint32_t) * m, st>>>(
-            sh, fwd, counts, ix->W, ix->ct_perm, ix->ct_off, (uint32_t)ct_table_rows(ix),
+            sh, fwd, counts, ix->W, ix->ct_perm, ix->ct_off, (uint32_t)gkm_row_count(ix),
             ix->spec.weighted ? ix->spec.wd : nullptr, ix->ct_ids, ix->ct_wts);
         cudaError_t e = cudaGetLastError();
         if (e != cudaSuccess) s = gkm_cuda_status(e, "gather lists");
@@ -1226,7 +1191,7 @@ static CtPlan ct_plan(const gkm_index *ix, int64_t B, int64_t W, int64_t windows
     while (p.rb > 32 && p.rb / wt / 2 >= B) p.rb /= 2;
     p.qg = p.rb / wt;
     p.groups = (B + p.qg - 1) / p.qg;
-    p.rows = ct_table_rows(ix);
+    p.rows = gkm_row_count(ix);
     const int per_sm = p.wide ? G_BLOCKS_W : G_BLOCKS;
     p.blocks = gkm_query_blocks() * per_sm;
     // few SVs: a power of two of lane groups within a warp for each (2,000 SVs of 200 ..
@@ -1328,7 +1293,7 @@ extern "C" int gkm_count_table_query(const gkm_index_t *ix, const uint32_t *bx, 
     a.order = order;
     a.qg = p.qg;
     a.rb = p.rb;
-    a.sh = ct_shape(ix);
+    a.sh = gkm_rows_of(ix);
     a.lists = ix->ct_lists;
     uint8_t *w = (uint8_t *)workspace;
     // the zero row, self counts, excess list lengths, dirty bits and excess counts start at zero

@@ -3,8 +3,9 @@
 Window-delta form: a substitution at p changes only the <= l windows that
 cover p.  Kernels with an l-mer table read the changed windows' table weights
 and the mutant self-kernels in one fused pass (gkm_ism_table); other kernels
-(RBF) add the changed windows' index hits to the reference row's kernel
-values and reduce over the SVs per mutant (gkm_index_mutants).
+(RBF) count the window pairs each substitution changes once per SV and reduce
+over the SVs (gkm_ism_pairs), or where that does not apply add the changed
+windows' index hits to the reference row's kernel values (gkm_index_mutants).
 """
 
 from __future__ import annotations
@@ -77,8 +78,11 @@ def _ism_index(model, fwd, rc, counts, L, check=True, work=None, table_work=None
     rbf = isinstance(kernel, RbfKernel)
     gamma = kernel.gamma if rbf else 0.0
     out = torch.empty((B, 4, L), dtype=torch.float64, device=fwd.device)
+    pairs = ctypes.c_int64()
+    call("gkm_ism_pairs_workspace", index.handle, W, L, ctypes.byref(pairs))
     if work is None:
-        work = ism_workspace(model, B, L, fwd.device)
+        work = (torch.empty(pairs.value, dtype=torch.uint8, device=fwd.device) if pairs.value
+                else ism_workspace(model, B, L, fwd.device))
 
     def run():
         # the reference rows' K_raw; their scores come from it inside the call
@@ -90,6 +94,11 @@ def _ism_index(model, fwd, rc, counts, L, check=True, work=None, table_work=None
         else:
             inv_dx = torch.ones(B, dtype=torch.float64, device=fwd.device)
             inv_dmut = torch.ones((4, L, B), dtype=torch.float64, device=fwd.device)
+        if 0 < pairs.value <= work.numel():
+            call("gkm_ism_pairs", index.handle, ptr(fwd), ptr(counts), B, W, L, ptr(ref_raw), ptr(inv_dx),
+                 ptr(inv_dmut), ptr(model._inv_ds()), ptr(model._sv_coef()), float(gamma), int(rbf), ptr(out),
+                 ptr(work), int(work.numel()), stream_handle())
+            return out
         call("gkm_index_mutants", index.handle, ptr(fwd), ptr(counts), B, W, L, ptr(ref_raw), None,
              ptr(inv_dx), ptr(inv_dmut), ptr(model._inv_ds()), ptr(model._sv_coef()), float(gamma), int(rbf),
              ptr(out), ptr(work), int(work.numel()), stream_handle())

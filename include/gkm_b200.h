@@ -265,6 +265,17 @@ int gkm_index_mutants(const gkm_index_t *index, const uint32_t *fwd, const int32
                       double gamma, int32_t rbf, double *out, void *workspace,
                       int64_t workspace_bytes, gkm_stream_t stream);
 
+/* The same deltas from one pass over the window pairs of each row and SV within
+ * dmax + 1 mismatches, without K of every (mutant, SV).  gkm_ism_pairs_workspace:
+ * *bytes of device workspace (256-byte aligned, used until the call completes), 0
+ * where gkm_index_mutants serves rows of W windows and L positions.  inv_dx [B]:
+ * 1 / sqrt(K(x, x)) (1 unnormalised). */
+int gkm_ism_pairs_workspace(const gkm_index_t *index, int64_t W, int64_t L, int64_t *bytes);
+int gkm_ism_pairs(const gkm_index_t *index, const uint32_t *fwd, const int32_t *counts, int64_t B, int64_t W,
+                  int64_t L, const double *ref_raw, const double *inv_dx, const double *inv_dmut,
+                  const double *inv_ds, const double *coef, double gamma, int32_t rbf, double *out,
+                  void *workspace, int64_t workspace_bytes, gkm_stream_t stream);
+
 /* scores[b] = sum_s coef[s] f(raw[b, s] / max(sqrt(dx[b] ds[s]), 1e-10)) + bias
  * over a materialised [B, S] block (dx, ds nullable: no normalisation).
  * Replaces _normalized_dot (svm.py:42-61). */
