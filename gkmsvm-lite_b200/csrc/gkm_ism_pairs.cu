@@ -151,27 +151,47 @@ __global__ void __launch_bounds__(PL_THREADS) pair_lists(PairArgs a)
     }
 }
 
-// Bytes of shared memory per position: G, C twice (cleared while the other is in
-// use), both strands' words, weight.
-constexpr int PG_BYTES = 64 + 2 * 16 + 8 + 1;
+// Shared-memory add where m is not zero (predicated rather than branched around).
+__device__ __forceinline__ void pair_add(uint32_t m, uint32_t addr, uint32_t v)
+{
+    asm volatile("{\n\t.reg .pred p;\n\tsetp.ne.u32 p, %0, 0;\n\t@p red.shared.add.u32 [%1], %2;\n\t}" ::"r"(m), "r"(addr),
+                 "r"(v)
+                 : "memory");
+}
+
+// A two's complement word as a double: placed in the mantissa of 2^52 with its sign bit
+// flipped, exactly.
+__device__ __forceinline__ double pair_double(uint32_t x)
+{
+    return __hiloint2double(0x43300000, (int)(x ^ 0x80000000u)) - 4503601774854144.0;  // 2^52 + 2^31
+}
+
+// Shared memory of a gather block: G (16 planes of a multiple of 32 positions: most
+// pairs have the same t, so that a position's counters side by side would leave 8 of
+// the 32 banks to them), C twice (cleared while the other is in use), both strands'
+// words, weights.
+__host__ __device__ __forceinline__ int64_t pg_plane(int64_t L) { return (L + 31) & ~(int64_t)31; }
+inline size_t pg_bytes(int64_t L) { return (size_t)(64 * pg_plane(L) + (2 * 16 + 8 + 1) * L); }
 
 // One block per SV at a time; thread t has positions t and t + T of every SV, their
 // normalisers and sums in registers.  Bound by instruction issue (181M pairs at 500 bp
 // against 72,000 SVs of 350 bp).  Measured there: the walk and its reduction 7.1 ms,
-// lists, gather and sums 2.5 ms.
+// lists, gather and sums 2.2 ms (with a position's 16 counters side by side 2.4).
 template <int T, bool WT>
 __global__ void __launch_bounds__(T, 1024 / T) pair_gather(PairArgs a)
 {
     extern __shared__ __align__(16) uint8_t pg_smem[];
     constexpr int WARPS = T / 32;
+    __shared__ uint2 slot_s[WARPS][32];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const gkm_rows sh = a.sh;
     const int l = sh.l, n = a.counts[a.b], P = n > 0 ? n + l - 1 : 0;
-    uint4 *G = (uint4 *)pg_smem;  // [P][base]: four t
-    uint4 *C = G + 4 * a.L;       // [2][n]: four m
+    const uint32_t plane = (uint32_t)pg_plane(a.L);
+    uint32_t *G = (uint32_t *)pg_smem;    // [base][t][plane]
+    uint4 *C = (uint4 *)(G + 16 * plane);  // [2][n]: four m
     uint32_t *word = (uint32_t *)(C + 2 * a.L);  // [2][n]
     uint8_t *wx = (uint8_t *)(word + 2 * a.L);
-    for (int k = threadIdx.x; k < 4 * P + 2 * n; k += T) (k < 4 * P ? G : C - 4 * P)[k] = make_uint4(0, 0, 0, 0);
+    for (int k = threadIdx.x; k < 4 * (int)plane + 2 * n; k += T) ((uint4 *)G)[k] = make_uint4(0, 0, 0, 0);  // (and C)
     for (int i = threadIdx.x; i < n; i += T) {
         const uint32_t v = a.fwd[a.b * a.W + i];
         word[i] = v;
@@ -193,7 +213,8 @@ __global__ void __launch_bounds__(T, 1024 / T) pair_gather(PairArgs a)
         }
     }
     const double zx = a.inv_dx[a.b];
-    uint32_t *Gw = (uint32_t *)G;
+    const uint32_t gbase = (uint32_t)__cvta_generic_to_shared(G);
+    uint2 *slot = slot_s[warp];
     int par = 0;
     for (int64_t g = blockIdx.x; g < a.S && P > 0; g += gridDim.x, par ^= 1) {
         const uint32_t p0 = a.goff[g], wins = a.goff[g + 1] - p0;
@@ -215,38 +236,42 @@ __global__ void __launch_bounds__(T, 1024 / T) pair_gather(PairArgs a)
                 const uint32_t y = __shfl_up_sync(GKM_FULL, upto, o);
                 if (lane >= o) upto += y;
             }
-            beg -= upto - len;  // entry h of the chunk is ents[beg + h]
-            const uint32_t all = __shfl_sync(GKM_FULL, upto, 31);
-            // pair h of the chunk: its window's lane and its entry
-            auto fetch = [&](uint32_t h, int &b) -> uint32_t {
-                b = 0;  // windows that end at or before h
-#pragma unroll
-                for (int o = 16; o; o >>= 1)
-                    if (__shfl_sync(GKM_FULL, upto, b + o - 1) <= h) b += o;
-                const uint32_t at = __shfl_sync(GKM_FULL, beg, b) + h;
-                return h < all ? (uint32_t)__ldg(a.ents + at) : 0u;
+            const uint32_t all = __shfl_sync(GKM_FULL, upto, 31), start = upto - len;
+            // the windows with pairs, side by side: pair h of the chunk is entry .x + h
+            // (in 32 bits: .x may lie below zero)
+            const uint32_t some = __ballot_sync(GKM_FULL, len != 0);
+            if (len) slot[__popc(some & ((1u << lane) - 1u))] = make_uint2(beg - start, u | ws << 24);
+            __syncwarp();
+            // Pairs h0 + lane: their window is the last one that starts at or before
+            // them, found by counting starts.
+            uint32_t begun = 0;
+            uint2 win;
+            auto fetch = [&](uint32_t h0) -> uint32_t {
+                const uint32_t at = start - h0, starts = __reduce_or_sync(GKM_FULL, len && at < 32 ? 1u << at : 0u);
+                win = slot[(begun + __popc(starts & (0xFFFFFFFFu >> (31 - lane))) - 1u) & 31u];
+                begun += __popc(starts);
+                return h0 + lane < all ? (uint32_t)__ldg(a.ents + (win.x + (h0 + lane))) : 0u;
             };
-            int b;
-            uint32_t e = fetch(lane, b);
+            uint32_t e = fetch(0);
             for (uint32_t h0 = 0; h0 < all; h0 += 32) {
-                const uint32_t uu = __shfl_sync(GKM_FULL, u, b), inc = WT ? __shfl_sync(GKM_FULL, ws, b) : 1u;
-                const uint32_t now = e;
+                const uint32_t now = e, uu = win.y & 0xFFFFFFu, i = now & 0x7FFFu, st = now >> 15;
                 const bool in = h0 + lane < all;
-                e = fetch(h0 + 32 + lane, b);  // in flight meanwhile
-                if (in) {
-                    const uint32_t i = now & 0x7FFFu, st = now >> 15, x = uu ^ word[i + (st ? n : 0)];
-                    uint32_t m = (x | (x >> 1)) & 0x55555555u;
-                    const uint32_t nm = __popc(m), w = WT ? inc * wx[i] : 1u;
-                    if ((int)nm <= sh.D) atomicAdd(Cw + 4 * i + nm, w);
-                    // strand 1 reads the row backwards, complemented
-                    const uint32_t from = i + (st ? l - 1 : 0), ub = st ? ~uu : uu;
-                    while (m) {
-                        const int bit = __ffs(m) - 1, j = bit >> 1;
-                        m &= m - 1;
-                        atomicAdd(Gw + 16 * (st ? from - j : from + j) + 4 * ((ub >> bit) & 3u) + nm - 1, w);
-                    }
+                const uint32_t w = WT ? (win.y >> 24) * wx[i] : 1u;
+                e = fetch(h0 + 32);  // in flight meanwhile
+                const uint32_t x = uu ^ word[i + (st ? n : 0)];
+                uint32_t m = in ? (x | (x >> 1)) & 0x55555555u : 0u;
+                const uint32_t nm = __popc(m);
+                if (in && (int)nm <= sh.D) atomicAdd(Cw + 4 * i + nm, w);
+                // strand 1 reads the row backwards, complemented
+                const uint32_t to = gbase + 4 * (i + (st ? l - 1 : 0) + plane * (nm - 1)), step = st ? -2 : 2, ub = st ? ~uu : uu;
+#pragma unroll
+                for (int k = 0; k < 4; k++) {
+                    const uint32_t bit = 31 - __clz(m);
+                    pair_add(m, to + step * bit + 16 * plane * ((ub >> (bit & 31u)) & 3u), w);
+                    m &= ~(1u << (bit & 31u));
                 }
             }
+            __syncwarp();
         }
         __syncthreads();
         const int64_t s = a.perm[g];
@@ -264,17 +289,19 @@ __global__ void __launch_bounds__(T, 1024 / T) pair_gather(PairArgs a)
             uint32_t own[3][4];
 #pragma unroll
             for (int k = 0; k < 3; k++) {
-                uint4 *at = G + 4 * p + k + (k >= xp[q]);
-                const uint4 v = *at;
-                *at = make_uint4(0, 0, 0, 0);
-                own[k][0] = v.x, own[k][1] = v.y, own[k][2] = v.z, own[k][3] = v.w;
-                t[1] -= v.x, t[2] -= v.y, t[3] -= v.z;
+                uint32_t *at = G + 4 * plane * (k + (k >= xp[q])) + p;
+#pragma unroll
+                for (int j = 0; j < 4; j++) {
+                    own[k][j] = at[j * plane];
+                    at[j * plane] = 0;
+                    if (j < 3) t[j + 1] -= own[k][j];
+                }
             }
 #pragma unroll
             for (int k = 0; k < 3; k++) {
                 double d = ref;
 #pragma unroll
-                for (int j = 0; j < 4; j++) d += a.dh[j] * ((double)own[k][j] - (double)t[j]);
+                for (int j = 0; j < 4; j++) d += a.dh[j] * pair_double(own[k][j] - t[j]);
                 const double kn = d * z[q][k] * ds;
                 sum[q][k] += co * (a.rbf ? exp(a.gamma * (kn - 1.0)) : kn);
             }
@@ -342,7 +369,7 @@ static bool pair_plan(const gkm_index *ix, int64_t W, int64_t L, PairPlan &p)
     // an SV's G and C fit shared memory
     if (!ix->ct_ids || W < 1 || L > 2048 || W > L) return false;
     p.threads = L <= 512 ? 256 : L <= 1024 ? 512 : 1024;
-    p.smem = (size_t)PG_BYTES * L;
+    p.smem = pg_bytes(L);
     if ((int64_t)p.smem > gkm_smem_limit()) return false;
     p.blocks = gkm_sm_count() * (1024 / p.threads);
     p.tiles = gkm_row_count(ix) / PL_ROWS;
