@@ -575,6 +575,52 @@ __global__ void __launch_bounds__(CT_THREADS, CT_BLOCKS) count_tiles(CtArgs a)
     // apart, write the quarters of a row, so that a store writes eight rows side by
     // side.  The words are summed by carry-save adders (two logic operations a word)
     // and the fields of the six sums added up.
+    // sum of a word's fields (unweighted: t = 0 and 1 are the bytes' low fields, t = 3
+    // and 2 the high ones, 32 and 16 times too large)
+    auto field_sum = [](uint32_t w) -> uint32_t {
+        return WT ? __dp4a(w >> 9, 0x00010101u, w & 0x1FFu)
+                  : __dp4a(w & 0x0F1F0F1Fu, 0x01010101u, __dp4a(w & 0xF0E0F0E0u, 0x02010201u, 0u) >> 5);
+    };
+    auto queue = [&](uint32_t at, uint32_t w) {
+        const int n = atomicAdd(&nlist[par], 1);
+        if (n < CT_LIST) {
+            list_at[par][n] = (uint16_t)at;
+            list_w[par][n] = w;
+        }
+    };
+    auto check = [&](uint32_t sum) {
+        const uint32_t wsum = __reduce_add_sync(GKM_FULL, sum), wadds = __reduce_add_sync(GKM_FULL, adds);
+        if (lane == 0) {
+            atomicAdd(&chk[par][0], wsum);
+            atomicAdd(&chk[par][1], wadds);
+        }
+    };
+    // narrow rows (a few queries): a row per thread
+    auto write_few = [&]() {
+        uint32_t sum = 0;
+#pragma unroll
+        for (int i = 0; i < CT_ROWS / CT_THREADS; i++) {
+            const uint32_t p = i * CT_THREADS + threadIdx.x;
+            uint32_t w[4], any = 0;
+#pragma unroll
+            for (int j = 0; j < 4; j++) {
+                w[j] = j < words ? cnt[j * CT_ROWS + p] : 0u;
+                sum += field_sum(w[j]);
+                any |= w[j];
+            }
+            if (any & slow_mask)
+#pragma unroll
+                for (int j = 0; j < 4; j++)
+                    if (w[j] & slow_mask) queue(j * CT_ROWS + p, w[j]);
+            if (WT)
+#pragma unroll
+                for (int j = 0; j < 4; j++) w[j] = (w[j] & 0xFFu) | ((w[j] >> 1) & 0xFFFFFF00u);
+            uint8_t *T = a.T + ((size_t)tile * CT_ROWS + ct_phys(p)) * a.rb;
+            if (a.rb == 8) *(uint2 *)T = make_uint2(w[0], w[1]);
+            else *(uint4 *)T = make_uint4(w[0], w[1], w[2], w[3]);
+        }
+        check(sum);
+    };
     auto write_tile = [&](auto FULL) {
         constexpr bool full = decltype(FULL)::value;  // every word of a row is counted and stored
         const int part = (lane >> 3) & 3, j0 = 4 * part;
@@ -615,10 +661,7 @@ __global__ void __launch_bounds__(CT_THREADS, CT_BLOCKS) count_tiles(CtArgs a)
         for (int k = 0; k < 6; k++) {
             const uint32_t w = sums[k];
             any |= w;
-            // (unweighted: t = 0 and 1 are the bytes' low fields, t = 3 and 2 the high
-            // ones, 32 and 16 times too large)
-            sum += (WT ? __dp4a(w >> 9, 0x00010101u, w & 0x1FFu)
-                       : __dp4a(w & 0x0F1F0F1Fu, 0x01010101u, __dp4a(w & 0xF0E0F0E0u, 0x02010201u, 0u) >> 5)) << k;
+            sum += field_sum(w) << k;
         }
         // a lane that saw such a word: its 32 words again, one per lane
         for (uint32_t some = __ballot_sync(GKM_FULL, (any & slow_mask) != 0); some; some &= some - 1) {
@@ -626,20 +669,12 @@ __global__ void __launch_bounds__(CT_THREADS, CT_BLOCKS) count_tiles(CtArgs a)
             const int j = ((from >> 3) & 3) * 4 + (lane & 3),
                       pos = ((lane >> 4) * CT_THREADS + warp * 32 + from) ^ (2 * (lane & 12));
             const uint32_t w = j < words ? cnt[j * CT_ROWS + pos] : 0u;
-            if (!(w & slow_mask)) continue;
-            const int n = atomicAdd(&nlist[par], 1);
-            if (n < CT_LIST) {
-                list_at[par][n] = (uint16_t)(j * CT_ROWS + pos);
-                list_w[par][n] = w;
-            }
+            if (w & slow_mask) queue(j * CT_ROWS + pos, w);
         }
-        const uint32_t wsum = __reduce_add_sync(GKM_FULL, sum), wadds = __reduce_add_sync(GKM_FULL, adds);
-        if (lane == 0) {
-            atomicAdd(&chk[par][0], wsum);
-            atomicAdd(&chk[par][1], wadds);
-        }
+        check(sum);
     };
-    if (words == CT_SLOTS && a.rb >= 4 * CT_SLOTS) write_tile(std::true_type{});
+    if (words <= 4 && a.rb <= 16) write_few();
+    else if (words == CT_SLOTS && a.rb >= 4 * CT_SLOTS) write_tile(std::true_type{});
     else write_tile(std::false_type{});
     __syncthreads();
 
@@ -750,17 +785,30 @@ __device__ __forceinline__ void ct_finish(const CtArgs &a, int64_t s, int j0, co
     }
 }
 
-// RB-byte rows, 16 bytes per lane, RB / 16 lanes per SV; persistent blocks take
+__device__ __forceinline__ void ct_load(uint32_t (&r)[4], const uint8_t *p)
+{
+    const uint4 v = __ldg((const uint4 *)p);
+    r[0] = v.x, r[1] = v.y, r[2] = v.z, r[3] = v.w;
+}
+
+__device__ __forceinline__ void ct_load(uint32_t (&r)[2], const uint8_t *p)
+{
+    const uint2 v = __ldg((const uint2 *)p);
+    r[0] = v.x, r[1] = v.y;
+}
+
+// RB-byte rows, 16 bytes (RB = 8: 8) per lane, RB / 16 lanes per SV; persistent blocks take
 // SVs round robin in gather order (long SVs first); where there are fewer SVs than
-// lane groups, `split` groups share an SV's windows.  Bound by L2 and HBM latency
-// times bandwidth: every lane keeps two stages of eight row pieces in flight in
-// its own slots of shared memory (asynchronous copies; nothing is shared between
-// lanes, so no barriers) while it adds a third.
+// lane groups, `split` groups share an SV's windows.  Bound by L1's line lookups where
+// L2 holds the table (24.5M rows at one per clock and SM are 87 us; one query 112 us),
+// by L2 and HBM past it (32 queries: 172 us in 64-byte, weighted 290 us in 128-byte
+// rows).
 template <int RB, bool WT, bool RAW, bool SPLIT>
 __global__ void __launch_bounds__(G_THREADS, WT ? G_BLOCKS_W : G_BLOCKS) gather_kernel(CtArgs a)
 {
-    constexpr int NQ = WT ? 4 : 8;  // queries a lane owns
-    constexpr int LPG = RB / 16, QG = LPG * NQ;
+    constexpr int NW = RB < 16 ? RB / 4 : 4;     // words a lane loads of a row
+    constexpr int NQ = WT ? NW : 2 * NW;         // queries a lane owns
+    constexpr int LPG = RB / (4 * NW), QG = LPG * NQ;
     const int split = SPLIT ? a.split : 1, lanes = LPG * split, GPB = G_THREADS / lanes;  // lanes per SV, SVs per block
     __shared__ uint4 rows_s[4 * G_THREADS];
     __shared__ double inv_dx[QG];
@@ -787,7 +835,7 @@ __global__ void __launch_bounds__(G_THREADS, WT ? G_BLOCKS_W : G_BLOCKS) gather_
     }
     for (int j = threadIdx.x; j < G_THREADS / 32 * QG; j += G_THREADS) (&part_s[0][0])[j] = 0.0;
     some = __syncthreads_or(some);
-    const uint8_t *base = a.T + sub * 16;
+    const uint8_t *base = a.T + sub * 4 * NW;
     const int64_t rounds = (a.S + (int64_t)gridDim.x * GPB - 1) / ((int64_t)gridDim.x * GPB);
     for (int64_t it = 0; it < rounds; it++) {
         const int64_t g = (it * gridDim.x + blockIdx.x) * GPB + threadIdx.x / lanes;
@@ -805,38 +853,34 @@ __global__ void __launch_bounds__(G_THREADS, WT ? G_BLOCKS_W : G_BLOCKS) gather_
             id[4] = i1.x, id[5] = i1.y, id[6] = i1.z, id[7] = i1.w;
         };
         load_ids(turn);
-        uint32_t acc[16];  // WT: [query][t]; else [word][t], two 16-bit sums each
+        uint32_t acc[4 * NW];  // WT: [query][t]; else [word][t], two 16-bit sums each
 #pragma unroll
-        for (int k = 0; k < 16; k++) acc[k] = 0;
+        for (int k = 0; k < 4 * NW; k++) acc[k] = 0;
         // 16 bits per query: carry-save adders over the 32-bit words sum rows with
         // ~2 logic operations per row and word whatever the fields; every 32 rows the
         // carries of weight 32 are added field by field into 16-bit sums (31 x 2,048
         // rows < 2^16).  (p8, p16: carries waiting for the second of a pair)
-        uint32_t ones[4] = {}, twos[4] = {}, fours[4] = {}, eights[4] = {}, s16[4] = {}, p8[4] = {}, p16[4] = {};
+        uint32_t ones[NW] = {}, twos[NW] = {}, fours[NW] = {}, eights[NW] = {}, s16[NW] = {}, p8[NW] = {}, p16[NW] = {};
         for (uint32_t k = turn, n = 0; k < nst; k += split, n++) {
-            uint4 r[8];
+            uint32_t r[8][NW];
 #pragma unroll
-            for (int j = 0; j < 8; j++) r[j] = __ldg((const uint4 *)(base + (size_t)id[j] * RB));
+            for (int j = 0; j < 8; j++) ct_load(r[j], base + (size_t)id[j] * RB);
             uint2 wt = make_uint2(0x01010101u, 0x01010101u);
             if (WT && a.wts) wt = __ldg((const uint2 *)(a.wts + p0) + k);
             load_ids(k + split);
             if constexpr (!WT) {
-                uint32_t f[2][4];
+                uint32_t f[2][NW];
 #pragma unroll
-                for (int h = 0; h < 2; h++) {
-                    const uint4 r0 = r[4 * h], r1 = r[4 * h + 1], r2 = r[4 * h + 2], r3 = r[4 * h + 3];
-                    const uint32_t x0[4] = {r0.x, r0.y, r0.z, r0.w}, x1[4] = {r1.x, r1.y, r1.z, r1.w},
-                                   x2[4] = {r2.x, r2.y, r2.z, r2.w}, x3[4] = {r3.x, r3.y, r3.z, r3.w};
+                for (int h = 0; h < 2; h++)
 #pragma unroll
-                    for (int w = 0; w < 4; w++) {
+                    for (int w = 0; w < NW; w++) {
                         uint32_t t0, t1;
-                        ct_fa(ones[w], t0, x0[w], x1[w]);
-                        ct_fa(ones[w], t1, x2[w], x3[w]);
+                        ct_fa(ones[w], t0, r[4 * h][w], r[4 * h + 1][w]);
+                        ct_fa(ones[w], t1, r[4 * h + 2][w], r[4 * h + 3][w]);
                         ct_fa(twos[w], f[h][w], t0, t1);
                     }
-                }
 #pragma unroll
-                for (int w = 0; w < 4; w++) {
+                for (int w = 0; w < NW; w++) {
                     uint32_t e;
                     ct_fa(fours[w], e, f[0][w], f[1][w]);
                     if ((n & 1) == 0) {
@@ -862,11 +906,9 @@ __global__ void __launch_bounds__(G_THREADS, WT ? G_BLOCKS_W : G_BLOCKS) gather_
 #pragma unroll
                 for (int h = 0; h < 2; h++) {
                     const uint32_t ww = h ? wt.y : wt.x;
-                    const uint4 r0 = r[4 * h], r1 = r[4 * h + 1], r2 = r[4 * h + 2], r3 = r[4 * h + 3];
-                    const uint32_t w0[4] = {r0.x, r0.y, r0.z, r0.w}, w1[4] = {r1.x, r1.y, r1.z, r1.w},
-                                   w2[4] = {r2.x, r2.y, r2.z, r2.w}, w3[4] = {r3.x, r3.y, r3.z, r3.w};
+                    const uint32_t *w0 = r[4 * h], *w1 = r[4 * h + 1], *w2 = r[4 * h + 2], *w3 = r[4 * h + 3];
 #pragma unroll
-                    for (int q = 0; q < 4; q++) {
+                    for (int q = 0; q < NW; q++) {
                         const uint32_t x0 = __byte_perm(w0[q], w1[q], 0x5140), x1 = __byte_perm(w0[q], w1[q], 0x7362);
                         const uint32_t y0 = __byte_perm(w2[q], w3[q], 0x5140), y1 = __byte_perm(w2[q], w3[q], 0x7362);
                         acc[4 * q] = __dp4a(__byte_perm(x0, y0, 0x5410), ww, acc[4 * q]);
@@ -879,7 +921,7 @@ __global__ void __launch_bounds__(G_THREADS, WT ? G_BLOCKS_W : G_BLOCKS) gather_
         }
         if constexpr (!WT) {
 #pragma unroll
-            for (int w = 0; w < 4; w++) {
+            for (int w = 0; w < NW; w++) {
                 // the waiting carries, then the planes below 32
                 uint32_t x = eights[w] & p8[w], y;
                 eights[w] ^= p8[w];
@@ -896,7 +938,7 @@ __global__ void __launch_bounds__(G_THREADS, WT ? G_BLOCKS_W : G_BLOCKS) gather_
         }
         if (SPLIT) {  // the groups' sums, in the first
 #pragma unroll
-            for (int k = 0; k < 16; k++)
+            for (int k = 0; k < 4 * NW; k++)
                 for (int o = LPG; o < lanes; o <<= 1) acc[k] += __shfl_xor_sync(GKM_FULL, acc[k], o);
             live = live && turn == 0;
         }
@@ -908,10 +950,13 @@ __global__ void __launch_bounds__(G_THREADS, WT ? G_BLOCKS_W : G_BLOCKS) gather_
         const uint32_t dirty = live ? (*db >> (dat & 7)) & ((1u << NQ) - 1u) : 0u;
         const double z = RAW || !live ? 0.0 : a.inv_ds[s], coef = RAW || !live ? 0.0 : a.coef[s];
         __syncwarp();
-        if (dirty) *db = 0;
+        if (dirty) {
+            if (QG < 8) atomicAnd(a.dirty + (dat >> 5), ~(((1u << NQ) - 1u) << (dat & 31)));  // two SVs share the byte
+            else *db = 0;
+        }
         uint4 *sums = rows_s + threadIdx.x;
 #pragma unroll
-        for (int k = 0; k < 4; k++) sums[k * G_THREADS] = make_uint4(acc[4 * k], acc[4 * k + 1], acc[4 * k + 2], acc[4 * k + 3]);
+        for (int k = 0; k < NW; k++) sums[k * G_THREADS] = make_uint4(acc[4 * k], acc[4 * k + 1], acc[4 * k + 2], acc[4 * k + 3]);
 #pragma unroll 1
         for (int w = 0; w < NQ / 4; w++) {
             uint32_t n[4][4];
@@ -1150,8 +1195,7 @@ void gkm_ct_free(gkm_index *ix)
     cudaFree(ix->ct_lists);
 }
 
-// The row width of a call: 32 bytes for batches that fit a few groups of them,
-// else 128.
+// How a call is laid out: the row width and the workspace's parts.
 struct CtPlan {
     bool wide;                // four bytes per query (weighted kernels, dense rows), else two
     int rb, qg, blocks, split;
@@ -1188,16 +1232,18 @@ static CtPlan ct_plan(const gkm_index *ix, int64_t B, int64_t W, int64_t windows
     // 32 queries a group: 64- or (weighted) 128-byte rows; the narrowest rows that
     // hold a smaller batch
     p.rb = wt * 32;
-    while (p.rb > 32 && p.rb / wt / 2 >= B) p.rb /= 2;
+    while (p.rb > 4 * wt && p.rb / wt / 2 >= B) p.rb /= 2;
     p.qg = p.rb / wt;
     p.groups = (B + p.qg - 1) / p.qg;
     p.rows = gkm_row_count(ix);
     const int per_sm = p.wide ? G_BLOCKS_W : G_BLOCKS;
     p.blocks = gkm_query_blocks() * per_sm;
-    // few SVs: a power of two of lane groups within a warp for each (2,000 SVs of 200 ..
-    // 500 bp: 94 -> 47 us per group of 32 weighted queries, 36 -> 12 us unweighted)
+    // a power of two of lane groups within a warp for each SV, until every lane has
+    // work (2,000 SVs of 200 .. 500 bp: 94 -> 47 us per group of 32 weighted queries, 36
+    // -> 12 us unweighted; one query against 72,000: 125 -> 112 us)
+    const int lanes = p.rb < 16 ? 1 : p.rb / 16;
     p.split = 1;
-    while (p.rb / 16 * p.split < 32 && ix->S * (p.rb / 16) * p.split * 2 <= (int64_t)p.blocks * G_THREADS) p.split *= 2;
+    while (lanes * p.split < 32 && ix->S * lanes * p.split < (int64_t)p.blocks * G_THREADS) p.split *= 2;
     auto up = [](int64_t n) { return (n + 255) & ~(int64_t)255; };
     p.table = up((p.rows + 2) * p.rb);
     p.self = up(B * 4 * 8);
@@ -1393,7 +1439,10 @@ extern "C" int gkm_count_table_query(const gkm_index_t *ix, const uint32_t *bx, 
         if (raw) GKM_GATHER_AS(RB, WT, true);                                                             \
         else GKM_GATHER_AS(RB, WT, false);                                                                \
     } while (0)
-        if (p.rb == 32 && wt) GKM_GATHER(32, true);
+        if (p.rb == 8) GKM_GATHER(8, false);
+        else if (p.rb == 16 && wt) GKM_GATHER(16, true);
+        else if (p.rb == 16) GKM_GATHER(16, false);
+        else if (p.rb == 32 && wt) GKM_GATHER(32, true);
         else if (p.rb == 32) GKM_GATHER(32, false);
         else if (p.rb == 64 && wt) GKM_GATHER(64, true);
         else if (p.rb == 64) GKM_GATHER(64, false);
