@@ -381,10 +381,33 @@ __global__ void __launch_bounds__(CT_THREADS, CT_BLOCKS) count_tiles(CtArgs a)
             for (int t = 0; t < 4; t++)
                 if (c[t]) atomicAdd(a.self + (a.r0 + q0 + q) * 4 + t, (unsigned long long)n0 * c[t]);
     };
+    // What a clipped entry's fields do not hold, x of query q of the pass in table row
+    // `row`, where over: to the group's list (weighted, level t = 0), else to the row's
+    // SVs at once by the whole warp.  All lanes call it.
+    auto spill = [&](bool over, uint32_t row, int q, const uint32_t (&x)[4]) {
+        const bool listed = WT && over && !(x[1] | x[2] | x[3]);
+        const uint32_t some = __ballot_sync(GKM_FULL, listed);
+        if (some) {
+            uint32_t base = 0;
+            if (lane == 0) base = atomicAdd(a.nexc, (unsigned)__popc(some));
+            const uint32_t pos = __shfl_sync(GKM_FULL, base, 0) + __popc(some & ((1u << lane) - 1u));
+            if (listed && pos < a.cap_exc) {
+                a.exc[pos] = row | (unsigned long long)(q0 + q) << 22 | (unsigned long long)x[0] << 32;
+                over = false;
+            }
+        }
+        for (uint32_t rest = __ballot_sync(GKM_FULL, over); rest; rest &= rest - 1) {
+            const int j = __ffs(rest) - 1;
+            const uint64_t ex[4] = {__shfl_sync(GKM_FULL, x[0], j), __shfl_sync(GKM_FULL, x[1], j),
+                                    __shfl_sync(GKM_FULL, x[2], j), __shfl_sync(GKM_FULL, x[3], j)};
+            ct_excess<WT>(a, sh.lmer(__shfl_sync(GKM_FULL, row, j)), q0 + __shfl_sync(GKM_FULL, q, j), ex, lane, 32);
+            __syncwarp();
+        }
+    };
     // A second look at counter word w, `at` = j * CT_ROWS + position of a tile, one
     // query per lane (unweighted: two neighbouring lanes share the word): the
-    // query's self-kernel part and, weighted, a clipped count's entry and excess,
-    // which goes to the group's list (full: to the SVs at once).  All lanes call it.
+    // query's self-kernel part and, weighted, a clipped count's entry and excess.  All
+    // lanes call it.
     auto look = [&](uint32_t tl, bool in, uint32_t at, uint32_t w) {
         const uint32_t j = at / CT_ROWS, q = WT ? j : 2 * j + (lane & 1);
         const uint32_t v = !in ? 0u : WT ? w : (w >> (16 * (lane & 1))) & 0xFFFFu;
@@ -393,20 +416,10 @@ __global__ void __launch_bounds__(CT_THREADS, CT_BLOCKS) count_tiles(CtArgs a)
         if (v & slow_mask) self_part(c, q);
         if constexpr (WT) {
             const bool over = (v & 0x100u) != 0;
-            const uint32_t overs = __ballot_sync(GKM_FULL, over);
-            if (!overs) return;
-            uint32_t base = 0, x[4];
-            if (lane == 0) base = atomicAdd(a.nexc, (unsigned)__popc(overs));
-            const uint32_t pos = __shfl_sync(GKM_FULL, base, 0) + __popc(overs & ((1u << lane) - 1u));
-            if (!over) return;
+            uint32_t x[4] = {0, 0, 0, 0};
             const uint32_t row = tl * CT_ROWS + ct_phys((at & (CT_ROWS - 1)) ^ ct_swap(j));
-            ((uint32_t *)(a.T + (size_t)row * a.rb))[q0 + q] = clip(c, x);
-            if (pos < a.cap_exc) {
-                a.exc[pos] = row | (unsigned long long)(q0 + q) << 22 | (unsigned long long)x[0] << 32;
-            } else {
-                const uint64_t ex[4] = {x[0], 0, 0, 0};
-                ct_excess<WT>(a, sh.lmer(row), q0 + (int)q, ex, 0, 1);
-            }
+            if (over) ((uint32_t *)(a.T + (size_t)row * a.rb))[q0 + q] = clip(c, x);
+            spill(over, row, (int)q, x);
         }
     };
     // the words a tile queued, spread over the warps
@@ -711,8 +724,7 @@ __global__ void __launch_bounds__(CT_THREADS, CT_BLOCKS) count_tiles(CtArgs a)
                         ((uint32_t *)T)[qa + q] = v;
                     else
                         ((uint16_t *)T)[qa + q] = (uint16_t)v;
-                    const uint64_t ex[4] = {x[0], x[1], x[2], x[3]};
-                    if (x[0] | x[1] | x[2] | x[3]) ct_excess<WT>(a, sh.lmer(tile * CT_ROWS + suf), q0 + qa + q, ex, 0, 1);
+                    spill((x[0] | x[1] | x[2] | x[3]) != 0, tile * CT_ROWS + suf, qa + q, x);
                 }
             }
         }
