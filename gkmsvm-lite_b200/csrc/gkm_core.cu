@@ -26,28 +26,47 @@ static int staged_windows(int64_t W) { return (int)(W < 1 ? 1 : W < SMEM_WINDOWS
 // Packing (kernels/packed.py:130-187)
 // ---------------------------------------------------------------------------
 
-__global__ void pack_kernel(const uint8_t *__restrict__ codes, const int64_t *__restrict__ lengths,
-                            int64_t B, int64_t L, int l, uint32_t *__restrict__ fwd,
-                            uint32_t *__restrict__ rc, int32_t *__restrict__ counts)
+constexpr int PACK_THREADS = 256, PACK_WINDOWS = 4 * PACK_THREADS;
+
+// PACK_WINDOWS windows of a row per block: its bases go to shared memory as two bits
+// each, a window is then two words funnel-shifted.  Bound by the stores.  Measured
+// 8,192 rows of 2,000 bases (50 .. 2,000 used): a window per thread, l byte loads each,
+// 86 us; this 40 us.
+__global__ void __launch_bounds__(PACK_THREADS) pack_kernel(
+    const uint8_t *__restrict__ codes, const int64_t *__restrict__ lengths, int64_t L, int l, int64_t chunks,
+    uint32_t *__restrict__ fwd, uint32_t *__restrict__ rc, int32_t *__restrict__ counts)
 {
-    int64_t W = L - l + 1;
-    int64_t idx = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (idx >= B * W) return;
-    int64_t b = idx / W, i = idx - b * W;
+    __shared__ uint32_t bases[PACK_WINDOWS / 16 + 2];  // 16 a word, and those past the last window
+    const int64_t W = L - l + 1, b = blockIdx.x / chunks, c0 = (blockIdx.x - b * chunks) * PACK_WINDOWS;
     int64_t n = W;
     if (lengths) {
         n = lengths[b] - l + 1;
         n = n < 0 ? 0 : (n > W ? W : n);
     }
-    if (i == 0 && counts) counts[b] = (int32_t)n;
-    uint32_t w = GKM_PAD;
-    if (i < n) {
-        const uint8_t *c = codes + b * L + i;
-        w = 0;
-        for (int k = 0; k < l; k++) w |= ((uint32_t)(c[k] & 3u)) << (2 * k);
+    if (c0 == 0 && threadIdx.x == 0 && counts) counts[b] = (int32_t)n;
+    if (c0 < n) {
+        const uint8_t *c = codes + b * L;
+        const int64_t end = n + l - 1;
+        for (int k = threadIdx.x; k < PACK_WINDOWS / 4 + 8; k += PACK_THREADS) {
+            const int64_t p = c0 + 4 * k;
+            uint32_t v = 0;
+#pragma unroll
+            for (int j = 0; j < 4; j++)
+                if (p + j < end) v |= (c[p + j] & 3u) << (2 * j);
+            ((uint8_t *)bases)[k] = (uint8_t)v;
+        }
+        __syncthreads();
     }
-    fwd[idx] = w;
-    if (rc) rc[b * W + (W - 1 - i)] = w == GKM_PAD ? GKM_PAD : gkm_rc_word(w, l);
+    const uint32_t mask = (1u << (2 * l)) - 1u;
+#pragma unroll
+    for (int k = 0; k < PACK_WINDOWS / PACK_THREADS; k++) {
+        const int at = k * PACK_THREADS + threadIdx.x;
+        const int64_t i = c0 + at;
+        if (i >= W) break;
+        const uint32_t w = i < n ? __funnelshift_r(bases[at >> 4], bases[(at >> 4) + 1], 2 * (at & 15)) & mask : GKM_PAD;
+        fwd[b * W + i] = w;
+        if (rc) rc[b * W + (W - 1 - i)] = w == GKM_PAD ? GKM_PAD : gkm_rc_word(w, l);
+    }
 }
 
 // ---------------------------------------------------------------------------
@@ -905,7 +924,10 @@ extern "C" int gkm_pack(const gkm_spec *spec, const uint8_t *codes, const int64_
     int64_t n = B * W;
     if (n == 0) return GKM_OK;
     GKM_PREFER_SHARED(pack_kernel);
-    pack_kernel<<<(unsigned)((n + 255) / 256), 256, 0, (cudaStream_t)stream>>>(codes, lengths, B, L, spec->l, fwd, rc, counts);
+    const int64_t chunks = (W + PACK_WINDOWS - 1) / PACK_WINDOWS;
+    if (B * chunks > 0x7FFFFFFFLL) return gkm_fail(GKM_ERR_UNSUPPORTED, "too many rows in one packing launch");
+    pack_kernel<<<(unsigned)(B * chunks), PACK_THREADS, 0, (cudaStream_t)stream>>>(codes, lengths, L, spec->l, chunks, fwd,
+                                                                                rc, counts);
     GKM_CHECK_LAUNCH("pack");
     return GKM_OK;
 }
