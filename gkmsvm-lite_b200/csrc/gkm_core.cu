@@ -8,6 +8,8 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include <cooperative_groups.h>
+
 #include <type_traits>
 
 #include "gkm_common.cuh"
@@ -849,16 +851,23 @@ __global__ void raw_score_kernel(const double *__restrict__ raw, int64_t S, cons
     if (threadIdx.x == 0) out[b] = acc + bias;
 }
 
-__global__ void impact_kernel(const double *__restrict__ raw, int64_t n, int64_t S,
-                              const double *__restrict__ dr, const double *__restrict__ ds,
-                              const double *__restrict__ coef, double gamma, int rbf,
-                              double *__restrict__ out)
+// A cluster of blocks per row (a row a block left most SMs idle: 96 rows x 72,000 SVs
+// 353 us, this 103 us); their sums meet in the first block's shared memory and are
+// added in rank order.
+constexpr int IMPACT_BLOCKS = 8;
+
+__global__ void __cluster_dims__(IMPACT_BLOCKS, 1, 1) __launch_bounds__(256) impact_kernel(
+    const double *__restrict__ raw, int64_t n, int64_t S, const double *__restrict__ dr, const double *__restrict__ ds,
+    const double *__restrict__ coef, double gamma, int rbf, double *__restrict__ out)
 {
-    __shared__ double red[32];
-    int64_t b = blockIdx.x;
+    __shared__ double red[32], sums[IMPACT_BLOCKS];
+    auto cluster = cooperative_groups::this_cluster();
+    const unsigned rank = cluster.block_rank();
+    cluster.sync();  // every block of the cluster runs before one writes to another
+    const int64_t b = blockIdx.x / IMPACT_BLOCKS;
     double fl = rbf ? exp(-gamma) : 0.0;
     double acc = 0.0;
-    for (int64_t s = threadIdx.x; s < S; s += blockDim.x) {
+    for (int64_t s = rank * blockDim.x + threadIdx.x; s < S; s += IMPACT_BLOCKS * blockDim.x) {
         double k = raw[b * S + s];
         double dk = raw[(n + b) * S + s] - k;
         if (dr) {
@@ -873,7 +882,13 @@ __global__ void impact_kernel(const double *__restrict__ raw, int64_t n, int64_t
         acc += coef[s] * dk;
     }
     acc = gkm_block_sum(acc, red);
-    if (threadIdx.x == 0) out[b] = acc;
+    if (threadIdx.x == 0) cluster.map_shared_rank(sums, 0)[rank] = acc;
+    cluster.sync();
+    if (rank == 0 && threadIdx.x == 0) {
+        double t = 0.0;
+        for (int k = 0; k < IMPACT_BLOCKS; k++) t += sums[k];
+        out[b] = t;
+    }
 }
 
 __global__ void gram_finish_kernel(const double *__restrict__ raw, int64_t N, int64_t M,
@@ -1144,7 +1159,7 @@ extern "C" int gkm_impact(const double *raw, int64_t n, int64_t S, const double 
 {
     if (n == 0) return GKM_OK;
     GKM_PREFER_SHARED(impact_kernel);
-    impact_kernel<<<(unsigned)n, 256, 0, (cudaStream_t)stream>>>(raw, n, S, dr, ds, coef, gamma, rbf, out);
+    impact_kernel<<<(unsigned)(n * IMPACT_BLOCKS), 256, 0, (cudaStream_t)stream>>>(raw, n, S, dr, ds, coef, gamma, rbf, out);
     GKM_CHECK_LAUNCH("impact");
     return GKM_OK;
 }
