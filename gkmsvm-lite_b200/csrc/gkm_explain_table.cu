@@ -13,8 +13,8 @@
 // table is 1.5 GB).
 //
 // Lookups: each window's row A[u] ([4, l], times the window's weight, the
-// perturbation deltas folded in) becomes its [4, l] part, and the parts of the
-// windows covering each position are added in window order (explain_gather in
+// perturbation deltas folded in) is its [4, l] part, and the parts of the windows
+// covering each position are added in window order (explain_gather in
 // gkm_explain.cu does the same for the per-window neighbour sums).
 #include <cuda_runtime.h>
 #include <stdint.h>
@@ -82,52 +82,62 @@ __global__ void explain_fill_products(const double *__restrict__ fv, const doubl
     }
 }
 
-// one window's part [4, l] from its table row: base u_k ^ d at position k gets
-// A[u, d, k] (perturbation: the other three bases also get A[u, 0, k], the
-// window's own base nothing), times the window weight
-__global__ void explain_table_parts(const double *__restrict__ A, const uint32_t *__restrict__ fwd,
-                                    const int32_t *__restrict__ cnt, int64_t B, int64_t W, int l, int weighted,
-                                    const uint8_t *__restrict__ wd, int perturbation, double *__restrict__ part)
-{
-    const int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (t >= B * W * 4 * l) return;
-    const int k = (int)(t % l);
-    const int base = (int)((t / l) % 4);
-    const int64_t bw = t / (4 * l);
-    const int64_t b = bw / W, i = bw - b * W;
-    const int n = cnt[b];
-    double v = 0.0;
-    if (i < n) {
-        const uint32_t u = fwd[b * W + i];
-        const int uk = (int)((u >> (2 * k)) & 3u);
-        const int d = base ^ uk;
-        const double *row = A + (int64_t)u * 4 * l;
-        if (perturbation)
-            v = d == 0 ? 0.0 : row[d * l + k] + row[k];
-        else
-            v = row[d * l + k];
-        if (weighted) v *= (double)gkm_wt(wd, n, (int)i);
-    }
-    part[t] = v;
-}
+constexpr int ET_WINDOWS = 128, ET_THREADS = 256;
 
-// out[b, base, p] = inv_dx[b] * sum over windows i covering p of part[b, i, base, p - i]
-__global__ void explain_table_gather(const double *__restrict__ part, const int32_t *__restrict__ cnt, int64_t B,
-                                     int64_t W, int64_t L, int l, const double *__restrict__ inv_dx,
-                                     double *__restrict__ out)
+__host__ __device__ __forceinline__ int et_stride(int l) { return 4 * l + 1; }  // (odd: a column's rows on all banks)
+
+// The windows over ET_WINDOWS - l + 1 positions of a row per block.  Their parts [4, l]
+// come from the table rows to shared memory -- base u_k ^ d at position k gets A[u, d,
+// k] (perturbation: the other three bases also get A[u, 0, k], the window's own base
+// nothing), times the window weight -- and
+//     out[b, base, p] = inv_dx[b] * sum over windows i covering p of part[i, base, p - i]
+// is added up from there in window order.  Bound by the reads of the table rows (352
+// bytes at l = 11, anywhere in 1.5 GB).  Measured (512 x 1,000 bp): parts to memory 156
+// us and their sums 64 us; this 90 us (138 with loads to registers).
+__global__ void __launch_bounds__(ET_THREADS) explain_table_rows(
+    const double *__restrict__ A, const uint32_t *__restrict__ fwd, const int32_t *__restrict__ cnt, int64_t W, int64_t L,
+    int l, int64_t tiles, int weighted, const uint8_t *__restrict__ wd, const double *__restrict__ inv_dx,
+    int perturbation, double *__restrict__ out)
 {
-    const int64_t idx = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (idx >= B * 4 * L) return;
-    const int64_t b = idx / (4 * L);
-    const int64_t r = idx - b * 4 * L;
-    const int base = (int)(r / L);
-    const int64_t p = r - (int64_t)base * L;
+    extern __shared__ double part[];
+    __shared__ uint32_t us[ET_WINDOWS];
+    const int T = ET_WINDOWS - l + 1, row_n = 4 * l, stride = et_stride(l);
+    const int64_t b = blockIdx.x / tiles, p0 = (blockIdx.x - b * tiles) * T, i0 = p0 - l + 1;
     const int n = cnt[b];
-    const int64_t i0 = p - l + 1 > 0 ? p - l + 1 : 0;
-    const int64_t i1 = p < n - 1 ? p : n - 1;
-    double s = 0.0;
-    for (int64_t i = i0; i <= i1; i++) s += part[((b * W + i) * 4 + base) * l + (p - i)];
-    out[idx] = s * inv_dx[b];
+    if (threadIdx.x < ET_WINDOWS) {
+        const int64_t i = i0 + threadIdx.x;
+        us[threadIdx.x] = i >= 0 && i < n ? fwd[b * W + i] : GKM_PAD;
+    }
+    __syncthreads();
+    // asynchronous copies: all of a block's rows are in flight at once
+    for (int e = threadIdx.x; e < ET_WINDOWS * row_n; e += ET_THREADS) {
+        const int w = e / row_n, r = e - w * row_n, d = r / l, k = r - d * l;
+        const uint32_t u = us[w];
+        if (u == GKM_PAD) continue;  // (not read below)
+        const uint32_t to = (uint32_t)__cvta_generic_to_shared(part + w * stride + (d ^ (int)((u >> (2 * k)) & 3u)) * l + k);
+        asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"(to), "l"(A + (int64_t)u * row_n + r) : "memory");
+    }
+    asm volatile("cp.async.wait_all;" ::: "memory");
+    __syncthreads();
+    const double z = inv_dx[b];
+    for (int o = threadIdx.x; o < 4 * T; o += ET_THREADS) {
+        const int base = o / T;
+        const int64_t p = p0 + o - base * T;
+        if (p >= L) continue;
+        const int64_t first = p - l + 1 > 0 ? p - l + 1 : 0, last = p < n - 1 ? p : n - 1;
+        double s = 0.0;
+        for (int64_t i = first; i <= last; i++) {
+            const int w = (int)(i - i0), k = (int)(p - i);
+            double v = part[w * stride + base * l + k];
+            if (perturbation) {
+                const int own = (int)((us[w] >> (2 * k)) & 3u);
+                v = base == own ? 0.0 : v + part[w * stride + own * l + k];
+            }
+            if (weighted) v *= (double)gkm_wt(wd, n, (int)i);
+            s += v;
+        }
+        out[(b * 4 + base) * L + p] = s * z;
+    }
 }
 
 }  // namespace
@@ -186,20 +196,12 @@ extern "C" int gkm_explain_table(const gkm_spec *spec, const double *A, const ui
     if (B == 0 || W == 0 || L == 0) return GKM_OK;
     cudaStream_t st = (cudaStream_t)stream;
     const int l = spec->l;
-    double *part = nullptr;
-    if (cudaMallocAsync(&part, sizeof(double) * B * W * 4 * l, st) != cudaSuccess)
-        return gkm_fail(GKM_ERR_OOM, "explain table parts");
-    int s = GKM_OK;
-    const int64_t np = B * W * 4 * l;
-    explain_table_parts<<<(unsigned)((np + 255) / 256), 256, 0, st>>>(A, fwd, counts, B, W, l, spec->weighted,
-                                                                       spec->wd, perturbation, part);
-    cudaError_t e = cudaGetLastError();
-    if (e != cudaSuccess) s = gkm_cuda_status(e, "explain_table_parts");
-    if (s == GKM_OK) {
-        const int64_t no = B * 4 * L;
-        explain_table_gather<<<(unsigned)((no + 255) / 256), 256, 0, st>>>(part, counts, B, W, L, l, inv_dx, out);
-        if ((e = cudaGetLastError()) != cudaSuccess) s = gkm_cuda_status(e, "explain_table_gather");
-    }
-    cudaFreeAsync(part, st);
-    return s;
+    const int64_t T = ET_WINDOWS - l + 1, tiles = (L + T - 1) / T;
+    if (B * tiles > 0x7FFFFFFFLL) return gkm_fail(GKM_ERR_UNSUPPORTED, "too many rows in one explain launch");
+    const size_t smem = sizeof(double) * ET_WINDOWS * et_stride(l);
+    cudaFuncSetAttribute(explain_table_rows, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    explain_table_rows<<<(unsigned)(B * tiles), ET_THREADS, smem, st>>>(A, fwd, counts, W, L, l, tiles, spec->weighted,
+                                                                         spec->wd, inv_dx, perturbation, out);
+    GKM_CHECK_LAUNCH("explain_table_rows");
+    return GKM_OK;
 }
