@@ -56,7 +56,7 @@ constexpr uint32_t CT_F0 = 0, CT_F1 = 8, CT_F2 = 12, CT_F3 = 5;
 constexpr int CT_R2 = 4, CT_R3 = 20;  // rounds of 32 lanes over the 106 / 376 neighbour masks of budgets 2 / 3
 constexpr int CT_ROUNDS = 1 + CT_R2 + CT_R3;
 constexpr int CT_BALL = 694;      // masks of up to six positions within three mismatches
-constexpr int CT_LIST1 = 112, CT_LIST2 = 32;  // windows of budgets 1 and 2 a warp lists at a time
+constexpr int CT_WLIST = 128;     // windows of budgets 1 and 2 a warp lists at a time
 constexpr int G_THREADS = 128;
 constexpr int G_BLOCKS = 4, G_BLOCKS_W = 6;   // gather blocks per SM, unweighted / weighted
 
@@ -302,7 +302,7 @@ __global__ void __launch_bounds__(CB_THREADS) ct_buckets(CtArgs a, int64_t B)
 // written 64 bytes at a time, and two blocks share an SM, so that one counts while the
 // other writes.  Tiles of six positions and passes of half as many queries, one block
 // of 1,024 threads per SM, a window per lane for budget 1: 110 us a group of 32 x 300
-// bp, this 88 us (weighted: 268 and 190).
+// bp, this 86 us (weighted: 268 and 184).
 template <bool WT>
 __global__ void __launch_bounds__(CT_THREADS, CT_BLOCKS) count_tiles(CtArgs a)
 {
@@ -310,8 +310,8 @@ __global__ void __launch_bounds__(CT_THREADS, CT_BLOCKS) count_tiles(CtArgs a)
     extern __shared__ __align__(16) uint8_t ct_smem[];
     __shared__ uint2 l3[CT_R3 * 32];
     __shared__ uint16_t ball_s[CT_BALL];
-    constexpr int LIST = CT_LIST1 + 8 + CT_LIST2;  // (eight more of budget 1 are read)
-    __shared__ uint32_t list_s[CT_WARPS * LIST];
+    __shared__ uint32_t list_s[CT_WARPS * (CT_WLIST + 8)];  // (up to eight more are read)
+    __shared__ uint32_t slot_s[CT_WARPS * 32];
     // by tile parity: the entries that need a second look, and the fields' sum and
     // the adds made
     __shared__ uint16_t list_at[2][CT_LIST];
@@ -496,70 +496,69 @@ __global__ void __launch_bounds__(CT_THREADS, CT_BLOCKS) count_tiles(CtArgs a)
                 }
             }
         }
-        // budget 0: a bucket per lane
+        // The windows of the lanes' buckets beg .. beg + len - 1 as one list: f(lane's
+        // record, index of lane 0's, windows in all), 32 at a time.
+        auto flatten = [&](uint32_t beg, uint32_t len, auto f) {
+            uint32_t upto = len;
+#pragma unroll
+            for (int o = 1; o < 32; o <<= 1) {
+                const uint32_t y = __shfl_up_sync(GKM_FULL, upto, o);
+                if (lane >= o) upto += y;
+            }
+            const uint32_t all = __shfl_sync(GKM_FULL, upto, 31), start = upto - len;
+            if (all == 0) return;
+            // the buckets that hold windows, side by side: window h of the list is
+            // record slot + h (in 32 bits: a slot may lie below zero)
+            uint32_t *slot = slot_s + 32 * warp;
+            const uint32_t some = __ballot_sync(GKM_FULL, len != 0);
+            if (len) slot[__popc(some & ((1u << lane) - 1u))] = beg - start;
+            __syncwarp();
+            // a window's bucket is the last one that starts at or before it
+            uint32_t begun = 0;
+            auto fetch = [&](uint32_t c) -> uint32_t {
+                const uint32_t at = start - c, starts = __reduce_or_sync(GKM_FULL, len && at < 32u ? 1u << at : 0u);
+                const uint32_t own = begun + __popc(starts & (0xFFFFFFFFu >> (31 - lane))) - 1u;
+                begun += __popc(starts);
+                return load_rec(c + lane < all ? slot[own & 31u] + (c + lane) : 0u);
+            };
+            uint32_t rec = fetch(0);
+            for (uint32_t c = 0; c < all; c += 32) {
+                const uint32_t now = rec;
+                if (c + 32 < all) rec = fetch(c + 32);  // in flight meanwhile
+                f(now, c, all);
+            }
+            __syncwarp();
+        };
         const int near = nb3 + nb2 + nb1;
         for (int b = CT_WARPS - 1 - warp; b * 32 < nb0; b += CT_WARPS) {
             uint32_t r = 0, e = 0;
             if (b * 32 + lane < nb0) bucket(near + b * 32 + lane, r, e);
-            auto zero = [&](uint32_t rec, uint32_t i, uint32_t n) {
+            if (!WT) adds += e - r;
+            flatten(r, e - r, [&](uint32_t rec, uint32_t c, uint32_t all) {
                 uint32_t sa, inc;
                 where(rec, sa, inc);
-                add(sa, 0u, 1u, inc, i, n);
-                if (WT && i < n) adds += weight(rec);
-            };
-            if (!WT) adds += e - r;
-            const uint32_t some = min(e, r + 128u);
-            for (; r < some; r += 4) {
-                uint32_t x[4];
-#pragma unroll
-                for (int k = 0; k < 4; k++) x[k] = load_rec(r + k);
-#pragma unroll
-                for (int k = 0; k < 4; k++) zero(x[k], r + k, some);
-            }
-            r = some;
-            // the rest of a crowded bucket (low-complexity rows) by all lanes
-            for (uint32_t rest = __ballot_sync(GKM_FULL, r < e); rest; rest &= rest - 1) {
-                const int j = __ffs(rest) - 1;
-                const uint32_t re = __shfl_sync(GKM_FULL, e, j);
-                for (uint32_t k = __shfl_sync(GKM_FULL, r, j) + lane; k < re; k += 32) zero(load_rec(k), k, re);
-            }
+                add(sa, 0u, 1u, inc, c + lane, all);
+                if (WT && c + lane < all) adds += weight(rec);
+            });
         }
-        // budgets 1 and 2: lanes 0 .. n1 - 1 and n1 .. n1 + n2 - 1 have the warp's
-        // buckets of each and list up to cap windows of them at a time
+        // budgets 1 and 2: lanes 0 .. n1 - 1 and n1 .. n1 + n2 - 1 have the warp's buckets
         if (nb1) {
-            const int n1 = (nb1 + CT_WARPS - 1) / CT_WARPS, n2 = (nb2 + CT_WARPS - 1) / CT_WARPS;
+            const int n1 = (nb1 + CT_WARPS - 1) / CT_WARPS;
             const bool is1 = lane < n1;
             const int k = is1 ? nb3 + nb2 + warp + CT_WARPS * lane : nb3 + warp + CT_WARPS * (lane - n1);
             uint32_t r = 0, e = 0;
             if (k < (is1 ? near : nb3 + nb2)) bucket(k, r, e);
             if (!WT) adds += (is1 ? 16u : 106u) * (e - r);
-            const uint32_t cap = is1 ? CT_LIST1 / n1 : n2 ? CT_LIST2 / n2 : 0;
-            uint32_t *list = list_s + warp * LIST;
-            while (__any_sync(GKM_FULL, r < e)) {
-                const uint32_t m = min(cap, e - r), v = is1 ? m : m << 16;
-                uint32_t x = v;
-#pragma unroll
-                for (int o = 1; o < 16; o <<= 1) {
-                    const uint32_t y = __shfl_up_sync(GKM_FULL, x, o);
-                    if (lane >= o) x += y;
-                }
-                const uint32_t all = __shfl_sync(GKM_FULL, x, 15), n_1 = all & 0xFFFFu, n_2 = all >> 16;
-                uint32_t *to = list + (is1 ? (x - v) & 0xFFFFu : CT_LIST1 + 8 + ((x - v) >> 16));
-                uint32_t w = 0;
-                for (uint32_t c = 0; c < m; c += 4) {
-                    uint32_t y[4];
-#pragma unroll
-                    for (int i = 0; i < 4; i++) y[i] = load_rec(r + c + i);
-#pragma unroll
-                    for (int i = 0; i < 4; i++)
-                        if (c + i < m) {
-                            to[c + i] = y[i];
-                            if (WT) w += weight(y[i]);
-                        }
-                }
-                if (WT) adds += (is1 ? 16u : 106u) * w;
-                r += m;
+            const uint32_t ones = __reduce_add_sync(GKM_FULL, is1 ? e - r : 0u);  // windows of budget 1
+            uint32_t *list = list_s + warp * (CT_WLIST + 8);
+            flatten(r, e - r, [&](uint32_t rec, uint32_t c, uint32_t all) {
+                const uint32_t at = c % CT_WLIST;
+                list[at + lane] = rec;
+                if (WT && c + lane < all) adds += (c + lane < ones ? 16u : 106u) * weight(rec);
+                if (at + 32 < CT_WLIST && c + 32 < all) return;
+                // a full list, or the last
                 __syncwarp();
+                const uint32_t from = c - at, n = min((uint32_t)CT_WLIST, all - from), n_1 = min(n, ones > from ? ones - from : 0u);
                 for (uint32_t j = lane >> 4; j < n_1 + (lane >> 4); j += 8) {  // half a warp per window
 #pragma unroll
                     for (int i = 0; i < 4; i++) {
@@ -569,14 +568,14 @@ __global__ void __launch_bounds__(CT_THREADS, CT_BLOCKS) count_tiles(CtArgs a)
                     }
                 }
 #pragma unroll 2
-                for (uint32_t j = 0; j < n_2; j++) {
+                for (uint32_t j = n_1; j < n; j++) {
                     uint32_t sa, inc;
-                    where(list[CT_LIST1 + 8 + j], sa, inc);
+                    where(list[j], sa, inc);
 #pragma unroll
-                    for (int i = 0; i < CT_R2; i++) add(sa, e2[i].x, e2[i].y, inc, j, n_2);
+                    for (int i = 0; i < CT_R2; i++) add(sa, e2[i].x, e2[i].y, inc, j, n);
                 }
                 __syncwarp();
-            }
+            });
         }
         return adds;
     };
@@ -1273,7 +1272,7 @@ static CtPlan ct_plan(const gkm_index *ix, int64_t B, int64_t W, int64_t windows
     p.chunk = (64LL << 20) / (rec * p.rec_cap * p.passes);
     if (p.chunk < 1) p.chunk = 1;
     if (p.chunk > p.groups) p.chunk = p.groups;
-    p.recs = up(rec * (p.rec_cap * p.passes * p.chunk + 8));  // (count_tiles reads up to eight past a bucket)
+    p.recs = up(rec * p.rec_cap * p.passes * p.chunk);
     p.roff = up(4 * (int64_t)(p.n_pre + 1) * p.passes * p.chunk);
     p.bytes = p.table + p.self + p.nexc + p.dirty + p.c + p.partial + p.recs + p.roff + p.exc;
     return p;
