@@ -30,11 +30,39 @@ static int staged_windows(int64_t W) { return (int)(W < 1 ? 1 : W < SMEM_WINDOWS
 
 constexpr int PACK_THREADS = 256, PACK_WINDOWS = 4 * PACK_THREADS;
 
+// Rows of at least this many windows take blocks of their own (pack_rows), shorter ones
+// a thread per window: calls over 4M bases in rows of 20 / 100 / 200 / 300 / 1,000 take
+// 38 / 49 / 51 / 50 / 51 us so, and 290 / 80 / 55 / 46 / 35 with a block a row.
+constexpr int PACK_ROW = 256;
+
+__global__ void pack_kernel(const uint8_t *__restrict__ codes, const int64_t *__restrict__ lengths,
+                            int64_t B, int64_t L, int l, uint32_t *__restrict__ fwd,
+                            uint32_t *__restrict__ rc, int32_t *__restrict__ counts)
+{
+    int64_t W = L - l + 1;
+    int64_t idx = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    if (idx >= B * W) return;
+    int64_t b = idx / W, i = idx - b * W;
+    int64_t n = W;
+    if (lengths) {
+        n = lengths[b] - l + 1;
+        n = n < 0 ? 0 : (n > W ? W : n);
+    }
+    if (i == 0 && counts) counts[b] = (int32_t)n;
+    uint32_t w = GKM_PAD;
+    if (i < n) {
+        const uint8_t *c = codes + b * L + i;
+        w = 0;
+        for (int k = 0; k < l; k++) w |= ((uint32_t)(c[k] & 3u)) << (2 * k);
+    }
+    fwd[idx] = w;
+    if (rc) rc[b * W + (W - 1 - i)] = w == GKM_PAD ? GKM_PAD : gkm_rc_word(w, l);
+}
+
 // PACK_WINDOWS windows of a row per block: its bases go to shared memory as two bits
 // each, a window is then two words funnel-shifted.  Bound by the stores.  Measured
-// 8,192 rows of 2,000 bases (50 .. 2,000 used): a window per thread, l byte loads each,
-// 86 us; this 40 us.
-__global__ void __launch_bounds__(PACK_THREADS) pack_kernel(
+// 8,192 rows of 2,000 bases (50 .. 2,000 used): pack_kernel 86 us, this 40 us.
+__global__ void __launch_bounds__(PACK_THREADS) pack_rows(
     const uint8_t *__restrict__ codes, const int64_t *__restrict__ lengths, int64_t L, int l, int64_t chunks,
     uint32_t *__restrict__ fwd, uint32_t *__restrict__ rc, int32_t *__restrict__ counts)
 {
@@ -938,11 +966,15 @@ extern "C" int gkm_pack(const gkm_spec *spec, const uint8_t *codes, const int64_
     int64_t W = L - spec->l + 1;
     int64_t n = B * W;
     if (n == 0) return GKM_OK;
-    GKM_PREFER_SHARED(pack_kernel);
+    cudaStream_t st = (cudaStream_t)stream;
     const int64_t chunks = (W + PACK_WINDOWS - 1) / PACK_WINDOWS;
-    if (B * chunks > 0x7FFFFFFFLL) return gkm_fail(GKM_ERR_UNSUPPORTED, "too many rows in one packing launch");
-    pack_kernel<<<(unsigned)(B * chunks), PACK_THREADS, 0, (cudaStream_t)stream>>>(codes, lengths, L, spec->l, chunks, fwd,
-                                                                                rc, counts);
+    if (W >= PACK_ROW && B * chunks <= 0x7FFFFFFFLL) {
+        GKM_PREFER_SHARED(pack_rows);
+        pack_rows<<<(unsigned)(B * chunks), PACK_THREADS, 0, st>>>(codes, lengths, L, spec->l, chunks, fwd, rc, counts);
+    } else {
+        GKM_PREFER_SHARED(pack_kernel);
+        pack_kernel<<<(unsigned)((n + 255) / 256), 256, 0, st>>>(codes, lengths, B, L, spec->l, fwd, rc, counts);
+    }
     GKM_CHECK_LAUNCH("pack");
     return GKM_OK;
 }

@@ -1,4 +1,5 @@
-"""Packed windows at the edges of a packing block (1,024 windows): rows of no, one,
+"""Packed windows at the edges of a packing block (1,024 windows) and of rows with blocks
+of their own (256 windows): rows of no, one,
 1,023 .. 1,025 and 2,049 windows, rows shorter than the batch, without lengths, l =
 2, 8, 11, 15, rows at odd byte offsets.  Exact."""
 
@@ -13,7 +14,7 @@ pytestmark = pytest.mark.gpu
 
 
 @pytest.mark.parametrize("l", [2, 8, 11, 15])
-@pytest.mark.parametrize("W", [1, 1023, 1024, 1025, 2049])
+@pytest.mark.parametrize("W", [1, 3, 255, 256, 1023, 1024, 1025, 2049])
 @pytest.mark.parametrize("ragged", [False, True])
 def test_windows(l, W, ragged):
     L = W + l - 1
