@@ -17,8 +17,8 @@
 // and a table row read serves every query of the group: at 72,000 SVs and 300 bp
 // rows an index walk visits 16.7M entries per query by shared-memory atomics,
 // the gather reads 24.5M / 32 rows of 64 bytes.  Measured against the walk (with
-// its query self-kernels): 1,000 x 300 bp, t=3: 43.5 -> 8.6 ms; 2,048 rows of 50 ..
-// 2,000 bp: 135 -> 20.4 ms; 512 of them, weighted t=5: 77.8 -> 8.4 ms; one 300 bp
+// its query self-kernels): 1,000 x 300 bp, t=3: 43.5 -> 8.5 ms; 2,048 rows of 50 ..
+// 2,000 bp: 135 -> 20.2 ms; 512 of them, weighted t=5: 77.8 -> 8.2 ms; one 300 bp
 // row: 1.3 -> 0.2 ms.
 //
 // Entries are exact.  Unweighted entries take 16 bits (5, 4, 4 and 3 for levels
