@@ -929,7 +929,7 @@ def run_b200(args):
             roofline = {"bound": "l2", "achieved": achieved, "peak": peak, "unit": "GB/s", "frac": achieved / peak,
                         "kernel": "count_tiles + gather_kernel", "alg_bytes_per_step": alg_bytes,
                         "replaces": {"hits": hits, "lookups": lookups},
-                        "binding_unit": "L2 to SM reads of the table rows (the gather: 9.1 TB/s while it runs), "
+                        "binding_unit": "table row reads in flight (the gather: 9.1 TB/s while it runs, HBM 45 %), "
                                         "issue and latency between barriers (the counting)",
                         "peak_source": ("MEASURED_PEAKS.json hbm_gbs" if peaks else "fallback 6.65 TB/s")
                                        + " (the HBM copy, for scale: the rows come from L2)"}
