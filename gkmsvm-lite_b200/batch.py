@@ -15,6 +15,7 @@ self-kernel plus W lookups per row), also captured.
 
 from __future__ import annotations
 
+import contextlib
 import gc
 import weakref
 
@@ -64,7 +65,10 @@ class _Graph:
         self.lengths = torch.zeros(rows, dtype=torch.int64, device=dev)
         self.out = torch.empty(rows, dtype=torch.float64, device=dev)
         self.graph = None
-        self.work = None  # count-table workspace, None where the index walk serves the shape
+        self.before = None  # the index's event counts before the last pass
+        # whether count tables serve the shape, and their workspace (None: the index walk)
+        self.tables = scorer.index is not None and scorer.index.table_bytes(rows, L - m.kernel.l + 1) > 0
+        self.work = None
         self._scorer = weakref.ref(scorer)  # no cycle: graphs go with their scorer
 
     @property
@@ -155,7 +159,10 @@ class _Graph:
 
 class BatchedScorer:
     """Scores [B, L] code batches against model's SVs in graph-captured
-    launches; results equal model(x) (same kernels, same order of sums)."""
+    launches; results equal model(x)'s to the rounding of the sum over SVs (a
+    batch's bucket, not its rows, picks the form of the query).  Batches may
+    come from any stream and thread as long as no two at once share a bucket:
+    count-table passes share one workspace and run one after the other."""
 
     def __init__(self, model, use_graphs: bool = True):
         self.model = model
@@ -172,7 +179,7 @@ class BatchedScorer:
             self.inv_ds = model._inv_ds()
             self.coef = model._sv_coef()
         self.use_graphs = use_graphs
-        self.work = engine.Workspace()  # count tables, shared by the buckets (their passes are serial)
+        self.work = engine.Workspace()  # count tables, shared by the buckets
         self._graphs: dict = {}
 
     def _graph(self, B: int, L: int) -> _Graph:
@@ -185,13 +192,22 @@ class BatchedScorer:
     def score(self, codes: torch.Tensor, lengths: torch.Tensor | None = None, events=None,
               check: bool = True) -> torch.Tensor:
         """[B] float64 scores (bias included) of device codes [B, L] with
-        device lengths [B] (None: every row L long).  events: optional CUDA
-        events recorded around the query phase.  check=False skips the index
-        flag read (no synchronisation); call check_flags() later."""
+        device lengths [B] (None: every row L long), in a buffer that the
+        bucket's next batch overwrites.  events: optional CUDA events recorded
+        around the query phase.  check=False skips the index flag read (no
+        synchronisation); call check_flags() later."""
         B, L = codes.shape
         g = self._graph(B, L)
         self._last = g
-        self._before = self.index.counters() if self.index is not None else None
+        with self.work.turn() if g.tables else contextlib.nullcontext():
+            self._pass(g, codes, lengths, events)
+        if check:
+            self.check_flags(g)
+        return g.out[:B]
+
+    def _pass(self, g, codes, lengths, events):
+        B, L = codes.shape
+        g.before = self.index.counters() if self.index is not None else None
         g.codes[:B, :L].copy_(codes)
         if L < g.L:
             g.codes[:B, L:].zero_()
@@ -209,9 +225,6 @@ class BatchedScorer:
             g._query()
             if events:
                 events[1].record()
-        if check and g.work is None:  # count tables are exact: nothing to wait for
-            self.check_flags(g)
-        return g.out[:B]
 
     def check_flags(self, g=None):
         """Waits for the last batch; reruns it eagerly with 32-bit counters if
@@ -224,7 +237,7 @@ class BatchedScorer:
         if g.work is not None:  # count tables are exact
             torch.cuda.current_stream().synchronize()
             return False
-        return self.index.settle(self._before, g._body)
+        return self.index.settle(g.before, g._body)
 
 
 class DirectScorer:
@@ -283,9 +296,12 @@ class DirectScorer:
     def check_flags(self, g=None):
         """Waits for the last batch; reruns it with 32-bit counters if a query
         block's 16-bit carries outgrew its log.  Returns True when it reran."""
-        if self.index is not None and self._rerun is not None:
-            return self.index.settle(self._before, self._rerun)
-        return False
+        if self.index is None:
+            return False
+        if self._rerun is None:  # count tables are exact
+            torch.cuda.current_stream().synchronize()
+            return False
+        return self.index.settle(self._before, self._rerun)
 
 
 class _PerRowGraph:
@@ -331,7 +347,9 @@ class _PerRowRunner:
     whole pass (packing, self-kernels, the persistent index queries over the
     device work queue, the reductions).  A bucket runs eagerly on its first
     use and is captured on its second, so one-off shapes pay no capture.
-    Results equal the eager pass's."""
+    Results equal the eager pass's.  Calls may come from any stream and thread
+    as long as no two at once share a bucket: passes that share the runner's
+    workspaces run one after the other."""
 
     row_granule = 8
     capture_after = 1  # eager runs of a bucket before it is captured
@@ -340,10 +358,17 @@ class _PerRowRunner:
         self.model = model
         self._graphs: dict = {}
         self._uses: dict = {}
-        self.table_work = engine.Workspace()  # count tables, shared by the buckets (their passes are serial)
+        self.table_work = engine.Workspace()  # count tables, shared by the buckets
 
     def body(self, codes, lengths):  # [rows, 4, L] on the device, no host synchronisation
         raise NotImplementedError
+
+    def shares(self) -> bool:
+        """Whether passes use the runner's workspaces."""
+        return True
+
+    def _turn(self):
+        return self.table_work.turn() if self.shares() else contextlib.nullcontext()
 
     def __call__(self, codes: torch.Tensor, lengths: torch.Tensor | None = None) -> torch.Tensor:
         """[B, 4, L] of device codes [B, L] (lengths: device [B], None: all L);
@@ -356,22 +381,28 @@ class _PerRowRunner:
             g = self._graphs[key] = _PerRowGraph(self, *key)
         index = self.model._sv_index() if self.model.use_lmer_index else None
         before = index.counters() if index is not None else None
-        g.codes[:B, :L].copy_(codes)
-        g.codes[:B, L:].zero_()
-        if lengths is None:
-            g.lengths[:B].fill_(L)
-        else:
-            g.lengths[:B].copy_(lengths)
-        g.lengths[B:].zero_()
-        uses = self._uses.get(key, 0)
-        self._uses[key] = uses + 1
-        if uses < self.capture_after:
-            g._body()
-        else:
-            g.run()
+        with self._turn():
+            g.codes[:B, :L].copy_(codes)
+            g.codes[:B, L:].zero_()
+            if lengths is None:
+                g.lengths[:B].fill_(L)
+            else:
+                g.lengths[:B].copy_(lengths)
+            g.lengths[B:].zero_()
+            uses = self._uses.get(key, 0)
+            self._uses[key] = uses + 1
+            if uses < self.capture_after:
+                g._body()
+            else:
+                g.run()
+
+        def rerun():
+            with self._turn():
+                g._body()
+
         if index is not None:
             # 16-bit counter carries that outgrew a block's log: rerun exactly
-            index.settle(before, g._body)
+            index.settle(before, rerun)
         out = g.out[:B, :, :L]
         past = torch.arange(L, device=out.device)[None, None, :] >= g.lengths[:B, None, None]
         return out.masked_fill(past, 0.0)
@@ -389,6 +420,9 @@ class BatchedIsm(_PerRowRunner):
         self.pass_positions = pass_positions
         self._work = None
         self._works = []  # every workspace a captured graph refers to
+
+    def shares(self) -> bool:
+        return self.model._lmer_table_for() is None
 
     def body(self, codes, lengths):
         from .ism import _ism_rows, ism_pass_bytes, ism_workspace_bytes
@@ -419,6 +453,9 @@ class BatchedExplain(_PerRowRunner):
 
         self.mode = _MODE_ALIASES[mode]
         self._table = {}
+
+    def shares(self) -> bool:
+        return isinstance(self.model.kernel, RbfKernel)
 
     def body(self, codes, lengths):
         from .explain import _explain_rows, _explain_table

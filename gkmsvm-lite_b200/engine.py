@@ -7,7 +7,9 @@ reads the entry count back) and explicit capacity checks.
 
 from __future__ import annotations
 
+import contextlib
 import ctypes
+import threading
 
 import numpy as np
 import torch
@@ -207,12 +209,34 @@ def masks_tensor(base, device) -> torch.Tensor:
 
 
 class Workspace:
-    """A device buffer that grows on request; every buffer handed out is kept
-    for the object's life, because captured graphs refer to it.  For one
-    stream at a time."""
+    """A device buffer that grows on request, shared by the passes of one
+    object; every buffer handed out is kept for the object's life, because
+    captured graphs refer to it.  Passes that use it are queued within
+    turn(), from any stream and thread."""
 
     def __init__(self):
         self._buffers = []
+        self._lock = threading.RLock()
+        self._done = None  # the last turn's end
+
+    @contextlib.contextmanager
+    def turn(self):
+        """Queues one pass: other threads wait until its launches are queued, and
+        the current stream (not the host) until the pass before is done with
+        the buffer.  (A caller that captures the pass orders its replays
+        itself: a capture cannot wait on work outside it.)"""
+        with self._lock:
+            st = torch.cuda.current_stream()
+            capturing = torch.cuda.is_current_stream_capturing()
+            if self._done is not None and not capturing:
+                st.wait_event(self._done)
+            try:
+                yield
+            finally:
+                if not capturing:
+                    done = torch.cuda.Event()
+                    done.record(st)
+                    self._done = done
 
     def get(self, n: int, device) -> torch.Tensor:
         if not self._buffers or self._buffers[-1].numel() < n:
