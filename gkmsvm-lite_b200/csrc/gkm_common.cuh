@@ -195,6 +195,21 @@ int gkm_radix_sort(uint32_t *&keys, uint32_t *&vals, uint32_t *&ktmp, uint32_t *
 #define GKM_PREFER_SHARED(fn) cudaFuncSetAttribute(fn, cudaFuncAttributePreferredSharedMemoryCarveout, \
                                                    (int)cudaSharedmemCarveoutMaxShared)
 
+// Lets launches of fn ask for up to `bytes` of dynamic shared memory.  The limit belongs
+// to fn and the device, not to a launch: every caller of one fn gives one value, the most
+// that any call asks for, so that threads launching fn at the same time never lower the
+// limit under each other's launches.
+template <class F>
+inline cudaError_t gkm_allow_shared(F *fn, int64_t bytes)
+{
+    return cudaFuncSetAttribute((const void *)fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
+}
+#define GKM_ALLOW_SHARED(fn, bytes)                                        \
+    do {                                                                   \
+        const cudaError_t e_ = gkm_allow_shared(fn, bytes);                \
+        if (e_ != cudaSuccess) return gkm_cuda_status(e_, "shared memory"); \
+    } while (0)
+
 int gkm_smem_limit();
 int gkm_sm_count();
 // Blocks a persistent index query may take on the calling thread's launches:

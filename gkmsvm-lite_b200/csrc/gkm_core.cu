@@ -277,6 +277,8 @@ __device__ __forceinline__ bool stage_planes(const uint32_t *frow, int n, int l,
     return __syncthreads_or(bad);
 }
 
+constexpr int SELF_PLANES = 200 * 1024;  // the most shared memory for a row's planes
+
 // bit plane words of a row of W windows: the bases and three words past them
 __host__ __device__ inline int plane_words(int64_t W, int l) { return (int)((W + l - 1 + 31) / 32) + 3; }
 
@@ -411,6 +413,7 @@ __global__ void __launch_bounds__(SELF_THREADS) self_kernel(
 // ---------------------------------------------------------------------------
 
 constexpr int JOIN_WARPS = 8;
+constexpr int JOIN_WINDOWS = 56000;  // the longest query row (in shared memory)
 
 template <int NW>
 __global__ void __launch_bounds__(JOIN_WARPS * 32) join_kernel(
@@ -681,6 +684,7 @@ __global__ void __launch_bounds__(MUT_THREADS) mutant_kernel(
 // mutant_kernel stays for d >= 4 and for rows whose planes outgrow shared memory.
 constexpr int MT_THREADS = 256;
 constexpr int MT_WINDOWS = 128;
+constexpr int MT_PLANES = 128 * 1024;  // the most shared memory for a row's planes
 
 // words of one plane: pw zeros, the row's pw, and what the last windows' partners
 // read past them (a tile's words and two more)
@@ -986,10 +990,10 @@ static int self_launch(const gkm_spec *spec, const uint32_t *fwd, const uint32_t
     if (B == 0) return GKM_OK;
     int pw = plane_words(W, spec->l);
     size_t smem = (size_t)4 * pw * sizeof(uint32_t);
-    if (smem > 200 * 1024) smem = pw = 0;
+    if (smem > SELF_PLANES) smem = pw = 0;
 #define GKM_SELF_AS(L, NL, WT)                                                                                \
     do {                                                                                                      \
-        cudaFuncSetAttribute(self_kernel<L, NL, WT>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem); \
+        GKM_ALLOW_SHARED((self_kernel<L, NL, WT>), SELF_PLANES);                                              \
         GKM_PREFER_SHARED((self_kernel<L, NL, WT>));                                                          \
         self_kernel<L, NL, WT><<<(unsigned)B, SELF_THREADS, smem, st>>>(                                      \
             *spec, fwd, rc, counts, W, diag, profile, table, bias, normalize, scores, raw, pw);               \
@@ -1037,7 +1041,7 @@ extern "C" int gkm_join_pairwise(const gkm_spec *spec, const uint32_t *bx, const
 {
     GKM_TRY(check_spec(spec));
     if (B == 0 || S == 0) return GKM_OK;
-    if (Wx > 56000) return gkm_fail(GKM_ERR_UNSUPPORTED, "query rows longer than 56,000 windows");
+    if (Wx > JOIN_WINDOWS) return gkm_fail(GKM_ERR_UNSUPPORTED, "query rows longer than 56,000 windows");
     size_t smem = (size_t)Wx * sizeof(uint32_t);
     dim3 grid((unsigned)B, (unsigned)((S + JOIN_WARPS - 1) / JOIN_WARPS));
     if (grid.y > 65535) return gkm_fail(GKM_ERR_UNSUPPORTED, "too many columns for one join launch");
@@ -1045,7 +1049,7 @@ extern "C" int gkm_join_pairwise(const gkm_spec *spec, const uint32_t *bx, const
     int nw = nw_for(spec->dmax);
 #define GKM_JOIN(NW)                                                                                   \
     do {                                                                                               \
-        cudaFuncSetAttribute(join_kernel<NW>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);  \
+        GKM_ALLOW_SHARED(join_kernel<NW>, JOIN_WINDOWS * sizeof(uint32_t));                            \
         join_kernel<NW><<<grid, JOIN_WARPS * 32, smem, st>>>(*spec, bx, cx, Wx, by, ry, cy, S, Wy, raw, \
                                                              profile);                                 \
     } while (0)
@@ -1115,12 +1119,12 @@ static int mutant_launch(const gkm_spec *spec, const uint32_t *fwd, const int32_
     // four levels, and rows whose bit planes fit shared memory: by diagonals
     const int pw = plane_words(W, spec->l) + 1;
     const size_t planes = (size_t)4 * mutant_plane(pw) * sizeof(uint32_t);
-    if (spec->dmax < 4 && planes <= 128 * 1024) {
+    if (spec->dmax < 4 && planes <= MT_PLANES) {
         const int P = MT_WINDOWS - spec->l + 1;
         const dim3 grid((unsigned)((L + P - 1) / P), (unsigned)B);
 #define GKM_MUT_AS(LT, WT)                                                                                     \
     do {                                                                                                       \
-        cudaFuncSetAttribute(mutant_tiles<LT, WT>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)planes);  \
+        GKM_ALLOW_SHARED((mutant_tiles<LT, WT>), MT_PLANES);                                                   \
         GKM_PREFER_SHARED((mutant_tiles<LT, WT>));                                                             \
         mutant_tiles<LT, WT><<<grid, MT_THREADS, planes, st>>>(*spec, fwd, counts, B, W, L, diag, mut_diag,    \
                                                                table, ref_raw, normalize, out, pw);            \
@@ -1141,7 +1145,7 @@ static int mutant_launch(const gkm_spec *spec, const uint32_t *fwd, const int32_
     int nw = nw_for(spec->dmax);
 #define GKM_MUT(NW)                                                                                      \
     do {                                                                                                 \
-        cudaFuncSetAttribute(mutant_kernel<NW>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);  \
+        GKM_ALLOW_SHARED(mutant_kernel<NW>, 2 * SMEM_WINDOWS * sizeof(uint32_t));                        \
         GKM_PREFER_SHARED(mutant_kernel<NW>);                                                            \
         mutant_kernel<NW><<<grid, MUT_THREADS, smem, st>>>(*spec, fwd, counts, B, W, L, diag, mut_diag,  \
                                                            table, ref_raw, normalize, out, sw);          \

@@ -1402,6 +1402,10 @@ extern "C" int gkm_count_table_query(const gkm_index_t *ix, const uint32_t *bx, 
     for (int m = 0; m < 4; m++) a.nball[m] = m <= a.sh.D ? ct_ball(a.sh.l - CT_POS, m, nullptr) : 0;
     a.n_pre = p.n_pre;
     a.rec_cap = p.rec_cap;
+    auto count = wt ? count_tiles<true> : count_tiles<false>;
+    // two blocks' shared memory, the rest of the SM's for L1
+    GKM_ALLOW_SHARED(count, sizeof(uint32_t) * CT_ROWS * (CT_SLOTS + 1));
+    cudaFuncSetAttribute(count, cudaFuncAttributePreferredSharedMemoryCarveout, 86);
     for (int64_t g = 0; g < p.groups; g++) {
         a.r0 = g * p.qg;
         a.nq = (int)(B - a.r0 < p.qg ? B - a.r0 : p.qg);
@@ -1430,10 +1434,6 @@ extern "C" int gkm_count_table_query(const gkm_index_t *ix, const uint32_t *bx, 
         // run side by side (their parts of a table row meet in L2)
         const int fit = gkm_query_blocks() * CT_BLOCKS / a.passes * a.passes;
         const unsigned grid = (unsigned)(a.items < fit ? a.items : fit > 0 ? fit : a.passes);
-        auto count = wt ? count_tiles<true> : count_tiles<false>;
-        // two blocks' shared memory, the rest of the SM's for L1
-        cudaFuncSetAttribute(count, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-        cudaFuncSetAttribute(count, cudaFuncAttributePreferredSharedMemoryCarveout, 86);
         count<<<grid, CT_THREADS, smem, st>>>(a);
         GKM_CHECK_LAUNCH("count_tiles");
         if (wt) {

@@ -556,8 +556,9 @@ extern "C" int gkm_explain_subsets(const gkm_spec *spec, const uint32_t *fwd, co
     a.part = part;
     const int stride = 1 + 3 * max_size;
     const size_t smem = sizeof(double) * (size_t)n_subsets * stride;
-    if ((int64_t)smem > gkm_smem_limit() - 2048) return gkm_fail(GKM_ERR_UNSUPPORTED, "%d subsets do not fit", n_subsets);
-    cudaFuncSetAttribute(explain_subsets, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    const int64_t most = gkm_smem_limit() - 2048;
+    if ((int64_t)smem > most) return gkm_fail(GKM_ERR_UNSUPPORTED, "%d subsets do not fit", n_subsets);
+    GKM_ALLOW_SHARED(explain_subsets, most);
     GKM_PREFER_SHARED(explain_subsets);
     explain_subsets<<<dim3((unsigned)W, (unsigned)B), XS_THREADS, smem, st>>>(a, stride);
     GKM_CHECK_LAUNCH("explain_subsets");

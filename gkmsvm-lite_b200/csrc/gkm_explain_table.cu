@@ -199,7 +199,7 @@ extern "C" int gkm_explain_table(const gkm_spec *spec, const double *A, const ui
     const int64_t T = ET_WINDOWS - l + 1, tiles = (L + T - 1) / T;
     if (B * tiles > 0x7FFFFFFFLL) return gkm_fail(GKM_ERR_UNSUPPORTED, "too many rows in one explain launch");
     const size_t smem = sizeof(double) * ET_WINDOWS * et_stride(l);
-    cudaFuncSetAttribute(explain_table_rows, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    GKM_ALLOW_SHARED(explain_table_rows, sizeof(double) * ET_WINDOWS * et_stride(ET_LMAX));
     explain_table_rows<<<(unsigned)(B * tiles), ET_THREADS, smem, st>>>(A, fwd, counts, W, L, l, tiles, spec->weighted,
                                                                          spec->wd, inv_dx, perturbation, out);
     GKM_CHECK_LAUNCH("explain_table_rows");

@@ -451,7 +451,7 @@ extern "C" int gkm_ism_pairs(const gkm_index_t *ix, const uint32_t *fwd, const i
     auto gather = p.threads == 256 ? (wt ? pair_gather<256, true> : pair_gather<256, false>)
                   : p.threads == 512 ? (wt ? pair_gather<512, true> : pair_gather<512, false>)
                                      : (wt ? pair_gather<1024, true> : pair_gather<1024, false>);
-    cudaFuncSetAttribute(gather, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)p.smem);
+    GKM_ALLOW_SHARED(gather, pg_bytes(2 * p.threads));
     for (a.b = 0; a.b < B; a.b++) {
         e = cudaMemsetAsync(a.cursor, 0, 4, st);
         if (e != cudaSuccess) return gkm_cuda_status(e, "ISM pair lists");
