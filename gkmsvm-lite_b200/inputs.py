@@ -230,9 +230,11 @@ def per_position(out: torch.Tensor, batch: SeqBatch, short) -> torch.Tensor:
 
 
 def device_codes(x, device) -> torch.Tensor:
-    """Codes as a contiguous uint8 tensor on device (pinned + async for host input)."""
+    """Codes as a contiguous uint8 tensor on device (pinned + async for host
+    input; a caller's own pinned tensor is read before this returns, because
+    the caller may refill it)."""
     if isinstance(x, torch.Tensor):
-        return x.to(device=device, dtype=torch.uint8, non_blocking=True).contiguous()
+        return x.to(device=device, dtype=torch.uint8, non_blocking=not x.is_pinned()).contiguous()
     t = torch.from_numpy(np.ascontiguousarray(x, dtype=np.uint8))
     if device.type == "cuda":
         t = t.pin_memory()
