@@ -1289,6 +1289,15 @@ static CtPlan ct_plan(const gkm_index *ix, int64_t B, int64_t W, int64_t windows
 constexpr double CT_CALL_US = 45.0, CT_ITEM_US = 12.0, CT_WINDOW_US = 8.5e-4, CT_GATHER_BYTES_US = 8.0e6;
 constexpr double WALK_FLOOR_US = 400.0, WALK_LOOKUP_US[2] = {8.0e-6, 5.8e-6}, WALK_HIT_US[2] = {1.1e-6, 2.0e-6};
 
+// Whether every count stays below 2^32: the (row, SV) weight products of rows of W
+// windows, summed over every pair of windows.
+static bool ct_exact(const gkm_index *ix, int64_t W)
+{
+    const bool wt = ix->spec.weighted != 0;
+    const uint64_t wx = wt ? gkm_weight_sum(ix, W) : (uint64_t)W, wy = wt ? gkm_weight_sum(ix, ix->W) : (uint64_t)ix->W;
+    return wx && wy && wx < (1ull << 32) / ((uint64_t)ix->strands * wy);
+}
+
 // Whether a query over B rows of W window slots, `windows` windows in all, may
 // take the count tables: the index has gather lists, no (row, SV, level) count
 // reaches 2^32, the shared counters rarely overflow, and the estimated time is
@@ -1296,10 +1305,8 @@ constexpr double WALK_FLOOR_US = 400.0, WALK_LOOKUP_US[2] = {8.0e-6, 5.8e-6}, WA
 static bool ct_applies(const gkm_index *ix, int64_t B, int64_t W, int64_t windows)
 {
     if (!ix->ct_ids || B < 1 || W < 1 || W > 60000 || B * ix->tiles > 0x7FFFFFFFLL) return false;
+    if (!ct_exact(ix, W)) return false;
     const bool wt = ix->spec.weighted != 0;
-    // (row, SV) weight products summed over every pair of windows
-    const uint64_t wx = wt ? gkm_weight_sum(ix, W) : (uint64_t)W, wy = wt ? gkm_weight_sum(ix, ix->W) : (uint64_t)ix->W;
-    if (!wx || !wy || wx >= (1ull << 32) / ((uint64_t)ix->strands * wy)) return false;
     // bytes hold the AT-rich rows of three times this mean
     if (ct_mean(ix, W) > 80.0) return false;
     const int64_t known = windows;
@@ -1336,8 +1343,9 @@ extern "C" int gkm_count_table_query(const gkm_index_t *ix, const uint32_t *bx, 
     if (order && diag_offset >= 0) return gkm_fail(GKM_ERR_INVALID, "a self-Gram takes rows in order");
     if (B < 0 || W < 1) return gkm_fail(GKM_ERR_INVALID, "rows %lld, windows per row %lld", (long long)B, (long long)W);
     if (B == 0) return GKM_OK;
-    // (counts stay below 2^32 only where gkm_count_table_workspace says so)
     if (!ix->ct_ids || W > 60000) return gkm_fail(GKM_ERR_UNSUPPORTED, "this index or shape has no count tables");
+    if (!ct_exact(ix, W))
+        return gkm_fail(GKM_ERR_UNSUPPORTED, "a pair count of rows of %lld windows could pass 2^32", (long long)W);
     const CtPlan p = ct_plan(ix, B, W, windows);
     if (!workspace || ((uintptr_t)workspace & 255) || workspace_bytes < p.bytes)
         return gkm_fail(GKM_ERR_CAPACITY, "count tables need a 256-byte aligned workspace of %lld bytes", (long long)p.bytes);

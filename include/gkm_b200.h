@@ -190,6 +190,7 @@ int gkm_index_count(const gkm_index_t *index, const uint32_t *bx, const int32_t 
  * then null), or scores [B] as in gkm_index_score, normalised by inv_dx [B] or,
  * when that is null and normalize is set, by 1 / sqrt(max(K(x, x), 1e-20)).
  * workspace: 256-byte aligned, used by this call only until it completes.
+ * GKM_ERR_UNSUPPORTED where a count of the shape could reach 2^32.
  * Replaces LmerIndex.pairwise / reduce (kernels/lmer_index.py:239-298) and
  * raw_diag_packed of the query rows (kernels/direct.py:109-137). */
 int gkm_count_table_workspace(const gkm_index_t *index, int64_t B, int64_t W, int64_t windows, int64_t *bytes);
