@@ -366,8 +366,8 @@ struct PairPlan {
 static bool pair_plan(const gkm_index *ix, int64_t W, int64_t L, PairPlan &p)
 {
     // the count tables' gather lists (and their limits); a thread has two positions and
-    // an SV's G and C fit shared memory
-    if (!ix->ct_ids || W < 1 || L > 2048 || W > L) return false;
+    // an SV's G and C fit shared memory; every window lies within the L positions
+    if (!ix->ct_ids || W < 1 || L > 2048 || W > L - ix->spec.l + 1) return false;
     p.threads = L <= 512 ? 256 : L <= 1024 ? 512 : 1024;
     p.smem = pg_bytes(L);
     if ((int64_t)p.smem > gkm_smem_limit()) return false;

@@ -269,7 +269,8 @@ int gkm_index_mutants(const gkm_index_t *index, const uint32_t *fwd, const int32
 /* The same deltas from one pass over the window pairs of each row and SV within
  * dmax + 1 mismatches, without K of every (mutant, SV).  gkm_ism_pairs_workspace:
  * *bytes of device workspace (256-byte aligned, used until the call completes), 0
- * where gkm_index_mutants serves rows of W windows and L positions.  inv_dx [B]:
+ * where gkm_index_mutants serves rows of W windows and L positions (W <= L - l + 1: a
+ * row's windows lie within its positions).  inv_dx [B]:
  * 1 / sqrt(K(x, x)) (1 unnormalised). */
 int gkm_ism_pairs_workspace(const gkm_index_t *index, int64_t W, int64_t L, int64_t *bytes);
 int gkm_ism_pairs(const gkm_index_t *index, const uint32_t *fwd, const int32_t *counts, int64_t B, int64_t W,
