@@ -824,9 +824,10 @@ int gkm_sm_count()
     return v;
 }
 
-extern "C" int gkm_index_create(const gkm_spec *spec, const uint32_t *fwd, const uint32_t *rc,
-                                const int32_t *counts, int64_t S, int64_t W, const uint32_t *masks,
-                                int32_t n_masks, int32_t tile_svs, gkm_index_t **out, gkm_stream_t stream)
+// tables: with the gather lists of the count tables.
+static int index_create(const gkm_spec *spec, const uint32_t *fwd, const uint32_t *rc, const int32_t *counts, int64_t S,
+                        int64_t W, const uint32_t *masks, int32_t n_masks, int32_t tile_svs, bool tables,
+                        gkm_index_t **out, gkm_stream_t stream)
 {
     if (!spec || !out) return gkm_fail(GKM_ERR_INVALID, "null spec or out");
     *out = nullptr;
@@ -986,7 +987,7 @@ extern "C" int gkm_index_create(const gkm_spec *spec, const uint32_t *fwd, const
         cudaMemsetAsync(ix->status, 0, 2 * sizeof(unsigned int), st);
         ix->bytes = (int64_t)sizeof(uint32_t) * ((ix->bwords ? 2 : 1) * nbuckets + 1) + (int64_t)eb +
                     sizeof(uint32_t) * n_masks;
-        status = gkm_ct_build(ix, fwd, counts, st);
+        if (tables) status = gkm_ct_build(ix, fwd, counts, st);
     } while (0);
     cudaFreeAsync(ecount, st);
     cudaFreeAsync(keys, st);
@@ -1003,6 +1004,20 @@ extern "C" int gkm_index_create(const gkm_spec *spec, const uint32_t *fwd, const
     }
     *out = ix;
     return GKM_OK;
+}
+
+extern "C" int gkm_index_create(const gkm_spec *spec, const uint32_t *fwd, const uint32_t *rc,
+                                const int32_t *counts, int64_t S, int64_t W, const uint32_t *masks,
+                                int32_t n_masks, int32_t tile_svs, gkm_index_t **out, gkm_stream_t stream)
+{
+    return index_create(spec, fwd, rc, counts, S, W, masks, n_masks, tile_svs, true, out, stream);
+}
+
+extern "C" int gkm_index_create_walk(const gkm_spec *spec, const uint32_t *fwd, const uint32_t *rc,
+                                     const int32_t *counts, int64_t S, int64_t W, const uint32_t *masks,
+                                     int32_t n_masks, int32_t tile_svs, gkm_index_t **out, gkm_stream_t stream)
+{
+    return index_create(spec, fwd, rc, counts, S, W, masks, n_masks, tile_svs, false, out, stream);
 }
 
 extern "C" int gkm_index_free(gkm_index_t *ix)

@@ -257,15 +257,18 @@ def table_workspace(index, B: int, W: int, windows: int, device, work: Workspace
 
 
 class DeviceIndex:
-    """An l-mer index handle over packed columns (owned; freed on close)."""
+    """An l-mer index handle over packed columns (owned; freed on close).
+    tables: with the lists that count-table queries and ISM pair lists read
+    (False for an index that only l-mer weights or index walks are read
+    from)."""
 
-    def __init__(self, spec: Spec, fwd, rc, counts, masks: torch.Tensor, tile_svs: int = 0):
+    def __init__(self, spec: Spec, fwd, rc, counts, masks: torch.Tensor, tile_svs: int = 0, tables: bool = True):
         self.spec = spec
         self.S = fwd.shape[0]
         self.masks = masks
         h = ctypes.c_void_p()
-        call("gkm_index_create", spec.ref, ptr(fwd), ptr(rc), ptr(counts), fwd.shape[0], fwd.shape[1],
-             ptr(masks), int(masks.numel()), int(tile_svs), ctypes.byref(h), _st())
+        call("gkm_index_create" if tables else "gkm_index_create_walk", spec.ref, ptr(fwd), ptr(rc), ptr(counts),
+             fwd.shape[0], fwd.shape[1], ptr(masks), int(masks.numel()), int(tile_svs), ctypes.byref(h), _st())
         self.handle = h
         e, t, ts, nb = ctypes.c_int64(), ctypes.c_int32(), ctypes.c_int32(), ctypes.c_int64()
         call("gkm_index_info", h, ctypes.byref(e), ctypes.byref(t), ctypes.byref(ts), ctypes.byref(nb))

@@ -99,7 +99,7 @@ def _explain_V(model) -> torch.Tensor:
         index = c.get("index")
         tmp = None
         if index is None:
-            tmp = engine.DeviceIndex(spec, fwd, rc, counts, model._masks())
+            tmp = engine.DeviceIndex(spec, fwd, rc, counts, model._masks(), tables=False)
             index = tmp
         c["explain_V"] = index.lmer_weights(coef.contiguous())
         if tmp is not None:

@@ -207,7 +207,7 @@ class GkmSVM:
             index = self._sv_cache.get("index")
             tmp = None
             if index is None:
-                tmp = engine.DeviceIndex(spec, fwd, rc, counts, self._masks())
+                tmp = engine.DeviceIndex(spec, fwd, rc, counts, self._masks(), tables=False)
                 index = tmp
             V = index.lmer_weights(coef.contiguous())
             self._lmer_table = engine.lmer_table(spec, V, self._masks())

@@ -52,7 +52,7 @@ class KernelColumnCache:
         self.index = None
         if isinstance(base, DirectGkmKernel) and n_windows > 0 and base.index_applies(n_windows):
             self.index = engine.DeviceIndex(self.spec, self.fwd, self.rc, self.counts,
-                                            engine.masks_tensor(base, dev))
+                                            engine.masks_tensor(base, dev), tables=False)
         self.rbf = isinstance(kernel, RbfKernel)
         self.gamma = kernel.gamma if self.rbf else 0.0
 

@@ -111,12 +111,19 @@ int gkm_dense_set_role_wait(int64_t ns);
 /* Builds the l-mer index over S columns (radix sort of the packed l-mers of
  * their forward and RC windows into per-SV-tile CSR buckets).  masks [n_masks]
  * (device): the XOR neighbour masks within dmax, each with its mismatch count
- * in bits 24..31.  tile_svs 0: chosen for shared memory.
+ * in bits 24..31.  tile_svs 0: chosen for shared memory.  With the lists that
+ * count-table queries and ISM pair lists read, where the index is within their
+ * limits; gkm_index_create_walk builds the index without them (the workspace
+ * calls of both then answer 0), for one that only serves walks or l-mer weights.
  * Replaces LmerIndex.__init__ (kernels/lmer_index.py:161-200). */
 int gkm_index_create(const gkm_spec *spec, const uint32_t *fwd, const uint32_t *rc,
                      const int32_t *counts, int64_t S, int64_t W, const uint32_t *masks,
                      int32_t n_masks, int32_t tile_svs, gkm_index_t **out,
                      gkm_stream_t stream);
+int gkm_index_create_walk(const gkm_spec *spec, const uint32_t *fwd, const uint32_t *rc,
+                          const int32_t *counts, int64_t S, int64_t W, const uint32_t *masks,
+                          int32_t n_masks, int32_t tile_svs, gkm_index_t **out,
+                          gkm_stream_t stream);
 int gkm_index_free(gkm_index_t *index);
 int gkm_index_info(const gkm_index_t *index, int64_t *entries, int32_t *tiles,
                    int32_t *tile_svs, int64_t *device_bytes);

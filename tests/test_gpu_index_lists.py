@@ -1,0 +1,59 @@
+"""Indexes without the count tables' lists: those that only l-mer weights or
+kernel columns are read from, and those whose lists do not fit the device."""
+
+import ctypes
+
+import numpy as np
+import pytest
+import torch
+
+import gkmsvm_lite_b200 as gk
+import gkmsvm_lite_b200.synthetic as syn
+from gkmsvm_lite_b200 import engine
+from gkmsvm_lite_b200._lib import call
+from gkmsvm_lite_b200.solver import KernelColumnCache
+
+pytestmark = pytest.mark.gpu
+
+PARAMS = {"L": 11, "k": 7, "d": 3, "gamma": 1.0}
+
+
+def _pairs_bytes(index, L):
+    n = ctypes.c_int64()
+    call("gkm_ism_pairs_workspace", index.handle, L - 10, L, ctypes.byref(n))
+    return n.value
+
+
+@pytest.mark.parametrize("kt", ["gkmrbf", "wgkmrbf"])
+def test_walk_index(kt):
+    rng = np.random.default_rng(8)
+    m = gk.GkmSVM(syn.random_codes(rng, 200, 150), rng.normal(size=200), 0.1, kt, PARAMS).cuda()
+    full, walk = m._sv_index(), engine.DeviceIndex(m._spec(), *m._sv_packed(), m._masks(), tables=False)
+    assert full.table_bytes(4, 90, 1 << 40) > 0 and _pairs_bytes(full, 100) > 0
+    assert walk.table_bytes(4, 90, 1 << 40) == 0 and _pairs_bytes(walk, 100) == 0
+    assert walk.nbytes < full.nbytes
+    f, _, c = engine.pack(m._spec(), torch.from_numpy(syn.random_codes(rng, 4, 100)).cuda(), None)
+    assert torch.equal(walk.pairwise(f, c)[0], full.pairwise(f, c)[0])
+    walk.close()
+
+
+@pytest.mark.parametrize("use", ["l-mer table", "explain", "training"])
+def test_who_builds_no_lists(use, monkeypatch):
+    made = []
+
+    def spy(name, *args):
+        made.append(name)
+        return call(name, *args)
+
+    monkeypatch.setattr(engine, "call", spy)
+    rng = np.random.default_rng(9)
+    x = syn.random_codes(rng, 100, 150)
+    m = gk.GkmSVM(x, rng.normal(size=100), 0.1, "gkm_esttrunc", PARAMS).cuda()
+    if use == "l-mer table":
+        m.use_lmer_table = True
+        m(x[:3])
+    elif use == "explain":
+        gk.gkmexplain(m, x[:3])
+    else:
+        KernelColumnCache(m.kernel, x).compute_columns([0, 1])
+    assert "gkm_index_create_walk" in made and "gkm_index_create" not in made
