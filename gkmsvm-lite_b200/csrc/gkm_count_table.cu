@@ -1204,6 +1204,9 @@ void gkm_ct_free(gkm_index *ix)
     cudaFree(ix->ct_off);
     cudaFree(ix->ct_perm);
     cudaFree(ix->ct_lists);
+    ix->ct_ids = ix->ct_off = ix->ct_perm = ix->ct_lists = nullptr;
+    ix->ct_wts = nullptr;
+    ix->ct_entries = 0;
 }
 
 // How a call is laid out: the row width and the workspace's parts.

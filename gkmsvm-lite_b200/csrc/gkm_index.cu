@@ -987,7 +987,6 @@ static int index_create(const gkm_spec *spec, const uint32_t *fwd, const uint32_
         cudaMemsetAsync(ix->status, 0, 2 * sizeof(unsigned int), st);
         ix->bytes = (int64_t)sizeof(uint32_t) * ((ix->bwords ? 2 : 1) * nbuckets + 1) + (int64_t)eb +
                     sizeof(uint32_t) * n_masks;
-        if (tables) status = gkm_ct_build(ix, fwd, counts, st);
     } while (0);
     cudaFreeAsync(ecount, st);
     cudaFreeAsync(keys, st);
@@ -997,6 +996,19 @@ static int index_create(const gkm_spec *spec, const uint32_t *fwd, const uint32_
     if (status == GKM_OK) {
         cudaError_t e = cudaStreamSynchronize(st);
         if (e != cudaSuccess) status = gkm_cuda_status(e, "index build");
+    }
+    if (status == GKM_OK && tables) {
+        // after the build's scratch has gone back: the lists then need no more memory at
+        // once than the build did.  Where they do not fit even so, the walk serves the index.
+        status = gkm_ct_build(ix, fwd, counts, st);
+        if (status == GKM_OK) {
+            cudaError_t e = cudaStreamSynchronize(st);
+            if (e != cudaSuccess) status = gkm_cuda_status(e, "gather lists");
+        } else if (status == GKM_ERR_OOM) {
+            (void)cudaGetLastError();  // an allocation's failure leaves nothing behind but its error
+            gkm_ct_free(ix);
+            status = GKM_OK;
+        }
     }
     if (status != GKM_OK) {
         gkm_index_free(ix);

@@ -113,7 +113,7 @@ int gkm_dense_set_role_wait(int64_t ns);
  * (device): the XOR neighbour masks within dmax, each with its mismatch count
  * in bits 24..31.  tile_svs 0: chosen for shared memory.  With the lists that
  * count-table queries and ISM pair lists read, where the index is within their
- * limits; gkm_index_create_walk builds the index without them (the workspace
+ * limits and the device has room for them; gkm_index_create_walk builds the index without them (the workspace
  * calls of both then answer 0), for one that only serves walks or l-mer weights.
  * Replaces LmerIndex.__init__ (kernels/lmer_index.py:161-200). */
 int gkm_index_create(const gkm_spec *spec, const uint32_t *fwd, const uint32_t *rc,

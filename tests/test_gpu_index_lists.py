@@ -57,3 +57,47 @@ def test_who_builds_no_lists(use, monkeypatch):
     else:
         KernelColumnCache(m.kernel, x).compute_columns([0, 1])
     assert "gkm_index_create_walk" in made and "gkm_index_create" not in made
+
+
+def test_lists_that_do_not_fit():
+    """With less and less free memory: wherever the index itself can be built, it
+    is built, with its lists or without."""
+    rng = np.random.default_rng(10)
+    base = gk.CenterWeightedGkmKernel(8, 4, d=3)
+    spec = engine.Spec(base, torch.device("cuda"))
+    # SVs of one window each: the lists pad them to eight and outweigh the index's own scratch
+    x = torch.from_numpy(syn.random_codes(rng, 4_000_000, 8)).cuda()
+    fwd, rc, counts = engine.pack(spec, x, None)
+    masks = engine.masks_tensor(base, torch.device("cuda"))
+    q, _, qc = engine.pack(spec, torch.from_numpy(syn.random_codes(rng, 1, 40)).cuda(), None)
+    del x
+
+    def build(tables):
+        try:
+            return engine.DeviceIndex(spec, fwd, rc, counts, masks, tables=tables)
+        except MemoryError:
+            return None
+
+    want, with_lists, without = None, 0, 0
+    for room in range(640, 140, -20):
+        torch.cuda.synchronize()
+        torch.cuda.empty_cache()
+        taken = torch.empty(torch.cuda.mem_get_info()[0] - (room << 20), dtype=torch.uint8, device="cuda")
+        try:
+            walk = build(False)
+            if walk is None:
+                break
+            walk.close()
+            index = build(True)
+        finally:
+            del taken
+            torch.cuda.empty_cache()
+        assert index is not None, f"{room} MB"
+        lists = index.table_bytes(1, 33, 1 << 40) > 0
+        with_lists += lists
+        without += not lists
+        raw = index.pairwise(q, qc)[0]
+        want = raw if want is None else want
+        assert torch.equal(raw, want)
+        index.close()
+    assert with_lists and without
