@@ -381,16 +381,19 @@ class DeviceIndex:
              int(bool(normalize)), ptr(inv_dx), ptr(diag), -1 if diag_offset is None else int(diag_offset), ptr(raw), ptr(inv_ds),
              ptr(coef), float(gamma), int(rbf), float(bias), ptr(scores), ptr(work), int(work.numel()), _st())
 
-    def rows(self, bx, rx, cx, normalize, *, diag_offset=None, out=None, check=True, windows=0, work=None):
-        """(K_raw [B, S], K(x, x) [B] or None without normalize) of packed
-        rows: through count tables where they are the cheaper form (work: a
+    def rows(self, bx, rx, cx, normalize, *, diag_offset=None, out=None, check=True, windows=0, work=None,
+             diag_rows=None):
+        """(K_raw [B, S], K(x, x) or None without normalize) of packed rows:
+        through count tables where they are the cheaper form (work: a
         Workspace that outlives the call, for captured graphs), else by the
-        walk and the self-kernel."""
+        walk and the self-kernel.  diag_rows: K(x, x) of at least the first so
+        many rows (None: of all)."""
         B, W = bx.shape
         tw = table_workspace(self, B, W, windows, bx.device, work)
         if tw is None:
             raw, _ = self.pairwise(bx, cx, diag_offset, out=out, check=check)
-            return raw, self_kernel(self.spec, bx, rx, cx) if normalize else None
+            n = B if diag_rows is None else diag_rows
+            return raw, (self_kernel(self.spec, bx[:n], None if rx is None else rx[:n], cx[:n]) if normalize else None)
         if out is None:
             out = torch.empty((B, self.S), dtype=torch.float64, device=bx.device)
         diag = torch.empty(B, dtype=torch.float64, device=bx.device) if normalize else None

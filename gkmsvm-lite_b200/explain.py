@@ -339,7 +339,7 @@ def mutation_impact(model, ref, alt, *, ref_lengths=None, alt_lengths=None, batc
         dr = None
         index = model._sv_index()
         if index is not None:
-            kb, dr = index.rows(fwd, rc, counts, base.normalize)
+            kb, dr = index.rows(fwd, rc, counts, base.normalize, diag_rows=n)
         else:
             if base.normalize:
                 dr = engine.self_kernel(spec, fwd[:n], None if rc is None else rc[:n], counts[:n])
