@@ -261,7 +261,8 @@ class DirectScorer:
         self._rerun = None
 
     def score(self, codes: torch.Tensor, lengths: torch.Tensor | None = None, events=None,
-              check: bool = True) -> torch.Tensor:
+              check: bool = True, windows: int = 0) -> torch.Tensor:
+        """BatchedScorer.score; windows: the rows' windows in all (0: unknown)."""
         m = self.model
         spec = m._spec()
         fwd, rc, counts = engine.pack(spec, codes, lengths)
@@ -270,7 +271,7 @@ class DirectScorer:
         if self.table is not None:
             out = engine.table_score(spec, self.table, fwd, rc, counts, m.bias, self.normalize)
         elif (out := self.index.scores(fwd, rc, counts, self.normalize, m._inv_ds(), m._sv_coef(), self.gamma,
-                                       self.rbf, m.bias)) is not None:
+                                       self.rbf, m.bias, windows=windows)) is not None:
             self._rerun = None  # count tables: exact
         else:
             if self.normalize:

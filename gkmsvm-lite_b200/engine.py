@@ -244,6 +244,16 @@ class Workspace:
         return self._buffers[-1][:n]
 
 
+def known_windows(fwd, lengths, l: int) -> int:
+    """The windows of packed rows fwd [B, W] in all, where the host knows the
+    rows' lengths (NumPy, or None: every row is full), else 0."""
+    if lengths is None:
+        return int(fwd.numel())
+    if isinstance(lengths, torch.Tensor):
+        return 0
+    return int(np.clip(lengths - l + 1, 0, None).sum())
+
+
 def table_workspace(index, B: int, W: int, windows: int, device, work: Workspace | None = None):
     """The workspace of a count-table query, or None where the walk serves the
     call or the device has no room for it."""

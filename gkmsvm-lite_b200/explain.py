@@ -220,7 +220,8 @@ def _explain_rows(model, x, lengths, mode, dev, table=None, check=True, work=Non
     pairs = table is None and _explain_uses_pairs(model, perturbation)
     if table is None and not pairs and isinstance(kernel, RbfKernel):
         index = model._sv_index()  # not None: _explain_uses_pairs
-        raw, dx = index.rows(fwd, rc, counts, base.normalize, check=check, work=work)
+        raw, dx = index.rows(fwd, rc, counts, base.normalize, check=check, work=work,
+                             windows=engine.known_windows(fwd, lengths, base.l))
     if not base.normalize:
         inv_dx = torch.ones(B, dtype=torch.float64, device=dev)
     else:
@@ -339,7 +340,8 @@ def mutation_impact(model, ref, alt, *, ref_lengths=None, alt_lengths=None, batc
         dr = None
         index = model._sv_index()
         if index is not None:
-            kb, dr = index.rows(fwd, rc, counts, base.normalize, diag_rows=n)
+            kb, dr = index.rows(fwd, rc, counts, base.normalize, diag_rows=n,
+                                windows=engine.known_windows(fwd, pair.lengths, base.l))
         else:
             if base.normalize:
                 dr = engine.self_kernel(spec, fwd[:n], None if rc is None else rc[:n], counts[:n])

@@ -63,10 +63,10 @@ def _ism_rows(model, x, lengths, dev, check=True, work=None, table_work=None):
     if table is not None:
         _, raw, diag = engine.table_score(spec, table, fwd, rc, counts, 0.0, base.normalize, want_parts=True)
         return engine.ism_table(spec, table, fwd, counts, L, raw, diag, base.normalize)
-    return _ism_index(model, fwd, rc, counts, L, check, work, table_work)
+    return _ism_index(model, fwd, rc, counts, L, check, work, table_work, engine.known_windows(fwd, lengths, base.l))
 
 
-def _ism_index(model, fwd, rc, counts, L, check=True, work=None, table_work=None):
+def _ism_index(model, fwd, rc, counts, L, check=True, work=None, table_work=None, windows=0):
     kernel = model.kernel
     base = kernel.base
     spec = model._spec()
@@ -86,7 +86,7 @@ def _ism_index(model, fwd, rc, counts, L, check=True, work=None, table_work=None
 
     def run():
         # the reference rows' K_raw; their scores come from it inside the call
-        ref_raw, diag = index.rows(fwd, rc, counts, base.normalize, check=False, work=table_work)
+        ref_raw, diag = index.rows(fwd, rc, counts, base.normalize, check=False, work=table_work, windows=windows)
         if base.normalize:
             mut = engine.mutant_diag(spec, fwd, counts, L, diag)
             inv_dx = 1.0 / torch.sqrt(torch.clamp(diag, min=1e-20))

@@ -280,12 +280,7 @@ class GkmSVM:
         dev = self._require_gpu()
         xt = device_codes(codes, dev)
         fwd, rc, counts = engine.pack(self._spec(), xt, lengths)
-        windows = 0
-        if lengths is None:
-            windows = int(fwd.numel())
-        elif not isinstance(lengths, torch.Tensor):
-            windows = int(np.clip(lengths - self.kernel.l + 1, 0, None).sum())
-        return self._score_packed(fwd, rc, counts, windows)
+        return self._score_packed(fwd, rc, counts, engine.known_windows(fwd, lengths, self.kernel.l))
 
     def _score_unbatched(self, batch: SeqBatch) -> torch.Tensor:
         W = max(batch.L - self.kernel.l + 1, 1)

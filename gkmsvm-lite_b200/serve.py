@@ -448,8 +448,12 @@ class GpuBackend:
         with torch.cuda.stream(stream):
             xd = torch.from_numpy(codes).pin_memory().to(self.model._device, non_blocking=True)
             ld = torch.from_numpy(lens).pin_memory().to(self.model._device, non_blocking=True)
-            scorer = self.direct[slot] if len(rows) <= self.direct_rows else self.scorers[slot]
-            out = scorer.score(xd, ld, check=False)
+            if len(rows) <= self.direct_rows:
+                scorer = self.direct[slot]
+                out = scorer.score(xd, ld, check=False, windows=int(np.clip(lens - self.model.kernel.l + 1, 0, None).sum()))
+            else:
+                scorer = self.scorers[slot]
+                out = scorer.score(xd, ld, check=False)
             host = torch.empty(out.shape, dtype=out.dtype, pin_memory=True)
             host.copy_(out, non_blocking=True)
             ev = torch.cuda.Event()
