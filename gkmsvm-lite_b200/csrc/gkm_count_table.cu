@@ -31,6 +31,7 @@
 // adds made) is counted again with 32-bit counters, one level of one query each,
 // and clipped alike.
 #include <cuda_runtime.h>
+#include <math.h>
 #include <stdint.h>
 #include <stdlib.h>
 
@@ -1281,15 +1282,23 @@ static CtPlan ct_plan(const gkm_index *ix, int64_t B, int64_t W, int64_t windows
     return p;
 }
 
-// Microseconds of a query, measured on B200 (l = 10 and 11, 300 .. 72,000 SVs of 200
-// .. 500 bp, 1 .. 1,024 rows of 30 .. 1,000 bp; 90 % of 322 shapes within 27 %, and
-// none that takes the tables by them is slower than the walk).  Count tables: a wave of
-// tile passes costs CT_ITEM_US plus CT_WINDOW_US per window of the pass's rows, the
-// gather reads the SVs' table rows at CT_GATHER_BYTES_US.  Index walk: its lookups and
-// hits, at least WALK_FLOOR_US (a few rows leave most SMs idle and a row's masks are a
-// serial walk).  At 72,000 SVs, t=3, the tables win from one 300 bp row (1.3 -> 0.2 ms)
-// on; at 30 bp rows from 64 at a time the walk does (1,024 rows: 7.5 against 4.0 ms).
+// Microseconds of a query, measured on B200 (l = 8 .. 11, d = 0 .. 3, 64 .. 72,000 SVs
+// of 200 .. 350 bp, 1 .. 1,024 rows of 30 .. 2,000 bp).  Count tables: a wave of tile
+// passes costs CT_ITEM_US plus CT_WINDOW_US per window of the pass's rows, the gather
+// reads the SVs' table rows at CT_GATHER_BYTES_US.  Short l-mers have few positions
+// outside the suffix, so most windows lie in the buckets of budget 0, which the warps
+// share 32 buckets at a time: at l = 8, d = 2 one warp lists 27 of 37 parts of a pass's
+// windows, CT_LIST_US per round of 32 (1,024 x 2,000 bp against 64 SVs: 13.0 ms, the
+// walk 5.9).  And weighted counts past a mean of CT_RECOUNT_MEAN overflow the shared
+// fields of most of their few tiles, which are then counted CT_RECOUNT times (the same
+// rows, weighted: 61.7 against 5.3 ms).  Index walk: its lookups and hits, at least
+// WALK_FLOOR_US (a few rows leave most SMs idle and a row's masks are a serial walk).
+// Of 4,450 measured shapes 3,022 take the tables by these, 3 of them slower so (by up to
+// 1.21; without the two terms for short l-mers 51, by up to 11.5).  At 72,000 SVs, t=3,
+// the tables win from one 300 bp row (1.3 -> 0.2 ms) on; at 30 bp rows from 64 at a time
+// the walk does (1,024 rows: 7.5 against 4.0 ms).
 constexpr double CT_CALL_US = 45.0, CT_ITEM_US = 12.0, CT_WINDOW_US = 8.5e-4, CT_GATHER_BYTES_US = 8.0e6;
+constexpr double CT_LIST_US = 0.3, CT_RECOUNT = 4.0, CT_RECOUNT_MEAN = 24.0;
 constexpr double WALK_FLOOR_US = 400.0, WALK_LOOKUP_US[2] = {8.0e-6, 5.8e-6}, WALK_HIT_US[2] = {1.1e-6, 2.0e-6};
 
 // Whether every count stays below 2^32: the (row, SV) weight products of rows of W
@@ -1318,12 +1327,21 @@ static bool ct_applies(const gkm_index *ix, int64_t B, int64_t W, int64_t window
     const int64_t items = p.rows / CT_ROWS * p.passes;
     const double row = (double)windows / B < W ? (double)windows / B : (double)W, waves = (double)((items + gkm_sm_count() * CT_BLOCKS - 1) / (gkm_sm_count() * CT_BLOCKS));
     const double queries = (double)(B < p.pass ? B : p.pass);
-    const double table = CT_CALL_US + p.groups * (waves * (CT_ITEM_US + CT_WINDOW_US * row * queries) +
-                                                  (double)ix->ct_entries * p.rb / CT_GATHER_BYTES_US);
+    // rounds of 32 windows that a warp lists from the buckets of budget 0
+    double far = 1.0;
+    for (int m = 0; m < ix->spec.dmax; m++) far *= 3.0 * (ix->spec.l - CT_POS - m) / (m + 1);
+    const double warps = far > 32.0 * CT_WARPS ? CT_WARPS : ceil(far / 32.0);
+    const double list = ix->strands * row * queries * far / p.n_pre / 32.0 / warps;
+    const double window = CT_WINDOW_US * row * queries;
+    double slow = CT_ITEM_US + (window > CT_LIST_US * list ? window : CT_LIST_US * list);
+    if (wt && ix->spec.l <= 9 && ct_mean(ix, W) > CT_RECOUNT_MEAN) slow *= CT_RECOUNT;
+    const double gather = (double)ix->ct_entries * p.rb / CT_GATHER_BYTES_US;
+    const double table = CT_CALL_US + p.groups * (waves * (CT_ITEM_US + window) + gather),
+                 table_slow = CT_CALL_US + p.groups * (waves * slow + gather);
     double walk = (double)windows * (ix->n_masks * (double)ix->tiles * WALK_LOOKUP_US[wt] +
                                      (double)ix->entries * ix->n_masks / ix->n_lmers * WALK_HIT_US[wt]);
     if (walk < WALK_FLOOR_US) walk = WALK_FLOOR_US;
-    return table < 0.9 * walk;
+    return table < 0.9 * walk && table_slow < walk;
 }
 
 extern "C" int gkm_count_table_workspace(const gkm_index_t *ix, int64_t B, int64_t W, int64_t windows, int64_t *bytes)
