@@ -276,6 +276,7 @@ class DeviceIndex:
         self.spec = spec
         self.S = fwd.shape[0]
         self.masks = masks
+        self.sms = torch.cuda.get_device_properties(fwd.device).multi_processor_count
         h = ctypes.c_void_p()
         call("gkm_index_create" if tables else "gkm_index_create_walk", spec.ref, ptr(fwd), ptr(rc), ptr(counts),
              fwd.shape[0], fwd.shape[1], ptr(masks), int(masks.numel()), int(tile_svs), ctypes.byref(h), _st())

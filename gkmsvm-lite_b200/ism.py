@@ -4,8 +4,9 @@ Window-delta form: a substitution at p changes only the <= l windows that
 cover p.  Kernels with an l-mer table read the changed windows' table weights
 and the mutant self-kernels in one fused pass (gkm_ism_table); other kernels
 (RBF) count the window pairs each substitution changes once per SV and reduce
-over the SVs (gkm_ism_pairs), or where that does not apply add the changed
-windows' index hits to the reference row's kernel values (gkm_index_mutants).
+over the SVs (gkm_ism_pairs), or where that does not apply or costs more add the
+changed windows' index hits to the reference row's kernel values
+(gkm_index_mutants).
 """
 
 from __future__ import annotations
@@ -18,7 +19,44 @@ import torch
 from . import engine
 from ._lib import call, ptr, stream_handle
 from .inputs import SeqBatch, device_codes, per_position
-from .kernels import RbfKernel
+from .kernels import RbfKernel, neighbor_count
+
+# Microseconds of an index-path pass of B rows, measured on B200 (l = 8 .. 11, d = 0 ..
+# 3, 64 .. 72,000 SVs of 200 .. 350 bp, 1 .. 64 rows of 20 .. 2,000 bp: of 2,697
+# shapes pair lists for all are slower than the walk in 1,227, by up to 12 times, by this
+# rule in 144, by up to 1.48; 45 are left to the walk that would be faster by up to 1.48).
+# Pair lists take the rows one after the other: per row the launches, per SV a block's
+# turn, per (SV, position) the mutants' terms, per window pair within dmax + 1 mismatches
+# the counters, per list entry the lists.  The walk takes all rows at once: lookups and
+# hits of the windows that the mutants change, and the reduction of every (mutant, SV).
+_PAIR_ROW_US, _PAIR_SV_US, _PAIR_TERM_US, _PAIR_US, _PAIR_ENTRY_US = 34.0, 6.0e-3, 1.93e-5, 5.7e-6, 1.14e-5
+_PAIR_LMER_US = 2.0e-6
+_WALK_CALL_US, _WALK_SV_US = 34.5, 6.3e-3
+# (unweighted, weighted)
+_WALK_POSITION_US, _WALK_TERM_US = (0.116, 0.085), (4.5e-5, 3.9e-5)
+_WALK_LOOKUP_US, _WALK_HIT_US = (7.1e-6, 4.8e-6), (1.1e-6, 1.7e-6)
+
+
+def _pairs_pay(base, index, B: int, L: int, sms: int) -> bool:
+    """Whether ISM of B rows of L positions costs less by pair lists (one row
+    at a time) than by the walk.  The walk is the faster form for many short
+    rows and small neighbourhoods (64 rows of 60 bp, d=1, 72,000 SVs: 18.8
+    against 34.4 ms; one of 1,000 bp, d=3: 8.7 against 3.8)."""
+    l, S, w = base.l, index.S, int(base.weighted)
+    W, n = L - l + 1, 4**l
+    near = neighbor_count(l, base.dmax + 1)
+    # a block takes an SV at a time, at least one turn each
+    blocks = sms * (4 if L <= 512 else 2 if L <= 1024 else 1)
+    turns = -(-S // blocks) * blocks
+    pairs = W * index.entries / S * turns * near / n
+    row = (_PAIR_ROW_US + _PAIR_SV_US * turns + _PAIR_TERM_US * turns * L + _PAIR_US * pairs + _PAIR_ENTRY_US * W * near
+           + _PAIR_LMER_US * n)
+    changed = 3 * B * L * min(l, W)
+    masks = int(index.masks.numel())
+    walk = (_WALK_CALL_US + _WALK_SV_US * S + B * L * (_WALK_POSITION_US[w] + _WALK_TERM_US[w] * S)
+            + changed * masks * (_WALK_LOOKUP_US[w] * index.tiles + _WALK_HIT_US[w] * index.entries / n))
+    return B * row < walk
+
 
 # Sequences per device pass: ISM outputs [B, 4, L] float64 per pass within this
 _BLOCK_BYTES = 1 * 2**30
@@ -79,7 +117,8 @@ def _ism_index(model, fwd, rc, counts, L, check=True, work=None, table_work=None
     gamma = kernel.gamma if rbf else 0.0
     out = torch.empty((B, 4, L), dtype=torch.float64, device=fwd.device)
     pairs = ctypes.c_int64()
-    call("gkm_ism_pairs_workspace", index.handle, W, L, ctypes.byref(pairs))
+    if _pairs_pay(base, index, B, L, index.sms):
+        call("gkm_ism_pairs_workspace", index.handle, W, L, ctypes.byref(pairs))
     if work is None:
         work = (torch.empty(pairs.value, dtype=torch.uint8, device=fwd.device) if pairs.value
                 else ism_workspace(model, B, L, fwd.device))

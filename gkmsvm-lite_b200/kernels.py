@@ -107,6 +107,7 @@ def mask_plan(table: tuple, l: int, min_matches: int):
             for j, c in zip(sizes, coef) if abs(c) > floor]
 
 
+@lru_cache(maxsize=64)
 def neighbor_count(l: int, dmax: int) -> int:
     return sum(comb(l, m) * 3**m for m in range(dmax + 1))
 
