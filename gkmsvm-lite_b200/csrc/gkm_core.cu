@@ -681,7 +681,8 @@ __global__ void __launch_bounds__(MUT_THREADS) mutant_kernel(
 // base, level).  Pairs whose second window covers the position, too, are the l x l
 // ones about it and are tested directly.  Bound by the integer pipe.  Measured (t=2,
 // 128 x 300 bp): mutant_kernel, every pair at every position, 685 us; this 76 us.
-// mutant_kernel stays for d >= 4 and for rows whose planes outgrow shared memory.
+// mutant_kernel stays for d >= 4, for rows whose planes outgrow shared memory and where
+// it is the faster form (tiles_pay).
 constexpr int MT_THREADS = 256;
 constexpr int MT_WINDOWS = 128;
 constexpr int MT_PLANES = 128 * 1024;  // the most shared memory for a row's planes
@@ -1110,16 +1111,45 @@ extern "C" int gkm_deltasvm_table(const gkm_spec *spec, const double *table, dou
     return GKM_OK;
 }
 
+// The share of window pairs of uniform bases within d mismatches.
+static double pair_share(int l, int d)
+{
+    double c = 1.0, n = 0.0, p = 1.0;
+    for (int m = 0; m <= d && m <= l; m++) {
+        n += c;
+        c = c * 3.0 * (l - m) / (m + 1);
+    }
+    for (int k = 0; k < l; k++) p *= 0.25;
+    return n * p;
+}
+
+// Whether mutant_tiles costs less than mutant_kernel for B rows of W windows.  Microseconds
+// measured on B200 (l = 3 .. 12, d = 0 .. 3, 1 and 32 rows of 20 .. 2,000 bp): a block of
+// mutant_tiles runs every diagonal of its row and each pair within dmax + 1 mismatches one
+// lane per l positions (weighted: 64-bit adds), however few blocks there are; mutant_kernel
+// has a block per position and looks at every window there.  A lone 300 bp row, l = 11, d =
+// 3: 38 against 15 us, 32 of them 46 against 178; short l-mers, where every pair is near:
+// 32 rows of 300 bp at l = 6, d = 3 296 against 119 us, weighted 940.
+static bool tiles_pay(const gkm_spec *spec, int64_t B, int64_t W, int64_t L)
+{
+    const int l = spec->l, P = MT_WINDOWS - l + 1;
+    const double near = pair_share(l, spec->dmax + 1), w = (double)W;
+    const double block = 20.0 + w * (0.016 + near * (spec->weighted ? 1.75 * (spec->dmax + 1) : 0.33 * l));
+    const double fill = (double)((L + P - 1) / P * B) / gkm_sm_count() / 2.1;
+    const double all = 12.0 + (double)B * (double)L * w * (10.0 + 4.0 * l) * 1e-6;
+    return block * (fill > 1.0 ? fill : 1.0) < all;
+}
+
 static int mutant_launch(const gkm_spec *spec, const uint32_t *fwd, const int32_t *counts, int64_t B,
                          int64_t W, int64_t L, const double *diag, double *mut_diag, const double *table,
                          const double *ref_raw, int normalize, double *out, cudaStream_t st)
 {
     if (B == 0 || L == 0) return GKM_OK;
     if (B > 65535) return gkm_fail(GKM_ERR_UNSUPPORTED, "more than 65,535 rows per ISM launch");
-    // four levels, and rows whose bit planes fit shared memory: by diagonals
+    // four levels, rows whose bit planes fit shared memory, and work enough: by diagonals
     const int pw = plane_words(W, spec->l) + 1;
     const size_t planes = (size_t)4 * mutant_plane(pw) * sizeof(uint32_t);
-    if (spec->dmax < 4 && planes <= MT_PLANES) {
+    if (spec->dmax < 4 && planes <= MT_PLANES && tiles_pay(spec, B, W, L)) {
         const int P = MT_WINDOWS - spec->l + 1;
         const dim3 grid((unsigned)((L + P - 1) / P), (unsigned)B);
 #define GKM_MUT_AS(LT, WT)                                                                                     \
@@ -1150,7 +1180,7 @@ static int mutant_launch(const gkm_spec *spec, const uint32_t *fwd, const int32_
         mutant_kernel<NW><<<grid, MUT_THREADS, smem, st>>>(*spec, fwd, counts, B, W, L, diag, mut_diag,  \
                                                            table, ref_raw, normalize, out, sw);          \
     } while (0)
-    if (nw == 1) GKM_MUT(1);  // (rows too long for mutant_tiles' planes)
+    if (nw == 1) GKM_MUT(1);
     else if (nw == 2) GKM_MUT(2);
     else GKM_MUT(4);
 #undef GKM_MUT
