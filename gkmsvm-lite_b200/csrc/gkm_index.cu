@@ -898,7 +898,7 @@ static int index_create(const gkm_spec *spec, const uint32_t *fwd, const uint32_
         free(h);
         if (ix->wmax == 0) ix->wmax = 1;
     }
-    int status = GKM_OK;
+    int status = GKM_OK, lists = GKM_OK;
     uint32_t *ecount = nullptr, *base = nullptr, *keys = nullptr, *vals = nullptr, *kt = nullptr, *vt = nullptr;
     uint32_t total = 0;
     int64_t nbuckets = T * ix->n_lmers;
@@ -987,6 +987,7 @@ static int index_create(const gkm_spec *spec, const uint32_t *fwd, const uint32_
         cudaMemsetAsync(ix->status, 0, 2 * sizeof(unsigned int), st);
         ix->bytes = (int64_t)sizeof(uint32_t) * ((ix->bwords ? 2 : 1) * nbuckets + 1) + (int64_t)eb +
                     sizeof(uint32_t) * n_masks;
+        if (tables) lists = gkm_ct_build(ix, fwd, counts, st);
     } while (0);
     cudaFreeAsync(ecount, st);
     cudaFreeAsync(keys, st);
@@ -997,19 +998,16 @@ static int index_create(const gkm_spec *spec, const uint32_t *fwd, const uint32_
         cudaError_t e = cudaStreamSynchronize(st);
         if (e != cudaSuccess) status = gkm_cuda_status(e, "index build");
     }
-    if (status == GKM_OK && tables) {
-        // after the build's scratch has gone back: the lists then need no more memory at
-        // once than the build did.  Where they do not fit even so, the walk serves the index.
-        status = gkm_ct_build(ix, fwd, counts, st);
-        if (status == GKM_OK) {
-            cudaError_t e = cudaStreamSynchronize(st);
-            if (e != cudaSuccess) status = gkm_cuda_status(e, "gather lists");
-        } else if (status == GKM_ERR_OOM) {
-            (void)cudaGetLastError();  // an allocation's failure leaves nothing behind but its error
-            gkm_ct_free(ix);
-            status = GKM_OK;
-        }
+    // Lists that did not fit beside the build's scratch are tried again now that it has
+    // gone back; where they do not fit even so, the walk serves the index.
+    for (int retry = 1; status == GKM_OK && lists == GKM_ERR_OOM; retry = 0) {
+        (void)cudaGetLastError();  // an allocation's failure leaves nothing behind but its error
+        gkm_ct_free(ix);
+        if (!retry) break;
+        lists = gkm_ct_build(ix, fwd, counts, st);
+        if (lists == GKM_OK && cudaStreamSynchronize(st) != cudaSuccess) lists = gkm_cuda_status(cudaGetLastError(), "gather lists");
     }
+    if (status == GKM_OK && lists != GKM_ERR_OOM) status = lists;
     if (status != GKM_OK) {
         gkm_index_free(ix);
         return status;
