@@ -282,6 +282,38 @@ constexpr int SELF_PLANES = 200 * 1024;  // the most shared memory for a row's p
 // bit plane words of a row of W windows: the bases and three words past them
 __host__ __device__ inline int plane_words(int64_t W, int l) { return (int)((W + l - 1 + 31) / 32) + 3; }
 
+// What both forms do with a row's level sums (tot of every thread).
+template <int NL>
+__device__ __forceinline__ void self_finish(const gkm_spec spec, uint64_t *tot, uint64_t *red, uint64_t *sums, double *dred, int64_t b,
+                            int n, const uint32_t *frow, double *diag, uint64_t *profile, const double *table, double bias,
+                            int normalize, double *scores, double *raw_out)
+{
+    block_reduce_levels<NL>(tot, red, sums);
+    double k = 0.0;
+#pragma unroll
+    for (int m = 0; m < NL; m++)
+        if (m <= spec.dmax) k += spec.h[m] * (double)sums[m];
+    if (threadIdx.x == 0) {
+        if (diag) diag[b] = k;
+        if (profile)
+            for (int m = 0; m <= spec.l; m++)
+                profile[b * (spec.l + 1) + m] = (m < NL && m <= spec.dmax) ? sums[m] : 0;
+    }
+    if (table) {
+        double t = 0.0;
+        for (int i = threadIdx.x; i < n; i += blockDim.x) {
+            double a = spec.weighted ? (double)gkm_wt(spec.wd, n, i) : 1.0;
+            t += a * table[frow[i]];
+        }
+        t = gkm_block_sum(t, dred);
+        if (threadIdx.x == 0) {
+            if (raw_out) raw_out[b] = t;
+            double s = normalize ? t / sqrt(fmax(k, 1e-10)) : t;
+            scores[b] = s + bias;
+        }
+    }
+}
+
 // Self-kernel of one row per block, optionally fused with the l-mer table sum
 // (svm.py:559-582: score = sum_i wt_i table[x_i] / sqrt(K(x, x)) + b).
 //
@@ -292,8 +324,9 @@ __host__ __device__ inline int plane_words(int64_t W, int l) { return (int)((W +
 // RC pairs are the diagonals of the sequence against its reverse complement, each
 // symmetric about its middle: half of it is summed.  Bound by the integer pipe;
 // measured fused with the table sum (t=2): 8,192 rows of 50 .. 2,000 bp 4,516 us
-// pair by pair -> 633 us, 512 rows of 1,000 bp 544 -> 71 us.  Rows whose windows do not overlap (not one sequence's) or whose planes do
-// not fit shared memory are still taken pair by pair.
+// pair by pair -> 633 us, 512 rows of 1,000 bp 544 -> 71 us.  Rows whose windows do not
+// overlap (not one sequence's) or whose planes do not fit shared memory are still taken
+// pair by pair.
 template <int L, int NL, bool WT>
 __global__ void __launch_bounds__(SELF_THREADS) self_kernel(
     gkm_spec spec, const uint32_t *__restrict__ fwd, const uint32_t *__restrict__ rc,
@@ -382,30 +415,44 @@ __global__ void __launch_bounds__(SELF_THREADS) self_kernel(
             if (threadIdx.x == 0) tot[0] += n;
         }
     }
-    block_reduce_levels<NL>(tot, red, sums);
-    double k = 0.0;
+    self_finish<NL>(spec, tot, red, sums, dred, b, n, frow, diag, profile, table, bias, normalize, scores, raw_out);
+}
+
+// The same pair by pair, for weighted kernels whose pairs mostly count (pairs_pay): there
+// the diagonals above take every counted pair one by one, with 64-bit sums, and this does
+// so with less work a pair.
+template <int NW>
+__global__ void __launch_bounds__(SELF_THREADS) self_pairs_kernel(
+    gkm_spec spec, const uint32_t *__restrict__ fwd, const uint32_t *__restrict__ rc,
+    const int32_t *__restrict__ counts, int64_t W, double *__restrict__ diag,
+    uint64_t *__restrict__ profile, const double *__restrict__ table, double bias, int normalize,
+    double *__restrict__ scores, double *__restrict__ raw_out, int sw)
+{
+    constexpr int NL = 4 * NW;
+    extern __shared__ uint32_t sm[];  // the row's forward and RC windows, sw words each
+    __shared__ uint64_t red[(SELF_THREADS / 32) * NL];
+    __shared__ uint64_t sums[NL];
+    __shared__ double dred[32];
+    const int64_t b = blockIdx.x;
+    const int n = counts[b];
+    const bool has_rc = spec.include_rc && rc != nullptr;
+    const uint32_t *frow = fwd + b * W, *rrow = has_rc ? rc + b * W : nullptr;
+    RowView rv = {frow, rrow, W, true};
+    if (n <= sw) {
+        for (int k = threadIdx.x; k < n; k += SELF_THREADS) {
+            sm[k] = frow[k];
+            if (has_rc) sm[sw + k] = rrow[W - 1 - k];
+        }
+        rv.f = sm;
+        rv.r = sm + sw;
+        rv.reversed = false;
+    }
+    __syncthreads();
+    uint64_t tot[NL];
 #pragma unroll
-    for (int m = 0; m < NL; m++)
-        if (m <= spec.dmax) k += spec.h[m] * (double)sums[m];
-    if (threadIdx.x == 0) {
-        if (diag) diag[b] = k;
-        if (profile)
-            for (int m = 0; m <= spec.l; m++)
-                profile[b * (spec.l + 1) + m] = (m < NL && m <= spec.dmax) ? sums[m] : 0;
-    }
-    if (table) {
-        double t = 0.0;
-        for (int i = threadIdx.x; i < n; i += blockDim.x) {
-            double a = spec.weighted ? (double)gkm_wt(spec.wd, n, i) : 1.0;
-            t += a * table[frow[i]];
-        }
-        t = gkm_block_sum(t, dred);
-        if (threadIdx.x == 0) {
-            if (raw_out) raw_out[b] = t;
-            double s = normalize ? t / sqrt(fmax(k, 1e-10)) : t;
-            scores[b] = s + bias;
-        }
-    }
+    for (int m = 0; m < NL; m++) tot[m] = 0;
+    self_pairs<NW>(rv, n, has_rc, spec.wd, spec.weighted, tot);
+    self_finish<NL>(spec, tot, red, sums, dred, b, n, frow, diag, profile, table, bias, normalize, scores, raw_out);
 }
 
 // ---------------------------------------------------------------------------
@@ -984,6 +1031,34 @@ extern "C" int gkm_pack(const gkm_spec *spec, const uint8_t *codes, const int64_
     return GKM_OK;
 }
 
+// The share of window pairs of uniform bases within d mismatches.
+static double pair_share(int l, int d)
+{
+    double c = 1.0, n = 0.0, p = 1.0;
+    for (int m = 0; m <= d && m <= l; m++) {
+        n += c;
+        c = c * 3.0 * (l - m) / (m + 1);
+    }
+    for (int k = 0; k < l; k++) p *= 0.25;
+    return n * p;
+}
+
+// Whether a weighted self-kernel costs less pair by pair: past this share of pairs that
+// count (d past 7 makes a pair dearer, 16 levels), and a larger one for many short rows,
+// whose warps the pair loop leaves half empty.  Measured on B200, by diagonals and pair by
+// pair: 32 rows of 2,000 bp, l = 8, d = 7 (90 % of the pairs) 3,494 and 1,086 us; l = 9, d =
+// 5 (17 %) 1,409 and 1,084; l = 9, d = 4 (5 %) 831 and 1,088; l = 15, d = 14 (99 %) 5,083
+// and 2,434; 512 rows of 150 bp, l = 12, d = 9 (61 %) 66 and 128.  Of 1,552 shapes (l = 3 ..
+// 15, every d) diagonals for all are slower by more than a tenth in 290, by up to 3.2
+// times, by this rule 9, by up to 1.25.
+static bool pairs_pay(const gkm_spec *spec, int64_t B, int64_t W)
+{
+    if (!spec->weighted) return false;
+    double share = spec->dmax < 4 ? 0.16 : spec->dmax < 8 ? 0.14 : 0.45;
+    if (B > 2 * gkm_sm_count() && W < 512) share *= 750.0 / (double)W;
+    return pair_share(spec->l, spec->dmax) > share;
+}
+
 static int self_launch(const gkm_spec *spec, const uint32_t *fwd, const uint32_t *rc, const int32_t *counts,
                        int64_t B, int64_t W, double *diag, uint64_t *profile, const double *table, double bias,
                        int normalize, double *scores, double *raw, cudaStream_t st)
@@ -992,6 +1067,23 @@ static int self_launch(const gkm_spec *spec, const uint32_t *fwd, const uint32_t
     int pw = plane_words(W, spec->l);
     size_t smem = (size_t)4 * pw * sizeof(uint32_t);
     if (smem > SELF_PLANES) smem = pw = 0;
+    if (pairs_pay(spec, B, W)) {
+        const int sw = staged_windows(W), nw = nw_for(spec->dmax);
+        const size_t staged = (size_t)2 * sw * sizeof(uint32_t);
+#define GKM_SELF_PAIRS(NW)                                                                                \
+    do {                                                                                                  \
+        GKM_ALLOW_SHARED(self_pairs_kernel<NW>, 2 * SMEM_WINDOWS * sizeof(uint32_t));                     \
+        GKM_PREFER_SHARED(self_pairs_kernel<NW>);                                                         \
+        self_pairs_kernel<NW><<<(unsigned)B, SELF_THREADS, staged, st>>>(                                 \
+            *spec, fwd, rc, counts, W, diag, profile, table, bias, normalize, scores, raw, sw);           \
+    } while (0)
+        if (nw == 1) GKM_SELF_PAIRS(1);
+        else if (nw == 2) GKM_SELF_PAIRS(2);
+        else GKM_SELF_PAIRS(4);
+#undef GKM_SELF_PAIRS
+        GKM_CHECK_LAUNCH("self_pairs_kernel");
+        return GKM_OK;
+    }
 #define GKM_SELF_AS(L, NL, WT)                                                                                \
     do {                                                                                                      \
         GKM_ALLOW_SHARED((self_kernel<L, NL, WT>), SELF_PLANES);                                              \
@@ -1109,18 +1201,6 @@ extern "C" int gkm_deltasvm_table(const gkm_spec *spec, const double *table, dou
                                                                                         query_norm, out, n);
     GKM_CHECK_LAUNCH("deltasvm_table");
     return GKM_OK;
-}
-
-// The share of window pairs of uniform bases within d mismatches.
-static double pair_share(int l, int d)
-{
-    double c = 1.0, n = 0.0, p = 1.0;
-    for (int m = 0; m <= d && m <= l; m++) {
-        n += c;
-        c = c * 3.0 * (l - m) / (m + 1);
-    }
-    for (int k = 0; k < l; k++) p *= 0.25;
-    return n * p;
 }
 
 // Whether mutant_tiles costs less than mutant_kernel for B rows of W windows.  Microseconds
