@@ -72,20 +72,36 @@ def _explain_subsets(model, perturbation: bool, dev):
     return c[key]
 
 
-# Seconds per bucket entry an RBF model's explain_windows visits from its windows,
-# and per index entry of a row_weights pass (four rows), measured on B200 at 72,000
-# SVs
-_BUCKET_VISIT_S = 4.1e-11
-_ROW_WEIGHTS_S = 5e-12
+# Microseconds of an RBF model's attributions past what both forms share, measured on
+# B200 (l = 6 .. 12, d = 0 .. 4, 64 .. 72,000 SVs of 200 .. 350 bp, 1 .. 50 rows of 40 ..
+# 1,500 bp).  By l-mer weights: per group of four rows the index entries and, one thread
+# after the other, the entries of a bucket; per row the writing of 4^l weights; per (window,
+# neighbour) a gather, a dearer one where a row's weights outgrow L2 (l = 12).  By buckets
+# (explain_windows): (window, neighbour) pairs, bucket entries visited, at least a warp's
+# way through the neighbours.
+_WEIGHTS_CALL_US, _WEIGHTS_GROUP_US, _WEIGHTS_ENTRY_US, _WEIGHTS_BUCKET_US = 323.0, 4.0, 3.9e-6, 0.94
+_WEIGHTS_LMER_US, _WEIGHTS_GATHER_US, _WEIGHTS_FAR_US = 1.5e-5, 1.5e-5, 1.0e-4
+_BUCKET_CALL_US, _BUCKET_MASK_US, _BUCKET_CHAIN_US = 840.0, 0.075, 0.023
+_BUCKET_LOOKUP_US, _BUCKET_VISIT_US, _BUCKET_SV_US = 2.4e-5, 1.6e-5, 9.6e-5
+_L2_BYTES = 126 * 2**20
 # device memory of the rows' l-mer weights at a time
 _ROW_WEIGHTS_BYTES = 512 * 2**20
 
 
 def _row_weights_pay(model, index, n_windows: int, rows: int, n_masks: int) -> bool:
     """Whether building each row's l-mer weights costs less than visiting the
-    buckets of its windows' neighbourhoods."""
-    visits = n_windows * n_masks * (index.entries / 4**model.kernel.base.l)
-    return visits * _BUCKET_VISIT_S > -(-rows // 4) * index.entries * _ROW_WEIGHTS_S + 4e-5
+    buckets of its windows' neighbourhoods.  Of 2,280 measured shapes the
+    slower form runs in 82, by up to 1.3 where it is this one (a rule without
+    the terms of 4^l and of a bucket's length: 5.7)."""
+    n = 4**model.kernel.base.l
+    groups, pairs, bucket = -(-rows // 4), n_windows * n_masks, index.entries / n
+    gather = _WEIGHTS_GATHER_US + (_WEIGHTS_FAR_US if 8 * n > _L2_BYTES else 0.0)
+    weights = (_WEIGHTS_CALL_US + groups * (_WEIGHTS_GROUP_US + _WEIGHTS_ENTRY_US * index.entries
+                                            + _WEIGHTS_BUCKET_US * bucket)
+               + rows * n * _WEIGHTS_LMER_US + pairs * gather)
+    buckets = (_BUCKET_CALL_US + n_masks * (_BUCKET_MASK_US + _BUCKET_CHAIN_US * bucket)
+               + pairs * (_BUCKET_LOOKUP_US + _BUCKET_VISIT_US * bucket) + rows * index.S * _BUCKET_SV_US)
+    return weights < 0.9 * buckets
 
 
 def _explain_V(model) -> torch.Tensor:
@@ -247,18 +263,22 @@ def _explain_rows(model, x, lengths, mode, dev, table=None, check=True, work=Non
         subsets = _explain_subsets(model, perturbation, dev)
         if index is not None and not _row_weights_pay(model, index, B * W, B, int(masks.numel())):
             subsets = None
+    n = 4**base.l
+    step = B
+    if subsets is not None and index is not None:
+        step = min(B, max(4, _ROW_WEIGHTS_BYTES // (8 * n) // 4 * 4))
+        try:  # (a captured pass: the workspace its K_raw rows are done with)
+            V = (torch.empty((step, n), dtype=torch.float64, device=dev) if work is None
+                 else work.get(8 * step * n, dev).view(torch.float64).view(step, n))
+        except torch.cuda.OutOfMemoryError:
+            subsets = None  # the buckets need no memory of their own
     if subsets is not None:
         subs, lists, n_with, size = subsets
-        n = 4**base.l
         out = torch.empty((B, 4, L), dtype=torch.float64, device=dev)
-        step = B if V is not None else max(4, _ROW_WEIGHTS_BYTES // (8 * n) // 4 * 4)
-        part = torch.empty((min(B, step), W, 4, base.l), dtype=torch.float64, device=dev)
+        part = torch.empty((step, W, 4, base.l), dtype=torch.float64, device=dev)
         for s in range(0, B, step):
             r = min(step, B - s)
             if index is not None:
-                # (a captured pass: the workspace its K_raw rows are done with)
-                V = (torch.empty((r, n), dtype=torch.float64, device=dev) if work is None
-                     else work.get(8 * r * n, dev).view(torch.float64).view(r, n))
                 for g in range(0, r, 4):
                     k = min(4, r - g)
                     width = 4 if k == 3 else k
