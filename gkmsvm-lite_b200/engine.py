@@ -209,10 +209,11 @@ def masks_tensor(base, device) -> torch.Tensor:
 
 
 class Workspace:
-    """A device buffer that grows on request, shared by the passes of one
-    object; every buffer handed out is kept for the object's life, because
-    captured graphs refer to it.  Passes that use it are queued within
-    turn(), from any stream and thread."""
+    """A device buffer that grows on request, by half at least, shared by the
+    passes of one object; every buffer handed out is kept for the object's
+    life, because captured graphs refer to it (all of them together take less
+    than five times the largest request).  Passes that use it are queued
+    within turn(), from any stream and thread."""
 
     def __init__(self):
         self._buffers = []
@@ -239,8 +240,13 @@ class Workspace:
                     self._done = done
 
     def get(self, n: int, device) -> torch.Tensor:
-        if not self._buffers or self._buffers[-1].numel() < n:
-            self._buffers.append(torch.empty(n, dtype=torch.uint8, device=device))
+        last = self._buffers[-1].numel() if self._buffers else 0
+        if last < n or last == 0:
+            try:
+                buffer = torch.empty(max(n, last + last // 2), dtype=torch.uint8, device=device)
+            except torch.cuda.OutOfMemoryError:
+                buffer = torch.empty(n, dtype=torch.uint8, device=device)
+            self._buffers.append(buffer)
         return self._buffers[-1][:n]
 
 

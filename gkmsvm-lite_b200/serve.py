@@ -351,7 +351,9 @@ class GpuBackend:
         multiples of 1,024 up to max_rows, side calls of max_side_rows, lengths
         64..max_len) on rows of length 0, which have no windows and so almost
         no work: a bucket's first use and its capture then never fall inside
-        a request's latency (the graphs do not depend on the rows' contents)."""
+        a request's latency (the graphs do not depend on the rows' contents).
+        The largest buckets go first: the scorers and runners then make the
+        workspace that serves all of them."""
         torch = self.torch
         from .batch import BatchedExplain, BatchedIsm, _bucket_len
 
@@ -361,8 +363,8 @@ class GpuBackend:
             lengths.append(lengths[-1] * 2)
         for i, scorer in enumerate(self.scorers):
             with torch.cuda.stream(self.streams[i]):
-                for rows in range(1024, max_rows + 1, 1024):
-                    for L in lengths:
+                for rows in reversed(range(1024, max_rows + 1, 1024)):
+                    for L in reversed(lengths):
                         x = torch.zeros((rows, L), dtype=torch.uint8, device=dev)
                         ln = torch.zeros(rows, dtype=torch.int64, device=dev)
                         for _ in range(2):
@@ -374,7 +376,7 @@ class GpuBackend:
                     runner = self.side_runners[key] = (BatchedIsm(self.model, self.side_pass_positions)
                                                        if key == "ism" else BatchedExplain(self.model, key[1]))
                 try:
-                    for L in lengths:
+                    for L in reversed(lengths):
                         x = torch.zeros((runner.row_granule, L), dtype=torch.uint8, device=dev)
                         ln = torch.zeros(runner.row_granule, dtype=torch.int64, device=dev)
                         for _ in range(2):

@@ -88,3 +88,17 @@ def test_threads_take_turns(cuda):
     launches = [e[0] for e in log if e[1] == "launch"]
     assert len(launches) == 3000
     assert all(len(set(launches[i:i + 5])) == 1 for i in range(0, 3000, 5))
+
+
+def test_growth_is_bounded():
+    """Requests that rise a little at a time, as a server's buckets do."""
+    w = engine.Workspace()
+    sizes = [1000 + 37 * k for k in range(60)]
+    for n in sizes:
+        assert w.get(n, "cpu").numel() == n
+    assert sum(b.numel() for b in w._buffers) <= 3 * sizes[-1]
+    assert len(w._buffers) <= 5
+    before = len(w._buffers)
+    for n in (0, 10, sizes[-1]):
+        assert w.get(n, "cpu").numel() == n
+    assert len(w._buffers) == before
