@@ -147,8 +147,9 @@ __device__ __forceinline__ int64_t ct_row_of(const CtArgs &a, int q)
 // Adds the excess counts ex (by t) of l-mer v and query q to the counts of the
 // SVs holding v, lanes lane, lane + nl, ... of its buckets.  Without folding the
 // rows of v and rc(v) hold the same counts and both strands of an SV are in the
-// buckets, so v <= rc(v) stands for both; a palindrome's bucket holds every
-// window twice in a row.
+// buckets, so v <= rc(v) stands for both; a palindrome's bucket holds every window of an
+// SV twice, the forward ones in window order and then mirrored (w1 w2 w2 w1: entry_gen's
+// order, kept by the stable sort), so that every second entry is every window once.
 template <bool WT>
 __device__ void ct_excess(const CtArgs &a, uint32_t v, int q, const uint64_t *ex, int lane, int nl)
 {

@@ -211,7 +211,8 @@ __global__ void entry_counts(const int32_t *__restrict__ counts, int64_t S, int 
 
 // Entries in column order: each SV's forward windows, then its RC windows in
 // RC-row order (kernels/lmer_index.py:171-176), so a stable sort keeps every
-// bucket ascending by SV.  key = tile << 2l | l-mer; value = local SV id |
+// bucket ascending by SV (the count tables read palindromes' buckets by this order, see
+// ct_excess).  key = tile << 2l | l-mer; value = local SV id |
 // window weight << 24.
 __global__ void entry_gen(gkm_spec spec, const uint32_t *__restrict__ fwd, const uint32_t *__restrict__ rc,
                           const int32_t *__restrict__ counts, const uint32_t *__restrict__ base, int64_t S,
