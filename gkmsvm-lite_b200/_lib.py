@@ -58,6 +58,8 @@ SIGNATURES = {
     "gkm_join_pairwise": [SPEC, P, P, I64, I64, P, P, P, I64, I64, P, P, P],
     "gkm_dense_pairwise": [SPEC, P, P, I64, I64, P, P, P, I64, I64, P, P, P, P],
     "gkm_dense_set_role_wait": [I64],
+    "gkm_self_form": [SPEC, I64, I64],
+    "gkm_mutant_form": [SPEC, I64, I64, I64],
     "gkm_index_create": [SPEC, P, P, P, I64, I64, P, I32, I32, P, P],
     "gkm_index_create_walk": [SPEC, P, P, P, I64, I64, P, I32, I32, P, P],
     "gkm_index_free": [P],

@@ -1220,16 +1220,38 @@ static bool tiles_pay(const gkm_spec *spec, int64_t B, int64_t W, int64_t L)
     return block * (fill > 1.0 ? fill : 1.0) < all;
 }
 
+// Whether mutant_tiles takes a launch: four levels, rows whose bit planes fit shared
+// memory, and work enough.
+static size_t tile_planes(const gkm_spec *spec, int64_t W, int *pw)
+{
+    *pw = plane_words(W, spec->l) + 1;
+    return (size_t)4 * mutant_plane(*pw) * sizeof(uint32_t);
+}
+static bool tiles_apply(const gkm_spec *spec, int64_t B, int64_t W, int64_t L)
+{
+    int pw;
+    return spec->dmax < 4 && tile_planes(spec, W, &pw) <= MT_PLANES && tiles_pay(spec, B, W, L);
+}
+
+extern "C" int gkm_self_form(const gkm_spec *spec, int64_t B, int64_t W)
+{
+    return spec && check_spec(spec) == GKM_OK && pairs_pay(spec, B, W) ? 1 : 0;
+}
+
+extern "C" int gkm_mutant_form(const gkm_spec *spec, int64_t B, int64_t W, int64_t L)
+{
+    return spec && check_spec(spec) == GKM_OK && tiles_apply(spec, B, W, L) ? 1 : 0;
+}
+
 static int mutant_launch(const gkm_spec *spec, const uint32_t *fwd, const int32_t *counts, int64_t B,
                          int64_t W, int64_t L, const double *diag, double *mut_diag, const double *table,
                          const double *ref_raw, int normalize, double *out, cudaStream_t st)
 {
     if (B == 0 || L == 0) return GKM_OK;
     if (B > 65535) return gkm_fail(GKM_ERR_UNSUPPORTED, "more than 65,535 rows per ISM launch");
-    // four levels, rows whose bit planes fit shared memory, and work enough: by diagonals
-    const int pw = plane_words(W, spec->l) + 1;
-    const size_t planes = (size_t)4 * mutant_plane(pw) * sizeof(uint32_t);
-    if (spec->dmax < 4 && planes <= MT_PLANES && tiles_pay(spec, B, W, L)) {
+    if (tiles_apply(spec, B, W, L)) {
+        int pw;
+        const size_t planes = tile_planes(spec, W, &pw);
         const int P = MT_WINDOWS - spec->l + 1;
         const dim3 grid((unsigned)((L + P - 1) / P), (unsigned)B);
 #define GKM_MUT_AS(LT, WT)                                                                                     \

@@ -107,6 +107,12 @@ int gkm_dense_pairwise(const gkm_spec *spec, const uint32_t *bx, const int32_t *
  * (up to 1 s) for its copies and MMAs in flight and frees its tensor memory.
  * No counterpart in gkmsvm-lite. */
 int gkm_dense_set_role_wait(int64_t ns);
+/* Test hooks: the form that a self-kernel of B rows of W windows takes (1: pair by
+ * pair, 0: by bit-sliced diagonals), and that of mutant self-kernels of B rows of W
+ * windows and L positions (1: by diagonals, a tile of positions a block, 0: a block
+ * per position).  The forms give equal results.  No counterpart in gkmsvm-lite. */
+int gkm_self_form(const gkm_spec *spec, int64_t B, int64_t W);
+int gkm_mutant_form(const gkm_spec *spec, int64_t B, int64_t W, int64_t L);
 
 /* Builds the l-mer index over S columns (radix sort of the packed l-mers of
  * their forward and RC windows into per-SV-tile CSR buckets).  masks [n_masks]

@@ -8,21 +8,11 @@ import pytest
 import torch
 
 import gkmsvm_lite_b200 as gk
-from gkmsvm_lite_b200 import engine
+from gkmsvm_lite_b200 import _lib, engine
 
 pytestmark = pytest.mark.gpu
 
-PROFILER = [torch.profiler.ProfilerActivity.CUDA]
-
-
-def _ran(fn):
-    """fn()'s result and the names of the kernels it launched."""
-    fn()
-    torch.cuda.synchronize()
-    with torch.profiler.profile(activities=PROFILER) as prof:
-        out = fn()
-        torch.cuda.synchronize()
-    return out, " ".join(e.key for e in prof.key_averages())
+FORMS = ["mutant_kernel", "mutant_tiles"]
 
 
 # kernel type, l, d, rows, length; the forms of the batch and of one row
@@ -45,10 +35,10 @@ def test_forms_agree(kt, l, d, B, L, batch, row):
     spec = m._spec()
     fwd, rc, counts = engine.pack(spec, torch.from_numpy(x).cuda(), xl)
     diag = engine.self_kernel(spec, fwd, rc, counts)
-    got, names = _ran(lambda: engine.mutant_diag(spec, fwd, counts, L, diag))
-    assert batch in names
+    W, form = fwd.shape[1], _lib.load().gkm_mutant_form
+    assert (FORMS[form(spec.ref, B, W, L)], FORMS[form(spec.ref, 1, W, L)]) == (batch, row)
+    got = engine.mutant_diag(spec, fwd, counts, L, diag)
     for b in range(0, B, max(1, B // 8)):
-        one, names = _ran(lambda: engine.mutant_diag(spec, fwd[b:b + 1].contiguous(), counts[b:b + 1].contiguous(), L,
-                                                     diag[b:b + 1].contiguous()))
-        assert row in names
+        one = engine.mutant_diag(spec, fwd[b:b + 1].contiguous(), counts[b:b + 1].contiguous(), L,
+                                 diag[b:b + 1].contiguous())
         assert torch.equal(one[:, :, 0], got[:, :, b])
