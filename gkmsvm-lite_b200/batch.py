@@ -207,7 +207,8 @@ class BatchedScorer:
 
     def _pass(self, g, codes, lengths, events):
         B, L = codes.shape
-        g.before = self.index.counters() if self.index is not None else None
+        if self.index is not None and g.work is None:  # (count tables count no events)
+            g.before = self.index.counters()
         g.codes[:B, :L].copy_(codes)
         if L < g.L:
             g.codes[:B, L:].zero_()
