@@ -158,14 +158,15 @@ def _explain_pair_tables(model, perturbation: bool, dev):
 
 
 # explain table limits and cost model ("auto"): build cost per entry of 4^l x l
-# and the direct l-mer path's cost per query window with its launches, measured on
-# B200 at l=11 (a first call that builds V and the table: 0.17 s), so a call of ~300k
-# windows pays for it; the direct path of large calls has since become faster (45 ns
-# a window), but a built table serves later calls at 0.6 ns
+# and the direct l-mer path's cost per query window, measured on B200 (2,000 to 72,000
+# SVs): the table takes 10.8 ms at l = 11 (10: 3.2, 12: 45), explain_subsets 40 ns a window
+# at l = 11, d = 3 (10: 28, 12: 117; d = 2: 9.5).  A call of ~280k windows pays for it at
+# l = 11, and a built table serves later calls at 0.6 ns a window.  (V, 4 to 18 ms by the
+# SVs, is needed by both.)
 _EXPLAIN_TABLE_MAX_L = 12
 _EXPLAIN_TABLE_BYTES = 2 * 2**30
-_TABLE_BUILD_S_PER_ENTRY = 1e-9
-_DIRECT_S_PER_WINDOW = 1.5e-7
+_TABLE_BUILD_S_PER_ENTRY = 2.4e-10
+_DIRECT_S_PER_WINDOW = 4e-8
 
 
 def _explain_table(model, n_windows: int, perturbation: bool, dev):
