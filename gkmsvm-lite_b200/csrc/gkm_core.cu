@@ -726,7 +726,8 @@ __global__ void __launch_bounds__(MUT_THREADS) mutant_kernel(
 // tile's windows against the row and against its reverse complement -- queued per
 // warp and taken one per lane: the pair's l positions add to the counts of (position,
 // base, level).  Pairs whose second window covers the position, too, are the l x l
-// ones about it and are tested directly.  Bound by the integer pipe.  Measured (t=2,
+// ones about it and are tested directly.  Bound by the integer pipe (52 %) and by how few
+// warps there are (27 %).  Measured (t=2,
 // 128 x 300 bp): mutant_kernel, every pair at every position, 685 us; this 76 us.
 // mutant_kernel stays for d >= 4, for rows whose planes outgrow shared memory and where
 // it is the faster form (tiles_pay).

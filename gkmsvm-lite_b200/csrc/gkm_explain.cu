@@ -255,7 +255,8 @@ __global__ void __launch_bounds__(XS_THREADS) explain_subsets(SubsetArgs a, int 
 // that every thread has work).  The RBF form of GkmExplain needs V of its own per
 // row; built once per row it costs one gather per index entry, where visiting the
 // buckets from every window costs windows x neighbours x entries per bucket (58,000
-// gathers a window at 72,000 SVs).  Bound by L2 sectors.  Measured (4 rows of 300 ..
+// gathers a window at 72,000 SVs).  Waits for the weights' sectors, each after its entry
+// (86 % of the warps resident, L2 at 40 %).  Measured (4 rows of 300 ..
 // 600 bp, 72,000 SVs): explain_windows over the buckets 4,318 us; a thread per l-mer
 // for its four rows, both strands, 527 us; this form 328 us.
 template <int R>

@@ -91,8 +91,9 @@ __host__ __device__ __forceinline__ int et_stride(int l) { return 4 * l + 1; }  
 // k] (perturbation: the other three bases also get A[u, 0, k], the window's own base
 // nothing), times the window weight -- and
 //     out[b, base, p] = inv_dx[b] * sum over windows i covering p of part[i, base, p - i]
-// is added up from there in window order.  Bound by the reads of the table rows (352
-// bytes at l = 11, anywhere in 1.5 GB).  Measured (512 x 1,000 bp): parts to memory 156
+// is added up from there in window order.  Bound by the copies' index arithmetic and
+// issue (integer pipe 52 %) and the reads of the table rows (352 bytes at l = 11, anywhere
+// in 1.5 GB: HBM 30 %).  Measured (512 x 1,000 bp): parts to memory 156
 // us and their sums 64 us; this 90 us (138 with loads to registers).
 __global__ void __launch_bounds__(ET_THREADS) explain_table_rows(
     const double *__restrict__ A, const uint32_t *__restrict__ fwd, const int32_t *__restrict__ cnt, int64_t W, int64_t L,
