@@ -67,6 +67,8 @@ SIGNATURES = {
     "gkm_index_status": [P, P, I32, P],
     "gkm_index_pairwise": [P, P, P, I64, I64, I64, P, P, P],
     "gkm_index_score": [P, P, P, I64, I64, P, P, P, D, I32, D, P, P, P],
+    "gkm_index_add_tables": [P, P, P, P],
+    "gkm_count_table_pays": [P, I64, I64, I64, I32, P],
     "gkm_count_table_workspace": [P, I64, I64, I64, P],
     "gkm_count_table_query": [P, P, P, I64, I64, I64, P, I32, P, P, I64, P, P, P, D, I32, D, P, P, I64, P],
     "gkm_index_lmer_weights": [P, P, P, P],

@@ -176,6 +176,8 @@ inline int64_t gkm_row_count(const gkm_index *ix)
 // Built with the index / freed with it (gkm_count_table.cu).
 int gkm_ct_build(gkm_index *ix, const uint32_t *fwd, const int32_t *counts, cudaStream_t st);
 void gkm_ct_free(gkm_index *ix);
+// Whether the walk cuts rows of W windows into ranges (gkm_index.cu).
+bool gkm_walk_splits(const gkm_index *ix, int64_t B, int64_t W);
 // Sum of the window weights of a row of n windows (0: past the weight table).
 uint64_t gkm_weight_sum(const gkm_index *ix, int64_t n);
 // Device-wide exclusive scan and stable LSD radix sort of pairs (gkm_index.cu);

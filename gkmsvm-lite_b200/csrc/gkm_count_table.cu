@@ -1144,13 +1144,19 @@ static int ct_ball_size(int n, int m)
     return c;
 }
 
+// 16-bit gather sums (31 x windows) and the in-block sort bound the SV rows; weighted
+// entries are bytes: three windows of the largest weight fit.
+static bool ct_limits(const gkm_index *ix)
+{
+    const int l = ix->spec.l, D = ix->spec.dmax;
+    return l >= 8 && l <= 11 && D >= 0 && D <= 3 && ix->W <= 2048 && ix->S >= 64 && ix->wmax <= 85;
+}
+
 int gkm_ct_build(gkm_index *ix, const uint32_t *fwd, const int32_t *counts, cudaStream_t st)
 {
     ix->ct_ids = nullptr;
     const gkm_rows sh = gkm_rows_of(ix);
-    // 16-bit gather sums (31 x windows) and the in-block sort bound the SV rows;
-    // weighted entries are bytes: three windows of the largest weight fit
-    if (sh.l < 8 || sh.l > 11 || sh.D < 0 || sh.D > 3 || ix->W > 2048 || ix->S < 64 || ix->wmax > 85) return GKM_OK;
+    if (!ct_limits(ix)) return GKM_OK;
     const int64_t S = ix->S;
     uint32_t *k0 = nullptr, *k1 = nullptr, *v1 = nullptr;
     int s = GKM_OK;
@@ -1305,6 +1311,14 @@ static CtPlan ct_plan(const gkm_index *ix, int64_t B, int64_t W, int64_t windows
 // the tables win from one 300 bp row (1.3 -> 0.2 ms) on; at 30 bp rows from 64 at a time
 // the walk does (1,024 rows: 7.5 against 4.0 ms).
 constexpr double CT_CALL_US = 45.0, CT_ITEM_US = 12.0, CT_WINDOW_US = 8.5e-4, CT_GATHER_BYTES_US = 8.0e6;
+// K_raw rows (form): the walk of whole rows allocates nothing and starts at WALK_RAW_US; rows
+// that it splits over the SMs cost at least WALK_FLOOR_US, for their counts.  By the scores'
+// rule 81 of 1,896 measured shapes took the tables although slower, by up to 4.4 (256 rows of
+// 30 bp against 64 SVs, l = 8, d = 2: 366 against 83 us), by this form's 6 do, by up to 1.26.
+// A Gram matrix's index makes its lists first, CT_LISTS_US (110 to 700 measured), and its
+// weighted counts at l = 10 are counted again the oftener the nearer their mean comes to
+// CT_RECOUNT_MEAN10 (2,000 bp rows: 968 us a group where one count takes 273).
+constexpr double WALK_RAW_US = 60.0, CT_LISTS_US = 300.0, CT_RECOUNT_MEAN10 = 55.0;
 constexpr double CT_LIST_US = 0.3, CT_RECOUNT = 4.0, CT_RECOUNT_MEAN = 24.0;
 constexpr double WALK_FLOOR_US = 400.0, WALK_LOOKUP_US[2] = {8.0e-6, 5.8e-6}, WALK_HIT_US[2] = {1.1e-6, 2.0e-6};
 
@@ -1318,12 +1332,12 @@ static bool ct_exact(const gkm_index *ix, int64_t W)
 }
 
 // Whether a query over B rows of W window slots, `windows` windows in all, may
-// take the count tables: the index has gather lists, no (row, SV, level) count
-// reaches 2^32, the shared counters rarely overflow, and the estimated time is
-// below the index walk's.
-static bool ct_applies(const gkm_index *ix, int64_t B, int64_t W, int64_t windows)
+// take the count tables: the index has gather lists or is within their limits, no (row,
+// SV, level) count reaches 2^32, the shared counters rarely overflow, and the estimated
+// time is below the index walk's.
+static bool ct_applies(const gkm_index *ix, int64_t B, int64_t W, int64_t windows, int form = GKM_ROWS_SCORES)
 {
-    if (!ix->ct_ids || B < 1 || W < 1 || W > 60000 || B * ix->tiles > 0x7FFFFFFFLL) return false;
+    if (!ct_limits(ix) || B < 1 || W < 1 || W > 60000 || B * ix->tiles > 0x7FFFFFFFLL) return false;
     if (!ct_exact(ix, W)) return false;
     const bool wt = ix->spec.weighted != 0;
     // bytes hold the AT-rich rows of three times this mean
@@ -1341,19 +1355,43 @@ static bool ct_applies(const gkm_index *ix, int64_t B, int64_t W, int64_t window
     const double window = CT_WINDOW_US * row * queries;
     double slow = CT_ITEM_US + (window > CT_LIST_US * list ? window : CT_LIST_US * list);
     if (wt && ix->spec.l <= 9 && ct_mean(ix, W) > CT_RECOUNT_MEAN) slow *= CT_RECOUNT;
-    const double gather = (double)ix->ct_entries * p.rb / CT_GATHER_BYTES_US;
+    if (wt && ix->spec.l == 10 && form == GKM_ROWS_GRAM) {
+        const double x = ct_mean(ix, W) / CT_RECOUNT_MEAN10;
+        slow *= 1.0 + (CT_RECOUNT - 1.0) * (x < 1.0 ? x * x : 1.0);
+    }
+    // (lists not made yet: four windows of padding an SV)
+    const double entries = ix->ct_ids ? (double)ix->ct_entries : (double)ix->entries / ix->strands + 4.0 * ix->S;
+    const double gather = entries * p.rb / CT_GATHER_BYTES_US;
     const double table = CT_CALL_US + p.groups * (waves * (CT_ITEM_US + window) + gather),
                  table_slow = CT_CALL_US + p.groups * (waves * slow + gather);
     double walk = (double)windows * (ix->n_masks * (double)ix->tiles * WALK_LOOKUP_US[wt] +
                                      (double)ix->entries * ix->n_masks / ix->n_lmers * WALK_HIT_US[wt]);
+    double raw = walk;
     if (walk < WALK_FLOOR_US) walk = WALK_FLOOR_US;
-    return table < 0.9 * walk && table_slow < walk;
+    if (form == GKM_ROWS_SCORES) return table < 0.9 * walk && table_slow < walk;
+    // K_raw rows: whole rows leave the last of their waves of SMs partly idle
+    if (form == GKM_ROWS_GRAM || !gkm_walk_splits(ix, B, W)) {
+        const double rows = (double)B * ix->tiles, sms = gkm_sm_count();
+        raw = WALK_RAW_US + raw * ceil(rows / sms) * sms / rows;
+        if (raw < walk) walk = raw;
+    }
+    const double lists = ix->ct_ids ? 0.0 : CT_LISTS_US;
+    return table + lists < 0.9 * walk && table_slow + lists < walk;
 }
 
 extern "C" int gkm_count_table_workspace(const gkm_index_t *ix, int64_t B, int64_t W, int64_t windows, int64_t *bytes)
 {
     if (!ix || !bytes) return gkm_fail(GKM_ERR_INVALID, "null argument");
-    *bytes = ct_applies(ix, B, W, windows) ? ct_plan(ix, B, W, windows).bytes : 0;
+    *bytes = ix->ct_ids && ct_applies(ix, B, W, windows) ? ct_plan(ix, B, W, windows).bytes : 0;
+    return GKM_OK;
+}
+
+extern "C" int gkm_count_table_pays(const gkm_index_t *ix, int64_t B, int64_t W, int64_t windows, int32_t form,
+                                    int32_t *pays)
+{
+    if (!ix || !pays) return gkm_fail(GKM_ERR_INVALID, "null argument");
+    if (form < GKM_ROWS_SCORES || form > GKM_ROWS_GRAM) return gkm_fail(GKM_ERR_INVALID, "form %d", form);
+    *pays = ct_applies(ix, B, W, windows, form) ? 1 : 0;
     return GKM_OK;
 }
 

@@ -1031,6 +1031,21 @@ extern "C" int gkm_index_create_walk(const gkm_spec *spec, const uint32_t *fwd, 
     return index_create(spec, fwd, rc, counts, S, W, masks, n_masks, tile_svs, false, out, stream);
 }
 
+extern "C" int gkm_index_add_tables(gkm_index_t *ix, const uint32_t *fwd, const int32_t *counts, gkm_stream_t stream)
+{
+    if (!ix || !fwd || !counts) return gkm_fail(GKM_ERR_INVALID, "null argument");
+    if (ix->ct_ids) return GKM_OK;
+    cudaStream_t st = (cudaStream_t)stream;
+    int s = gkm_ct_build(ix, fwd, counts, st);
+    if (s == GKM_OK) {
+        const cudaError_t e = cudaStreamSynchronize(st);
+        return e == cudaSuccess ? GKM_OK : gkm_cuda_status(e, "gather lists");
+    }
+    (void)cudaGetLastError();
+    gkm_ct_free(ix);
+    return s == GKM_ERR_OOM ? GKM_OK : s;
+}
+
 extern "C" int gkm_index_free(gkm_index_t *ix)
 {
     if (!ix) return GKM_OK;
@@ -1230,6 +1245,8 @@ __global__ void count_finish_score(CountFinish f)
     part = gkm_block_sum(part, red);
     if (threadIdx.x == 0) f.partial[row * f.tiles + t] = part;
 }
+
+bool gkm_walk_splits(const gkm_index *ix, int64_t B, int64_t W) { return split_plan(ix, B, W) > 1; }
 
 // split counts hold two levels per 64-bit word when no (row, SV, level) count
 // can reach 2^32: rows of W windows x the SV rows' window slots (both strands)

@@ -260,9 +260,15 @@ def known_windows(fwd, lengths, l: int) -> int:
     return int(np.clip(lengths - l + 1, 0, None).sum())
 
 
-def table_workspace(index, B: int, W: int, windows: int, device, work: Workspace | None = None):
+# what a count-table query computes: scores, K_raw rows, or those of a self-Gram
+ROWS_SCORES, ROWS_RAW, ROWS_GRAM = range(3)
+
+
+def table_workspace(index, B: int, W: int, windows: int, device, work: Workspace | None = None, form: int = ROWS_SCORES):
     """The workspace of a count-table query, or None where the walk serves the
     call or the device has no room for it."""
+    if form != ROWS_SCORES and not index.tables_pay(B, W, windows, form):
+        return None
     n = index.table_bytes(B, W, windows)
     if n == 0:
         return None
@@ -381,6 +387,18 @@ class DeviceIndex:
 
         return self.checked(run) if check else run()
 
+    def tables_pay(self, B: int, W: int, windows: int, form: int) -> bool:
+        """Whether a query of B rows of W window slots costs less by count
+        tables (form: ROWS_SCORES, ROWS_RAW or ROWS_GRAM)."""
+        pays = ctypes.c_int32()
+        call("gkm_count_table_pays", self.handle, B, W, int(windows), form, ctypes.byref(pays))
+        return bool(pays.value)
+
+    def add_tables(self, fwd, counts) -> None:
+        """Makes the count tables' lists of an index built without them, from
+        its columns."""
+        call("gkm_index_add_tables", self.handle, ptr(fwd), ptr(counts), _st())
+
     def table_bytes(self, B: int, W: int, windows: int = 0) -> int:
         """Workspace bytes of a count-table query of B rows of W window slots
         (windows in all; 0: unknown); 0 where the index walk serves it."""
@@ -406,7 +424,7 @@ class DeviceIndex:
         walk and the self-kernel.  diag_rows: K(x, x) of at least the first so
         many rows (None: of all)."""
         B, W = bx.shape
-        tw = table_workspace(self, B, W, windows, bx.device, work)
+        tw = table_workspace(self, B, W, windows, bx.device, work, ROWS_RAW if diag_offset is None else ROWS_GRAM)
         if tw is None:
             raw, _ = self.pairwise(bx, cx, diag_offset, out=out, check=check)
             n = B if diag_rows is None else diag_rows

@@ -101,3 +101,56 @@ def test_lists_that_do_not_fit():
         assert torch.equal(raw, want)
         index.close()
     assert with_lists and without
+
+
+@pytest.mark.parametrize("kt,l,d,N,L,tables", [
+    ("gkm_esttrunc", 11, 3, 1000, 300, True), ("wgkm", 8, 2, 64, 100, False), ("wgkm", 8, 2, 300, 300, False),
+    ("wgkm", 11, 0, 300, 60, False)])
+def test_gram_makes_lists_where_they_pay(kt, l, d, N, L, tables, monkeypatch):
+    made = []
+
+    def spy(name, *args):
+        made.append(name)
+        return call(name, *args)
+
+    monkeypatch.setattr(engine, "call", spy)
+    x = syn.random_codes(np.random.default_rng(11), N, L)
+    kernel = (gk.CenterWeightedGkmKernel if kt == "wgkm" else gk.EstTruncGkmKernel)(l, l - 4, d=d)
+    got = gk.compute_gram(kernel, x)
+    assert "gkm_index_create" not in made
+    assert ("gkm_index_add_tables" in made) == ("gkm_count_table_query" in made) == tables
+    monkeypatch.setattr(engine.DeviceIndex, "tables_pay", lambda *a: not tables)  # the other form
+    monkeypatch.setattr(engine.DeviceIndex, "table_bytes",
+                        lambda self, B, W, windows=0, real=engine.DeviceIndex.table_bytes: real(self, B, W, 1 << 40))
+    assert np.array_equal(got, gk.compute_gram(kernel, x))
+
+
+def test_lists_added_later():
+    rng = np.random.default_rng(12)
+    m = gk.GkmSVM(syn.random_codes(rng, 200, 150), rng.normal(size=200), 0.1, "wgkmrbf", PARAMS).cuda()
+    full, late = m._sv_index(), engine.DeviceIndex(m._spec(), *m._sv_packed(), m._masks(), tables=False)
+    fwd, _, counts = m._sv_packed()
+    assert late.table_bytes(4, 90, 1 << 40) == 0 and late.tables_pay(4, 90, 1 << 40, engine.ROWS_RAW)
+    late.add_tables(fwd, counts)
+    n = late.table_bytes(4, 90, 1 << 40)
+    assert n == full.table_bytes(4, 90, 1 << 40) > 0
+    f, _, c = engine.pack(m._spec(), torch.from_numpy(syn.random_codes(rng, 4, 100)).cuda(), None)
+    raw = torch.empty((4, 200), dtype=torch.float64, device="cuda")
+    late.table_query(f, c, work=torch.empty(n, dtype=torch.uint8, device="cuda"), raw=raw)
+    assert torch.equal(raw, full.pairwise(f, c)[0])
+    late.close()
+
+
+# SVs, weighted, l, d, rows, length; microseconds of K_raw rows by the walk and by tables
+@pytest.mark.parametrize("shape,walk,tables", [
+    ((64, 1, 8, 2, 256, 30), 83, 366), ((300, 1, 8, 1, 256, 30), 71, 251), ((3000, 0, 11, 1, 64, 30), 68, 167),
+    ((72000, 1, 11, 0, 16, 30), 78, 219), ((64, 0, 11, 3, 1, 100), 800, 59), ((3000, 0, 11, 3, 64, 300), 1619, 279),
+    ((300, 0, 8, 2, 64, 100), 544, 117), ((3000, 0, 8, 2, 1, 1000), 694, 55)])
+def test_faster_form_of_rows(shape, walk, tables):
+    S, weighted, l, d, B, L = shape
+    rng = np.random.default_rng(0)
+    lengths = rng.integers(200, 351, S)
+    m = gk.GkmSVM(syn.ragged_codes(rng, lengths), rng.normal(size=S), 0.1, "wgkmrbf" if weighted else "gkmrbf",
+                  {"L": l, "k": l - 4, "d": d, "gamma": 1.0}, sv_lengths=lengths).cuda()
+    W = L - l + 1
+    assert m._sv_index().tables_pay(B, W, B * W, engine.ROWS_RAW) == (tables < walk)

@@ -23,6 +23,7 @@ def _model(kt, n_sv):
     # count tables for every shape (more windows than there are: the walk never looks cheaper)
     index = m._sv_index()
     index.table_bytes = lambda B, W, windows=0: DeviceIndex.table_bytes(index, B, W, 1 << 40)
+    index.tables_pay = lambda *a: True
     return m
 
 

@@ -18,6 +18,7 @@ def test_warm_makes_one_workspace(kt):
                   {"L": 11, "k": 7, "d": 3, "gamma": 1.0}).cuda()
     index = m._sv_index()
     index.table_bytes = lambda B, W, windows=0: DeviceIndex.table_bytes(index, B, W, 1 << 40)  # tables for every shape
+    index.tables_pay = lambda *a: True
     backend = GpuBackend(m)
     backend.warm(max_len=512, max_rows=3072)
     for scorer in backend.scorers:
