@@ -414,7 +414,7 @@ class BatchedIsm(_PerRowRunner):
     """gkmsvm_lite_b200.ism of device code batches through bucket graphs."""
 
     def __init__(self, model, pass_positions: int = None):
-        """pass_positions: on the index path, at most this many positions per
+        """pass_positions: by the index walk, at most this many positions per
         pass (one short persistent query per pass, so that kernels of other
         streams get the SMs between passes); None: as many as 1.5 GiB of
         workspace holds."""
@@ -427,7 +427,7 @@ class BatchedIsm(_PerRowRunner):
         return self.model._lmer_table_for() is None
 
     def body(self, codes, lengths):
-        from .ism import _ism_rows, ism_pass_bytes, ism_workspace_bytes
+        from .ism import _ism_rows, ism_pairs_bytes, ism_pass_bytes, ism_workspace_bytes
 
         m = self.model
         work = None
@@ -437,7 +437,7 @@ class BatchedIsm(_PerRowRunner):
             # allocates it, never the capture)
             B, L = codes.shape
             cap = None if self.pass_positions is None else ism_pass_bytes(m, B, self.pass_positions)
-            need = ism_workspace_bytes(m, B, L, cap)
+            need = ism_pairs_bytes(m, B, L) or ism_workspace_bytes(m, B, L, cap)
             if self._work is None or self._work.numel() < need:
                 self._work = torch.empty(need, dtype=torch.uint8, device=codes.device)
                 self._works.append(self._work)

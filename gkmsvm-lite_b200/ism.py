@@ -116,11 +116,9 @@ def _ism_index(model, fwd, rc, counts, L, check=True, work=None, table_work=None
     rbf = isinstance(kernel, RbfKernel)
     gamma = kernel.gamma if rbf else 0.0
     out = torch.empty((B, 4, L), dtype=torch.float64, device=fwd.device)
-    pairs = ctypes.c_int64()
-    if _pairs_pay(base, index, B, L, index.sms):
-        call("gkm_ism_pairs_workspace", index.handle, W, L, ctypes.byref(pairs))
+    pairs = ism_pairs_bytes(model, B, L)
     if work is None:
-        work = (torch.empty(pairs.value, dtype=torch.uint8, device=fwd.device) if pairs.value
+        work = (torch.empty(pairs, dtype=torch.uint8, device=fwd.device) if pairs
                 else ism_workspace(model, B, L, fwd.device))
 
     def run():
@@ -133,7 +131,7 @@ def _ism_index(model, fwd, rc, counts, L, check=True, work=None, table_work=None
         else:
             inv_dx = torch.ones(B, dtype=torch.float64, device=fwd.device)
             inv_dmut = torch.ones((4, L, B), dtype=torch.float64, device=fwd.device)
-        if 0 < pairs.value <= work.numel():
+        if 0 < pairs <= work.numel():
             call("gkm_ism_pairs", index.handle, ptr(fwd), ptr(counts), B, W, L, ptr(ref_raw), ptr(inv_dx),
                  ptr(inv_dmut), ptr(model._inv_ds()), ptr(model._sv_coef()), float(gamma), int(rbf), ptr(out),
                  ptr(work), int(work.numel()), stream_handle())
@@ -144,6 +142,17 @@ def _ism_index(model, fwd, rc, counts, L, check=True, work=None, table_work=None
         return out
 
     return index.checked(run) if check else run()
+
+
+def ism_pairs_bytes(model, B: int, L: int) -> int:
+    """Workspace bytes of an index-path ISM of B rows x L positions by pair
+    lists, 0 where the walk serves it."""
+    index = model._sv_index()
+    base = model.kernel.base
+    n = ctypes.c_int64()
+    if _pairs_pay(base, index, B, L, index.sms):
+        call("gkm_ism_pairs_workspace", index.handle, L - base.l + 1, L, ctypes.byref(n))
+    return n.value
 
 
 def ism_workspace_bytes(model, B: int, L: int, cap: int = None) -> int:
