@@ -1318,7 +1318,11 @@ constexpr double CT_CALL_US = 45.0, CT_ITEM_US = 12.0, CT_WINDOW_US = 8.5e-4, CT
 // A Gram matrix's index makes its lists first, CT_LISTS_US (110 to 700 measured), and its
 // weighted counts at l = 10 are counted again the oftener the nearer their mean comes to
 // CT_RECOUNT_MEAN10 (2,000 bp rows: 968 us a group where one count takes 273).
-constexpr double WALK_RAW_US = 60.0, CT_LISTS_US = 300.0, CT_RECOUNT_MEAN10 = 55.0;
+// A self-Gram's walk never splits rows: its longest row on one SM is its least (64 rows of up
+// to 1,000 bp, l = 11, d = 3, weighted: 3,577 us, tables and lists 1,240).  Where the walk packs
+// its counters it takes WALK_GRAM_PACKED times as long as other rows (100 rows of up to
+// 400 bp, l = 11, d = 3: 5,400 us, tables and lists 1,060).
+constexpr double WALK_RAW_US = 60.0, CT_LISTS_US = 300.0, CT_RECOUNT_MEAN10 = 55.0, WALK_GRAM_PACKED = 2.2;
 constexpr double CT_LIST_US = 0.3, CT_RECOUNT = 4.0, CT_RECOUNT_MEAN = 24.0;
 constexpr double WALK_FLOOR_US = 400.0, WALK_LOOKUP_US[2] = {8.0e-6, 5.8e-6}, WALK_HIT_US[2] = {1.1e-6, 2.0e-6};
 
@@ -1370,10 +1374,15 @@ static bool ct_applies(const gkm_index *ix, int64_t B, int64_t W, int64_t window
     if (walk < WALK_FLOOR_US) walk = WALK_FLOOR_US;
     if (form == GKM_ROWS_SCORES) return table < 0.9 * walk && table_slow < walk;
     // K_raw rows: whole rows leave the last of their waves of SMs partly idle
-    if (form == GKM_ROWS_GRAM || !gkm_walk_splits(ix, B, W)) {
-        const double rows = (double)B * ix->tiles, sms = gkm_sm_count();
-        raw = WALK_RAW_US + raw * ceil(rows / sms) * sms / rows;
-        if (raw < walk) walk = raw;
+    const double rows = (double)B * ix->tiles, sms = gkm_sm_count();
+    const double longest = raw / (double)windows * W * sms / ix->tiles;
+    if (form == GKM_ROWS_GRAM || !gkm_walk_splits(ix, B, W)) raw = WALK_RAW_US + raw * ceil(rows / sms) * sms / rows;
+    if (form == GKM_ROWS_GRAM) {
+        // rows are never split, so the longest one bounds it
+        if (raw < WALK_RAW_US + longest) raw = WALK_RAW_US + longest;
+        walk = ix->packed ? WALK_GRAM_PACKED * raw : raw;
+    } else if (raw < walk && !gkm_walk_splits(ix, B, W)) {
+        walk = raw;
     }
     const double lists = ix->ct_ids ? 0.0 : CT_LISTS_US;
     return table + lists < 0.9 * walk && table_slow + lists < walk;
@@ -1391,7 +1400,8 @@ extern "C" int gkm_count_table_pays(const gkm_index_t *ix, int64_t B, int64_t W,
 {
     if (!ix || !pays) return gkm_fail(GKM_ERR_INVALID, "null argument");
     if (form < GKM_ROWS_SCORES || form > GKM_ROWS_GRAM) return gkm_fail(GKM_ERR_INVALID, "form %d", form);
-    *pays = ct_applies(ix, B, W, windows, form) ? 1 : 0;
+    // (the workspace call goes by the scores' rule)
+    *pays = ct_applies(ix, B, W, windows) && ct_applies(ix, B, W, windows, form) ? 1 : 0;
     return GKM_OK;
 }
 

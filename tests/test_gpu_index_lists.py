@@ -105,7 +105,7 @@ def test_lists_that_do_not_fit():
 
 @pytest.mark.parametrize("kt,l,d,N,L,tables", [
     ("gkm_esttrunc", 11, 3, 1000, 300, True), ("wgkm", 8, 2, 64, 100, False), ("wgkm", 8, 2, 300, 300, False),
-    ("wgkm", 11, 0, 300, 60, False)])
+    ("wgkm", 11, 0, 300, 60, False), ("gkm_esttrunc", 11, 3, 100, 400, True), ("wgkm", 11, 3, 64, 1000, True)])
 def test_gram_makes_lists_where_they_pay(kt, l, d, N, L, tables, monkeypatch):
     made = []
 
