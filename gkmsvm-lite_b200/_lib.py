@@ -62,12 +62,12 @@ SIGNATURES = {
     "gkm_mutant_form": [SPEC, I64, I64, I64],
     "gkm_index_create": [SPEC, P, P, P, I64, I64, P, I32, I32, P, P],
     "gkm_index_create_walk": [SPEC, P, P, P, I64, I64, P, I32, I32, P, P],
+    "gkm_index_create_for": [SPEC, P, P, P, I64, I64, P, I32, I32, I64, I64, I64, I32, P, P],
     "gkm_index_free": [P],
     "gkm_index_info": [P, P, P, P, P],
     "gkm_index_status": [P, P, I32, P],
     "gkm_index_pairwise": [P, P, P, I64, I64, I64, P, P, P],
     "gkm_index_score": [P, P, P, I64, I64, P, P, P, D, I32, D, P, P, P],
-    "gkm_index_add_tables": [P, P, P, P],
     "gkm_count_table_pays": [P, I64, I64, I64, I32, P],
     "gkm_count_table_workspace": [P, I64, I64, I64, P],
     "gkm_count_table_query": [P, P, P, I64, I64, I64, P, I32, P, P, I64, P, P, P, D, I32, D, P, P, I64, P],

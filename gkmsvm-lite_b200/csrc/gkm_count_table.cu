@@ -1315,14 +1315,14 @@ constexpr double CT_CALL_US = 45.0, CT_ITEM_US = 12.0, CT_WINDOW_US = 8.5e-4, CT
 // that it splits over the SMs cost at least WALK_FLOOR_US, for their counts.  By the scores'
 // rule 81 of 1,896 measured shapes took the tables although slower, by up to 4.4 (256 rows of
 // 30 bp against 64 SVs, l = 8, d = 2: 366 against 83 us), by this form's 6 do, by up to 1.26.
-// A Gram matrix's index makes its lists first, CT_LISTS_US (110 to 700 measured), and its
+// A Gram matrix's index makes its lists first, CT_LISTS_US (50 to 460 measured), and its
 // weighted counts at l = 10 are counted again the oftener the nearer their mean comes to
 // CT_RECOUNT_MEAN10 (2,000 bp rows: 968 us a group where one count takes 273).
 // A self-Gram's walk never splits rows: its longest row on one SM is its least (64 rows of up
-// to 1,000 bp, l = 11, d = 3, weighted: 3,577 us, tables and lists 1,240).  Where the walk packs
+// to 1,000 bp, l = 11, d = 3, weighted: 3,577 us, tables and lists 620).  Where the walk packs
 // its counters it takes WALK_GRAM_PACKED times as long as other rows (100 rows of up to
-// 400 bp, l = 11, d = 3: 5,400 us, tables and lists 1,060).
-constexpr double WALK_RAW_US = 60.0, CT_LISTS_US = 300.0, CT_RECOUNT_MEAN10 = 55.0, WALK_GRAM_PACKED = 2.2;
+// 400 bp, l = 11, d = 3: 5,400 us, tables and lists 490).
+constexpr double WALK_RAW_US = 60.0, CT_LISTS_US = 100.0, CT_RECOUNT_MEAN10 = 55.0, WALK_GRAM_PACKED = 2.2;
 constexpr double CT_LIST_US = 0.3, CT_RECOUNT = 4.0, CT_RECOUNT_MEAN = 24.0;
 constexpr double WALK_FLOOR_US = 400.0, WALK_LOOKUP_US[2] = {8.0e-6, 5.8e-6}, WALK_HIT_US[2] = {1.1e-6, 2.0e-6};
 

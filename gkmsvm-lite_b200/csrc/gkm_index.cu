@@ -825,10 +825,18 @@ int gkm_sm_count()
     return v;
 }
 
-// tables: with the gather lists of the count tables.
+// The query that an index is built for: rows of W window slots, windows in all.
+struct IndexQuery {
+    int64_t B, W, windows;
+    int32_t form;
+};
+
+// tables: with the gather lists of the count tables; query: if it pays for them (made here,
+// beside the build's scratch: made once the scratch has gone back they fill the stream's
+// memory pool again, 0.4 ms).
 static int index_create(const gkm_spec *spec, const uint32_t *fwd, const uint32_t *rc, const int32_t *counts, int64_t S,
                         int64_t W, const uint32_t *masks, int32_t n_masks, int32_t tile_svs, bool tables,
-                        gkm_index_t **out, gkm_stream_t stream)
+                        const IndexQuery *query, gkm_index_t **out, gkm_stream_t stream)
 {
     if (!spec || !out) return gkm_fail(GKM_ERR_INVALID, "null spec or out");
     *out = nullptr;
@@ -988,6 +996,12 @@ static int index_create(const gkm_spec *spec, const uint32_t *fwd, const uint32_
         cudaMemsetAsync(ix->status, 0, 2 * sizeof(unsigned int), st);
         ix->bytes = (int64_t)sizeof(uint32_t) * ((ix->bwords ? 2 : 1) * nbuckets + 1) + (int64_t)eb +
                     sizeof(uint32_t) * n_masks;
+        if (query) {
+            int32_t pays = 0;
+            status = gkm_count_table_pays(ix, query->B, query->W, query->windows, query->form, &pays);
+            if (status != GKM_OK) break;
+            tables = pays != 0;
+        }
         if (tables) lists = gkm_ct_build(ix, fwd, counts, st);
     } while (0);
     cudaFreeAsync(ecount, st);
@@ -1021,29 +1035,23 @@ extern "C" int gkm_index_create(const gkm_spec *spec, const uint32_t *fwd, const
                                 const int32_t *counts, int64_t S, int64_t W, const uint32_t *masks,
                                 int32_t n_masks, int32_t tile_svs, gkm_index_t **out, gkm_stream_t stream)
 {
-    return index_create(spec, fwd, rc, counts, S, W, masks, n_masks, tile_svs, true, out, stream);
+    return index_create(spec, fwd, rc, counts, S, W, masks, n_masks, tile_svs, true, nullptr, out, stream);
 }
 
 extern "C" int gkm_index_create_walk(const gkm_spec *spec, const uint32_t *fwd, const uint32_t *rc,
                                      const int32_t *counts, int64_t S, int64_t W, const uint32_t *masks,
                                      int32_t n_masks, int32_t tile_svs, gkm_index_t **out, gkm_stream_t stream)
 {
-    return index_create(spec, fwd, rc, counts, S, W, masks, n_masks, tile_svs, false, out, stream);
+    return index_create(spec, fwd, rc, counts, S, W, masks, n_masks, tile_svs, false, nullptr, out, stream);
 }
 
-extern "C" int gkm_index_add_tables(gkm_index_t *ix, const uint32_t *fwd, const int32_t *counts, gkm_stream_t stream)
+extern "C" int gkm_index_create_for(const gkm_spec *spec, const uint32_t *fwd, const uint32_t *rc,
+                                    const int32_t *counts, int64_t S, int64_t W, const uint32_t *masks,
+                                    int32_t n_masks, int32_t tile_svs, int64_t query_rows, int64_t query_W,
+                                    int64_t query_windows, int32_t form, gkm_index_t **out, gkm_stream_t stream)
 {
-    if (!ix || !fwd || !counts) return gkm_fail(GKM_ERR_INVALID, "null argument");
-    if (ix->ct_ids) return GKM_OK;
-    cudaStream_t st = (cudaStream_t)stream;
-    int s = gkm_ct_build(ix, fwd, counts, st);
-    if (s == GKM_OK) {
-        const cudaError_t e = cudaStreamSynchronize(st);
-        return e == cudaSuccess ? GKM_OK : gkm_cuda_status(e, "gather lists");
-    }
-    (void)cudaGetLastError();
-    gkm_ct_free(ix);
-    return s == GKM_ERR_OOM ? GKM_OK : s;
+    const IndexQuery q = {query_rows, query_W, query_windows, form};
+    return index_create(spec, fwd, rc, counts, S, W, masks, n_masks, tile_svs, false, &q, out, stream);
 }
 
 extern "C" int gkm_index_free(gkm_index_t *ix)

@@ -282,16 +282,19 @@ class DeviceIndex:
     """An l-mer index handle over packed columns (owned; freed on close).
     tables: with the lists that count-table queries and ISM pair lists read
     (False for an index that only l-mer weights or index walks are read
-    from)."""
+    from); query (rows, window slots, windows, form): only where this query
+    pays for them."""
 
-    def __init__(self, spec: Spec, fwd, rc, counts, masks: torch.Tensor, tile_svs: int = 0, tables: bool = True):
+    def __init__(self, spec: Spec, fwd, rc, counts, masks: torch.Tensor, tile_svs: int = 0, tables: bool = True,
+                 query: tuple | None = None):
         self.spec = spec
         self.S = fwd.shape[0]
         self.masks = masks
         self.sms = torch.cuda.get_device_properties(fwd.device).multi_processor_count
         h = ctypes.c_void_p()
-        call("gkm_index_create" if tables else "gkm_index_create_walk", spec.ref, ptr(fwd), ptr(rc), ptr(counts),
-             fwd.shape[0], fwd.shape[1], ptr(masks), int(masks.numel()), int(tile_svs), ctypes.byref(h), _st())
+        create = "gkm_index_create_for" if query else "gkm_index_create" if tables else "gkm_index_create_walk"
+        call(create, spec.ref, ptr(fwd), ptr(rc), ptr(counts), fwd.shape[0], fwd.shape[1], ptr(masks), int(masks.numel()),
+             int(tile_svs), *(int(v) for v in query or ()), ctypes.byref(h), _st())
         self.handle = h
         e, t, ts, nb = ctypes.c_int64(), ctypes.c_int32(), ctypes.c_int32(), ctypes.c_int64()
         call("gkm_index_info", h, ctypes.byref(e), ctypes.byref(t), ctypes.byref(ts), ctypes.byref(nb))
@@ -393,11 +396,6 @@ class DeviceIndex:
         pays = ctypes.c_int32()
         call("gkm_count_table_pays", self.handle, B, W, int(windows), form, ctypes.byref(pays))
         return bool(pays.value)
-
-    def add_tables(self, fwd, counts) -> None:
-        """Makes the count tables' lists of an index built without them, from
-        its columns."""
-        call("gkm_index_add_tables", self.handle, ptr(fwd), ptr(counts), _st())
 
     def table_bytes(self, B: int, W: int, windows: int = 0) -> int:
         """Workspace bytes of a count-table query of B rows of W window slots

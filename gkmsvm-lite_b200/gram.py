@@ -43,11 +43,10 @@ def compute_gram(kernel, X, Y=None, *, chunk_size=1000, verbose=False, out=None,
     use_index = isinstance(base, DirectGkmKernel) and n_windows > 0 and base.index_applies(n_windows)
     raw = torch.zeros((N, M), dtype=torch.float64, device=dev)
     if use_index:
-        index = engine.DeviceIndex(spec, by, ry, cy, engine.masks_tensor(base, dev), tables=False)
+        windows = xb.n_windows(base.l)
+        index = engine.DeviceIndex(spec, by, ry, cy, engine.masks_tensor(base, dev),
+                                   query=(*bx.shape, windows, engine.ROWS_GRAM if symmetric else engine.ROWS_RAW))
         try:
-            windows = xb.n_windows(base.l)
-            if index.tables_pay(*bx.shape, windows, engine.ROWS_GRAM if symmetric else engine.ROWS_RAW):
-                index.add_tables(by, cy)
             _, dx = index.rows(bx, rx, cx, base.normalize, diag_offset=0 if symmetric else None, out=raw, windows=windows)
         finally:
             index.close()

@@ -130,14 +130,18 @@ int gkm_index_create_walk(const gkm_spec *spec, const uint32_t *fwd, const uint3
                           const int32_t *counts, int64_t S, int64_t W, const uint32_t *masks,
                           int32_t n_masks, int32_t tile_svs, gkm_index_t **out,
                           gkm_stream_t stream);
-/* Adds the lists to an index built without them, from the same columns (before other
- * threads use the index); where the device has no room for them it stays without.
+/* With the lists only where a query of this form pays for them: of query_rows rows of query_W
+ * window slots, query_windows windows in all (0: unknown).
  * gkm_count_table_pays: *pays 1 where such a query costs less by count tables than by the
  * walk, whether the lists have been made or not: GKM_ROWS_SCORES scores of the rows
  * (gkm_count_table_workspace's rule), GKM_ROWS_RAW their K_raw rows, GKM_ROWS_GRAM those of
  * the index's own columns above the diagonal. */
 enum { GKM_ROWS_SCORES = 0, GKM_ROWS_RAW = 1, GKM_ROWS_GRAM = 2 };
-int gkm_index_add_tables(gkm_index_t *index, const uint32_t *fwd, const int32_t *counts, gkm_stream_t stream);
+int gkm_index_create_for(const gkm_spec *spec, const uint32_t *fwd, const uint32_t *rc,
+                         const int32_t *counts, int64_t S, int64_t W, const uint32_t *masks,
+                         int32_t n_masks, int32_t tile_svs, int64_t query_rows, int64_t query_W,
+                         int64_t query_windows, int32_t form, gkm_index_t **out,
+                         gkm_stream_t stream);
 int gkm_count_table_pays(const gkm_index_t *index, int64_t B, int64_t W, int64_t windows, int32_t form,
                          int32_t *pays);
 int gkm_index_free(gkm_index_t *index);

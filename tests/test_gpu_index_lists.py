@@ -107,38 +107,51 @@ def test_lists_that_do_not_fit():
     ("gkm_esttrunc", 11, 3, 1000, 300, True), ("wgkm", 8, 2, 64, 100, False), ("wgkm", 8, 2, 300, 300, False),
     ("wgkm", 11, 0, 300, 60, False), ("gkm_esttrunc", 11, 3, 100, 400, True), ("wgkm", 11, 3, 64, 1000, True)])
 def test_gram_makes_lists_where_they_pay(kt, l, d, N, L, tables, monkeypatch):
-    made = []
+    made, lists = [], []
 
     def spy(name, *args):
         made.append(name)
         return call(name, *args)
 
+    def close(index, real=engine.DeviceIndex.close):
+        lists.append(_pairs_bytes(index, 100) > 0)
+        real(index)
+
     monkeypatch.setattr(engine, "call", spy)
+    monkeypatch.setattr(engine.DeviceIndex, "close", close)
     x = syn.random_codes(np.random.default_rng(11), N, L)
     kernel = (gk.CenterWeightedGkmKernel if kt == "wgkm" else gk.EstTruncGkmKernel)(l, l - 4, d=d)
     got = gk.compute_gram(kernel, x)
-    assert "gkm_index_create" not in made
-    assert ("gkm_index_add_tables" in made) == ("gkm_count_table_query" in made) == tables
-    monkeypatch.setattr(engine.DeviceIndex, "tables_pay", lambda *a: not tables)  # the other form
+    assert lists == [tables] and ("gkm_count_table_query" in made) == tables
+    # the other form
+    create = engine.DeviceIndex.__init__
+    monkeypatch.setattr(engine.DeviceIndex, "__init__",
+                        lambda self, *a, query=None, **kw: create(self, *a, tables=not tables))
+    monkeypatch.setattr(engine.DeviceIndex, "tables_pay", lambda *a: not tables)
     monkeypatch.setattr(engine.DeviceIndex, "table_bytes",
                         lambda self, B, W, windows=0, real=engine.DeviceIndex.table_bytes: real(self, B, W, 1 << 40))
     assert np.array_equal(got, gk.compute_gram(kernel, x))
 
 
-def test_lists_added_later():
+@pytest.mark.parametrize("rows,lists", [(4000, True), (64, None), (0, False)])
+def test_lists_for_a_query(rows, lists):
+    """An index for a query has lists exactly where one without them says they pay."""
     rng = np.random.default_rng(12)
     m = gk.GkmSVM(syn.random_codes(rng, 200, 150), rng.normal(size=200), 0.1, "wgkmrbf", PARAMS).cuda()
-    full, late = m._sv_index(), engine.DeviceIndex(m._spec(), *m._sv_packed(), m._masks(), tables=False)
-    fwd, _, counts = m._sv_packed()
-    assert late.table_bytes(4, 90, 1 << 40) == 0 and late.tables_pay(4, 90, 1 << 40, engine.ROWS_RAW)
-    late.add_tables(fwd, counts)
-    n = late.table_bytes(4, 90, 1 << 40)
-    assert n == full.table_bytes(4, 90, 1 << 40) > 0
+    index = engine.DeviceIndex(m._spec(), *m._sv_packed(), m._masks(), query=(rows, 290, 290 * rows, engine.ROWS_RAW))
+    walk = engine.DeviceIndex(m._spec(), *m._sv_packed(), m._masks(), tables=False)
+    pays = walk.tables_pay(rows, 290, 290 * rows, engine.ROWS_RAW)
+    assert (index.table_bytes(4, 90, 1 << 40) > 0) == pays and lists in (None, pays)
+    walk.close()
     f, _, c = engine.pack(m._spec(), torch.from_numpy(syn.random_codes(rng, 4, 100)).cuda(), None)
-    raw = torch.empty((4, 200), dtype=torch.float64, device="cuda")
-    late.table_query(f, c, work=torch.empty(n, dtype=torch.uint8, device="cuda"), raw=raw)
-    assert torch.equal(raw, full.pairwise(f, c)[0])
-    late.close()
+    want = m._sv_index().pairwise(f, c)[0]
+    assert torch.equal(index.pairwise(f, c)[0], want)
+    if pays:
+        raw = torch.empty((4, 200), dtype=torch.float64, device="cuda")
+        work = torch.empty(index.table_bytes(4, 90, 1 << 40), dtype=torch.uint8, device="cuda")
+        index.table_query(f, c, work=work, raw=raw)
+        assert torch.equal(raw, want)
+    index.close()
 
 
 # SVs, weighted, l, d, rows, length; microseconds of K_raw rows by the walk and by tables
